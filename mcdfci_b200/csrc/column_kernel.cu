@@ -25,31 +25,46 @@
 //   [off4, off5)  beta-beta doubles
 //   [off5, total) alpha-beta doubles   (ia, ib, aa, ab), ab fastest so that
 //                 consecutive threads read consecutive integral-table entries
-// CTA g of the column's G CTAs takes the g-th contiguous slice, about three
-// rounds of one entry per thread; CTAs are independent, so the grid runs in as
-// many waves as the GPU needs.  Each thread starts the hash probe of its entry
-// before it reads the integral value, so an entry costs two memory round
-// trips: (table value, home slot key), then (z atomic, x).
+// CTA g of the column's G CTAs takes the g-th contiguous slice, in blocks of
+// kRounds entries per thread.
 //
-// Candidates.  Each warp keeps a sorted top-M list (M = 32, 64 or 128 >= m)
-// in registers: per round it sorts the 32 new keys with a bitonic network,
-// takes the element-wise maximum with the list reversed (the top M of the
-// union) and re-sorts with a bitonic merge; rounds whose keys cannot enter the
-// list are skipped.  The warp lists of a CTA merge as a tree in shared memory;
-// the CTA lists go to global memory, and the last CTA of the column to finish
-// (atomic ticket) merges them and writes the column's m candidates, new z and
-// dot products (summed in a fixed order).
+// What bounds it.  Every entry touches one pseudo-random slot of a table far
+// larger than L2.  Measured on 524,288 random slots of a 17 GB table: one
+// 32-byte load each 15 us, an atomic add that returns the old z after it 17 us,
+// but 65 us when x is loaded from the sector while its atomic is in flight
+// (33 us without the load).  So a probe reads key and x in one load, and the
+// add comes later with no load beside it.  Per launch, before (a 16-byte key
+// load, then x and the atomic together; sorted warp lists) and after: 24
+// orbitals 6a5b, k = 32, m = 64: 70.8 us and 47.9 us; 42 orbitals 24a23b,
+// k = 64, m = 128: 1,757 us and 1,316 us; 12 orbitals 6a6b, k = 1, m = 100
+// (the lists alone): 34.7 us and 19.8 us.
+//
+// A block has two phases.  The first needs only the picked determinant: it
+// decodes every entry, reads its matrix element and probes the table for its
+// slot, one record per entry in shared memory.  The second needs dx: it adds
+// to z (inserting where the rule says so), reads x and scores the entry.
+//
+// Candidates.  The keys of a block and the CTA's list so far (at most m) are
+// reduced to the m largest by a radix selection over the whole CTA
+// (cta_select): a histogram per pass and one barrier, no sort, since nothing
+// downstream depends on the order of a candidate list.  Each CTA's list goes
+// to global memory with its sums, and the last CTA of the column to finish
+// (atomic ticket) selects the column's m from the G lists and adds the sums
+// in a fixed order.  A full list's smallest key is a lower bound of the
+// column's m-th largest; the CTAs share the best such bound, and keys below
+// it are dropped before the selection.
 #include "device_common.cuh"
 #include <algorithm>
 
 #include "kernels.h"
-#include "toplist.cuh"
 
 namespace mcd {
 namespace {
 
 constexpr int kNT = 256;
 constexpr int kW = kNT / 32;
+constexpr int kRounds = 4;               // entries per thread and block
+constexpr int kBlock = kNT * kRounds;
 
 struct Prelude {
   uint64_t a, b;
@@ -64,6 +79,7 @@ __device__ void build_prelude(Prelude& P, Det d, int norb) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = lanemask_lt();
   int na = 0, nb = 0, va = 0, vb = 0;
+#pragma unroll 1
   for (int half = 0; half < 2; ++half) {
     const int p = lane + 32 * half;
     const bool inr = p < norb;
@@ -84,6 +100,7 @@ __device__ void build_prelude(Prelude& P, Det d, int norb) {
     vb += __popc(m);
   }
   int nocc = 0;
+#pragma unroll 1
   for (int j = 0; j < 4; ++j) {
     const int s = lane + 32 * j;
     const int p = s >> 1;
@@ -116,7 +133,9 @@ __device__ void build_prelude(Prelude& P, Det d, int norb) {
 // Pair index t -> (i, j), i < j, with t = j(j-1)/2 + i.
 __device__ __forceinline__ void pair_decode(int t, int& i, int& j) {
   int jj = static_cast<int>((1.0f + sqrtf(8.0f * static_cast<float>(t) + 1.0f)) * 0.5f);
+#pragma unroll 1
   while (jj * (jj - 1) / 2 > t) --jj;
+#pragma unroll 1
   while ((jj + 1) * jj / 2 <= t) ++jj;
   j = jj;
   i = t - jj * (jj - 1) / 2;
@@ -130,92 +149,126 @@ __device__ __forceinline__ double single_value(const HamDev& h, const Prelude& P
   const size_t base = (static_cast<size_t>(s) * n + p) * n + r;
   const double* st = h.st + base * h.nso;
   double v = __ldg(h.sh + base);
-  for (int x = 0; x < P.nocc; ++x) v += __ldg(st + P.occso[x]);
+  // Eight loads in flight, added in order.
+#pragma unroll 1
+  for (int x0 = 0; x0 < P.nocc; x0 += 8) {
+    double t[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) t[j] = x0 + j < P.nocc ? __ldg(st + P.occso[x0 + j]) : 0.0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (x0 + j < P.nocc) v += t[j];
+  }
   return v;
 }
 
-// Entry e of the column of P's determinant: (a2, b2) and the signed value.
-// Returns kNone when the reference stores no such excitation, kKeep for the
-// diagonal and singles (kept whatever their value, as get_single_excitation
-// does), and kIfNonzero for doubles, which the reference stores only with a
-// non-zero table value.  Leaving that test to the caller lets it start the
-// hash probe before the table value arrives.
+// An excitation packed into 27 bits: orbitals p, q, r, s (6 bits each) and the
+// kind.  kXAlpha, kXBeta: p -> r; kXAlphaAlpha, kXBetaBeta: p -> r and q -> s;
+// kXAlphaBeta: alpha p -> r with beta q -> s; kXDiag: none.
+enum : unsigned { kXDiag = 0, kXAlpha, kXBeta, kXAlphaAlpha, kXBetaBeta, kXAlphaBeta };
+
+// The determinant (a, b) after packed excitation x.
+__device__ __forceinline__ void apply_x(unsigned x, uint64_t& a, uint64_t& b) {
+  const unsigned kind = (x >> 24) & 7u;
+  const uint64_t m1 = (1ull << (x & 63u)) ^ (1ull << ((x >> 12) & 63u));
+  const uint64_t m2 = (1ull << ((x >> 6) & 63u)) ^ (1ull << ((x >> 18) & 63u));
+  // p = r (kXDiag) and q = s (the singles) leave the strings as they are.
+  const bool beta1 = kind == kXBeta || kind == kXBetaBeta, beta2 = kind >= kXBetaBeta;
+  a ^= (beta1 ? 0ull : m1) ^ (beta2 ? 0ull : m2);
+  b ^= (beta1 ? m1 : 0ull) ^ (beta2 ? m2 : 0ull);
+}
+
+// Parity of the occupied spin-orbitals between p and r in the interleaved
+// order (sign_alpha, sign_beta), for spin beta or alpha.
+__device__ __forceinline__ unsigned sign_one(bool beta, uint64_t a, uint64_t b, int p, int r) {
+  const int lo = min(p, r), hi = max(p, r);
+  const uint64_t below_hi = (1ull << hi) - 1ull, upto_lo = (2ull << lo) - 1ull;
+  // own string: (lo, hi); the other's: [lo, hi) for alpha, (lo, hi] for beta
+  const uint64_t open = below_hi & ~upto_lo;
+  const uint64_t other = open | (beta ? 1ull << hi : 1ull << lo);
+  const uint64_t own_bits = beta ? b : a, other_bits = beta ? a : b;
+  // lo = hi (no excitation) counts nothing
+  return lo == hi ? 0u : static_cast<unsigned>(__popcll((own_bits & open) ^ (other_bits & other))) & 1u;
+}
+
+// Entry e of the column of P's determinant: the packed excitation, (a2, b2)
+// and the signed value.  Returns kNone when the reference stores no such
+// excitation, kKeep for the diagonal and singles (kept whatever their value,
+// as get_single_excitation does), and kIfNonzero for doubles, which the
+// reference stores only with a non-zero table value.  One path for all kinds
+// after the orbitals are decoded: the code stays small, since the leader and
+// this kernel take turns in the instruction caches.
 enum : int { kNone = 0, kKeep = 1, kIfNonzero = 2 };
 
-__device__ __forceinline__ int gen_entry(const HamDev& h, const Prelude& P, int e, double hdiag,
+__device__ __forceinline__ int gen_entry(const HamDev& h, const Prelude& P, int e, double hdiag, unsigned& x,
                                          uint64_t& a2, uint64_t& b2, double& v) {
-  const uint64_t a = P.a, b = P.b;
   const int n = h.norb;
-  if (e == 0) {
-    a2 = a;
-    b2 = b;
-    v = hdiag;
-    return kKeep;
-  }
-  if (e < P.off2) {
-    const int t = e - 1;
-    const int i = t / P.va, ri = t - i * P.va;
-    const int p = P.occA[i], r = P.virA[ri];
-    if (!((__ldg(h.spres + p) >> r) & 1ull)) return kNone;
-    double val = single_value(h, P, 0, p, r);
-    if (sign_alpha(a, b, p, r)) val = -val;
-    a2 = a ^ (1ull << p) ^ (1ull << r);
-    b2 = b;
-    v = val;
-    return kKeep;
-  }
-  if (e < P.off3) {
-    const int t = e - P.off2;
-    const int i = t / P.vb, ri = t - i * P.vb;
-    const int p = P.occB[i], r = P.virB[ri];
-    if (!((__ldg(h.spres + n + p) >> r) & 1ull)) return kNone;
-    double val = single_value(h, P, 1, p, r);
-    if (sign_beta(a, b, p, r)) val = -val;
-    a2 = a;
-    b2 = b ^ (1ull << p) ^ (1ull << r);
-    v = val;
-    return kKeep;
-  }
-  if (e < P.off4) {
-    const int t = e - P.off3;
-    const int op = t / P.ca_vir, vp = t - op * P.ca_vir;
+  int p = 0, q = 0, r = 0, s = 0;
+  unsigned kind = kXDiag;
+  const double* val = nullptr;
+  if (e >= P.off5) {
+    const unsigned vb = P.vb, va = P.va, nb = P.nb;
+    const unsigned t0 = e - P.off5, t1 = t0 / vb, t2 = t1 / va, t3 = t2 / nb;
+    p = P.occA[t3];
+    q = P.occB[t2 - t3 * nb];
+    r = P.virA[t1 - t2 * va];
+    s = P.virB[t0 - t1 * vb];
+    kind = kXAlphaBeta;
+    val = h.wab + ((static_cast<size_t>(p) * n + q) * n + r) * n + s;
+  } else if (e >= P.off3) {  // same-spin doubles
+    const bool beta = e >= P.off4;
+    const unsigned t = e - (beta ? P.off4 : P.off3);
+    const unsigned cv = beta ? P.cb_vir : P.ca_vir;
+    const unsigned char* occ = beta ? P.occB : P.occA;
+    const unsigned char* vir = beta ? P.virB : P.virA;
+    const unsigned op = t / cv, vp = t - op * cv;
     int i, j, ri, sj;
     pair_decode(op, i, j);
     pair_decode(vp, ri, sj);
-    const int p = P.occA[i], q = P.occA[j], r = P.virA[ri], s = P.virA[sj];
-    const double val = __ldg(h.vss + static_cast<size_t>(pair_index(p, q)) * h.npair + pair_index(r, s));
-    v = sign_aa(a, b, p, q, r, s) ? -val : val;
-    a2 = a ^ (1ull << p) ^ (1ull << q) ^ (1ull << r) ^ (1ull << s);
-    b2 = b;
-    return kIfNonzero;
-  }
-  if (e < P.off5) {
-    const int t = e - P.off4;
-    const int op = t / P.cb_vir, vp = t - op * P.cb_vir;
-    int i, j, ri, sj;
-    pair_decode(op, i, j);
-    pair_decode(vp, ri, sj);
-    const int p = P.occB[i], q = P.occB[j], r = P.virB[ri], s = P.virB[sj];
+    p = occ[i];
+    q = occ[j];
+    r = vir[ri];
+    s = vir[sj];
+    kind = beta ? kXBetaBeta : kXAlphaAlpha;
     const size_t np = static_cast<size_t>(h.npair);
-    const double val = __ldg(h.vss + (np + pair_index(p, q)) * np + pair_index(r, s));
-    v = sign_bb(a, b, p, q, r, s) ? -val : val;
-    a2 = a;
-    b2 = b ^ (1ull << p) ^ (1ull << q) ^ (1ull << r) ^ (1ull << s);
-    return kIfNonzero;
+    val = h.vss + ((beta ? np : 0) + pair_index(p, q)) * np + pair_index(r, s);
+  } else if (e > 0) {
+    const bool beta = e >= P.off2;
+    const unsigned t = e - (beta ? P.off2 : 1);
+    const unsigned nv = beta ? P.vb : P.va;
+    const unsigned i = t / nv;
+    p = (beta ? P.occB : P.occA)[i];
+    r = (beta ? P.virB : P.virA)[t - i * nv];
+    kind = beta ? kXBeta : kXAlpha;
   }
-  int t = e - P.off5;
-  const int sbi = t % P.vb;
-  t /= P.vb;
-  const int rai = t % P.va;
-  t /= P.va;
-  const int pbi = t % P.nb;
-  const int pai = t / P.nb;
-  const int pa = P.occA[pai], pb = P.occB[pbi], ra = P.virA[rai], sb = P.virB[sbi];
-  const double val = __ldg(h.wab + ((static_cast<size_t>(pa) * n + pb) * n + ra) * n + sb);
-  v = sign_ab(a, b, pa, ra, pb, sb) ? -val : val;
-  a2 = a ^ (1ull << pa) ^ (1ull << ra);
-  b2 = b ^ (1ull << pb) ^ (1ull << sb);
-  return kIfNonzero;
+  x = static_cast<unsigned>(p) | (static_cast<unsigned>(q) << 6) | (static_cast<unsigned>(r) << 12) |
+      (static_cast<unsigned>(s) << 18) | (kind << 24);
+  v = hdiag;
+  int keep = kKeep;
+  if (val) {
+    v = __ldg(val);
+    keep = kIfNonzero;
+  } else if (kind != kXDiag) {
+    const int sp = kind == kXBeta ? 1 : 0;
+    if (!((__ldg(h.spres + sp * n + p) >> r) & 1ull)) return kNone;
+    v = single_value(h, P, sp, p, r);
+  }
+  // The first excitation on (a, b), the second on the result of the first.
+  a2 = P.a;
+  b2 = P.b;
+  unsigned neg = sign_one(kind == kXBeta || kind == kXBetaBeta, a2, b2, p, r);
+  const uint64_t m1 = (1ull << p) ^ (1ull << r), m2 = (1ull << q) ^ (1ull << s);
+  if (kind == kXBeta || kind == kXBetaBeta)
+    b2 ^= m1;
+  else
+    a2 ^= m1;
+  neg ^= sign_one(kind >= kXBetaBeta, a2, b2, q, s);
+  if (kind >= kXBetaBeta)
+    b2 ^= m2;
+  else
+    a2 ^= m2;
+  if (neg) v = -v;
+  return keep;
 }
 
 // |dz scale| > zt, the insertion rule (src/wavefunction.h:517-528): a double
@@ -230,262 +283,415 @@ __device__ __forceinline__ bool above_threshold(dd scale, double dz, double zt) 
 
 // ---------------------------------------------------------------------------
 
-// Reads a descending list stored in global memory by another CTA (through
-// L2, bypassing L1), reversed into ascending order for the bitonic merge.
-template <int R>
-__device__ __forceinline__ void toplist_load_global(TopList<R>& T, const unsigned long long* ok,
-                                                    const unsigned* op) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int j = 0; j < R; ++j) {
-    const int i = (R - 1 - j) * 32 + (31 - lane);
-    T.k[j] = __ldcg(ok + i);
-    T.p[j] = __ldcg(op + i);
-  }
-}
+// Per-entry record of a block's first phase: the slot (low word) where the
+// determinant was found or the probe ended at an empty slot, and above it the
+// packed excitation and these flags (neither: the column has no such entry).
+constexpr unsigned kRecFound = 1u << 27;
+constexpr unsigned kRecEmpty = 1u << 28;
 
-// Merge a list held in ascending order (as toplist_load_global leaves it)
-// into the descending list L.
-template <int R>
-__device__ __forceinline__ void toplist_merge_loaded(TopList<R>& L, const TopList<R>& T) {
+struct alignas(16) ColumnShared {
+  Prelude P;
+  unsigned long long val[kRounds][kNT];  // the entries' matrix elements, then their candidate keys
+  unsigned long long rec[kRounds][kNT];
+  double x[kRounds][kNT];  // x of the entries found
+  unsigned long long list_key[kMaxM];    // the CTA's candidates so far
+  unsigned list_slot[kMaxM];
+  alignas(16) unsigned hist[3][256];
+  unsigned w_cnt[kW], w_max[kW];
+  double w_sum[kPartSum][kW];
+  unsigned out, ties;
+  int last;
+};
+
+// Reduces the CTA's candidates, S.list's n_list and the keys k[0..kRounds) (0:
+// none) with payloads p, to the m largest in S.list, in no particular order,
+// by radix selection on bits(score) + 1: scores are +0 or positive, so their
+// bit patterns order like their values.  Returns how many there are, and
+// raises `bound` to the smallest value a kept key can have when some were
+// left out.  k[kRounds], p[kRounds] are scratch.  A pass counts the keys by
+// their distance below `ref` in units of 2^lo: first the top 15 bits (the
+// exponent and three mantissa bits) down from the largest key, with all keys
+// 255 or more steps below it in the last bin, then eight bits at a time within
+// the bin that holds the m-th largest, until the keys at and above a bin are
+// exactly m.  One barrier per pass: every warp scans the histogram itself, and
+// three histograms rotate so that the one cleared was last read before the
+// previous barrier.  Called by the whole CTA; ends with a barrier.
+__device__ __forceinline__ int cta_select(ColumnShared& S, unsigned long long (&k)[kRounds + 1],
+                                          unsigned (&p)[kRounds + 1], int n_list, int m, unsigned long long& bound) {
+  constexpr int N = kRounds + 1;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  bool any = false;
 #pragma unroll
-  for (int j = 0; j < R; ++j) {
-    if (T.k[j] > L.k[j]) {
-      L.k[j] = T.k[j];
-      L.p[j] = T.p[j];
+  for (int j = 0; j < kRounds; ++j) any |= k[j] != 0ull;
+  if (!__syncthreads_or(any)) return n_list;  // nothing new above the bound
+  k[kRounds] = tid < n_list ? S.list_key[tid] : 0ull;
+  p[kRounds] = tid < n_list ? S.list_slot[tid] : 0u;
+  unsigned cnt = 0, mx = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    cnt += k[j] != 0ull ? 1u : 0u;
+    mx = max(mx, static_cast<unsigned>(k[j] >> 49));
+  }
+  cnt = __reduce_add_sync(~0u, cnt);
+  mx = __reduce_max_sync(~0u, mx);
+  if (lane == 0) {
+    S.w_cnt[warp] = cnt;
+    S.w_max[warp] = mx;
+  }
+  S.hist[0][tid] = 0u;
+  if (tid == 0) {
+    S.out = 0u;
+    S.ties = 0u;
+  }
+  __syncthreads();
+  const unsigned total = __reduce_add_sync(~0u, lane < kW ? S.w_cnt[lane] : 0u);
+  const unsigned want = static_cast<unsigned>(m);
+  unsigned long long edge = 1ull;  // keep k >= edge, of the keys equal to it only `need` when tied
+  unsigned need = want;
+  bool tied = false;
+  if (total > want) {
+    unsigned long long ref = __reduce_max_sync(~0u, lane < kW ? S.w_max[lane] : 0u);
+    unsigned long long limit = ~0ull;  // distances counted (the first passes: all)
+    int lo = 49, buf = 0;
+#pragma unroll 1
+    while (true) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        const unsigned long long d = ref - (k[j] >> lo);  // wraps above ref
+        if (k[j] != 0ull && (k[j] >> lo) <= ref && d < limit)
+          atomicAdd(&S.hist[buf][d < 255ull ? static_cast<unsigned>(d) : 255u], 1u);
+      }
+      const int nxt = buf == 2 ? 0 : buf + 1;
+      S.hist[nxt][tid] = 0u;
+      __syncthreads();
+      // The bin of the need-th largest: lane l holds bins 8l .. 8l+7.
+      const uint4 u0 = *reinterpret_cast<const uint4*>(&S.hist[buf][8 * lane]);
+      const uint4 u1 = *reinterpret_cast<const uint4*>(&S.hist[buf][8 * lane + 4]);
+      buf = nxt;
+      const unsigned c[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+      const unsigned t = ((c[0] + c[1]) + (c[2] + c[3])) + ((c[4] + c[5]) + (c[6] + c[7]));
+      unsigned run = t;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned v = __shfl_up_sync(~0u, run, o);
+        if (lane >= o) run += v;
+      }
+      const int src = __ffs(__ballot_sync(~0u, run >= need)) - 1;
+      run -= t;
+      unsigned bin = 8u * lane, in_bin = c[0];
+#pragma unroll
+      for (int j = 0; j < 7; ++j) {
+        if (run + in_bin < need) {
+          run += in_bin;
+          in_bin = c[j + 1];
+          ++bin;
+        }
+      }
+      bin = __shfl_sync(~0u, bin, src);
+      in_bin = __shfl_sync(~0u, in_bin, src);
+      need -= __shfl_sync(~0u, run, src);
+      const bool rest = limit == ~0ull && bin == 255u;  // the bin of everything further down
+      if (!rest) edge = (ref - bin) << lo;
+      if (in_bin == need) break;
+      if (rest) {
+        ref -= 255ull;
+        continue;
+      }
+      if (lo == 0) {
+        tied = true;
+        break;
+      }
+      const int w = lo < 8 ? lo : 8;
+      lo -= w;
+      limit = 1ull << w;
+      ref = ((ref - bin) << w) | (limit - 1ull);
     }
+    if (edge == 0ull) edge = 1ull;
   }
-  bitonic_merge_desc<R>(L);
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    if (k[j] == 0ull || k[j] < edge) continue;
+    if (tied && k[j] == edge && atomicAdd(&S.ties, 1u) >= need) continue;
+    const unsigned pos = atomicAdd(&S.out, 1u);
+    S.list_key[pos] = k[j];
+    S.list_slot[pos] = p[j];
+  }
+  if (total > want && edge > bound) bound = edge;
+  __syncthreads();
+  return static_cast<int>(min(total, want));
 }
 
-template <int R>
-__device__ __forceinline__ void toplist_merge_global(TopList<R>& L, const unsigned long long* ok,
-                                                     const unsigned* op) {
-  TopList<R> T;
-  toplist_load_global<R>(T, ok, op);
-  toplist_merge_loaded<R>(L, T);
+// Continues a probe at slot i, which was empty when the first phase ended
+// there: the determinant may have been inserted since (by another column), or
+// i taken by another key.  Inserts it when `insert`; -1 when it stays absent.
+// The occupancy is counted per CTA, not here.
+__device__ __forceinline__ long long probe_again(const TableDev& t, uint64_t a, uint64_t b, uint64_t i, bool insert,
+                                                 bool& inserted) {
+  inserted = false;
+#pragma unroll 1
+  for (int q = 0; q < t.max_probe; ++q) {
+    uint64_t ka, kb;
+    if (insert)
+      cas_key(t.slots + i, a, b, ka, kb);
+    else
+      load_key(t.slots + i, ka, kb);
+    if (ka == kEmptyKey && kb == kEmptyKey) {
+      inserted = insert;
+      return insert ? static_cast<long long>(i) : -1;
+    }
+    if (ka == a && kb == b) return static_cast<long long>(i);
+    i = (i + 1) & t.mask;
+  }
+  atomicOr(t.err, kErrProbe);
+  return -1;
+}
+
+// One block of entries [at, at + kBlock) of the column, below stop: both
+// phases.  Leaves the candidate keys in S.val and their slots in S.rec.
+__device__ __forceinline__ void column_block(const ColumnLaunch& L, ColumnShared& S, int at, int stop, double hd,
+                                             unsigned dslot, int col, double dxc, dd scale, dd xss, double zt,
+                                             double& acc_newz, double& acc_dot, unsigned& emit, unsigned& upd,
+                                             unsigned& ins, bool timed) {
+  const int tid = threadIdx.x;
+  const int nr = min(kRounds, (stop - at + kNT - 1) / kNT);
+  // First phase: the entries' values and slots.
+#pragma unroll 1
+  for (int r = 0; r < nr; ++r) {
+    const long long q0 = timed ? clock64() : 0;
+    const int e = at + r * kNT + tid;
+    unsigned info = 0u;
+    uint64_t slot = 0;
+    double v = 0.0;
+    if (e < stop) {
+      uint64_t a2, b2, ka = 0, kb = 0;
+      double x = 0.0;
+      const int kind = gen_entry(L.ham, S.P, e, hd, info, a2, b2, v);
+      if (kind != kNone) {
+        // The probe starts at the home slot before the integral value is used
+        // (the diagonal entry's slot is the picked determinant's own).
+        slot = e == 0 ? static_cast<uint64_t>(dslot) : det_hash(a2, b2) & L.tab.mask;
+        load_slot(L.tab.slots + slot, ka, kb, x);
+      }
+      if (timed) atomicAdd(L.sect + 0, static_cast<unsigned long long>(clock64() - q0));
+      if (kind == kKeep || (kind == kIfNonzero && v != 0.0)) {
+#pragma unroll 1
+        for (int q = 1;; ++q) {
+          if (ka == a2 && kb == b2) {
+            info |= kRecFound;
+            S.x[r][tid] = x;
+            break;
+          }
+          if (ka == kEmptyKey && kb == kEmptyKey) {
+            info |= kRecEmpty;
+            break;
+          }
+          if (q >= L.tab.max_probe) {
+            atomicOr(L.tab.err, kErrProbe);
+            break;
+          }
+          slot = (slot + 1) & L.tab.mask;
+          load_slot(L.tab.slots + slot, ka, kb, x);
+        }
+      }
+    }
+    S.rec[r][tid] = slot | (static_cast<unsigned long long>(info) << 32);
+    S.val[r][tid] = static_cast<unsigned long long>(__double_as_longlong(v));
+    if (timed) atomicAdd(L.sect + 1, static_cast<unsigned long long>(clock64() - q0));
+  }
+  // Second phase: the z updates and the candidate keys.
+  const long long q2 = timed ? clock64() : 0;
+#pragma unroll 1
+  for (int r = 0; r < nr; ++r) {
+    const unsigned long long rec = S.rec[r][tid];
+    const unsigned info = static_cast<unsigned>(rec >> 32);
+    unsigned long long key = 0ull;
+    if (info & (kRecFound | kRecEmpty)) {
+      const double v = __longlong_as_double(static_cast<long long>(S.val[r][tid]));
+      ++emit;
+      const double dz = v * dxc;
+      long long slot = static_cast<long long>(rec & 0xFFFFFFFFull);
+      double x = 0.0;
+      if (info & kRecFound) {
+        x = S.x[r][tid];
+      } else {
+        bool inserted;
+        uint64_t a2 = S.P.a, b2 = S.P.b;
+        apply_x(info, a2, b2);
+        slot = probe_again(L.tab, a2, b2, static_cast<uint64_t>(slot), above_threshold(scale, dz, zt), inserted);
+        ins += inserted ? 1u : 0u;
+        // Found after all: inserted by another column, with x = 0, since the first phase.
+      }
+      if (slot >= 0) {
+        const double znew = atomicAdd(&L.tab.slots[slot].z, dz) + dz;
+        ++upd;
+        acc_newz += v * x;
+        acc_dot += dz * x;
+        key = static_cast<unsigned long long>(__double_as_longlong(score_of(x, znew, xss))) + 1ull;
+        S.rec[r][tid] = static_cast<unsigned long long>(slot);
+      }
+    }
+    S.val[r][tid] = key;
+  }
+  if (timed) atomicAdd(L.sect + 2, static_cast<unsigned long long>(clock64() - q2));
 }
 
 // One CTA's share of one column: CTA `blk` of the launch described by L
 // (column blk / groups, slice blk % groups).
-template <int R>
 __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
-  constexpr int M = 32 * R;
   const int G = L.groups;
   const int col = blk / G;
   const int g = blk - col * G;
-  IterState* S = L.st;
-  const int kcur = S->k_cur;
+  IterState* St = L.st;
+  const int kcur = St->k_cur;
   if (col >= kcur) return;
 
-  __shared__ Prelude P;
-  __shared__ unsigned long long s_key[kW][M];
-  __shared__ unsigned s_pay[kW][M];
-  __shared__ double w_newz[kW], w_dot[kW];
-  __shared__ unsigned w_emit[kW], w_upd[kW], w_ins[kW];
-  __shared__ int s_last;
+  __shared__ __align__(16) ColumnShared S;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool timed = L.sect != nullptr && threadIdx.x == 0;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool timed = L.sect != nullptr && tid == 0;
   const long long c_start = timed ? clock64() : 0;
   // The column's scalars are read while warp 0 decodes the determinant.
-  const double dxc = S->dx[col];
-  const double hd = S->hdiag[col];
-  const dd xss = S->xss;
-  const dd scale = S->scale;
-  const dd zt{S->zt, 0.0};
-  const unsigned dslot = static_cast<unsigned>(S->slot[col]);
-  if (warp == 0) build_prelude(P, S->det[col], L.ham.norb);
+  const double dxc = St->dx[col];
+  const double hd = St->hdiag[col];
+  const dd xss = St->xss;
+  const dd scale = St->scale;
+  const double zt = St->zt;
+  const unsigned dslot = static_cast<unsigned>(St->slot[col]);
+  if (warp == 0) build_prelude(S.P, St->det[col], L.ham.norb);
   __syncthreads();
-  const int total = P.total;
-  const int per = (total + G - 1) / G;
-  const int beg = min(total, g * per);
-  const int end = min(total, beg + per);
-  const int nrounds = (end - beg + kNT - 1) / kNT;
+  const int total = S.P.total;
+  // CTA g's slice: whole rounds of kNT entries, shared evenly.
+  const int chunks = (total + kNT - 1) / kNT;
+  const int beg = kNT * (g * chunks / G);
+  const int end = min(total, kNT * ((g + 1) * chunks / G));
 
-  TopList<R> T;
-  toplist_clear<R>(T);
   double acc_newz = 0.0, acc_dot = 0.0;
   unsigned emit = 0, upd = 0, ins = 0;
+  int n_list = 0;
+  unsigned long long bound = 0ull;  // a lower bound of the column's m-th largest key
 
-  unsigned long long t_gen = 0, t_probe = 0, t_upd = 0, t_off = 0;
   const long long c_rounds = timed ? clock64() : 0;
-  for (int r = 0; r < nrounds; ++r) {
-    long long q0 = timed ? clock64() : 0;
-    const int e = beg + r * kNT + threadIdx.x;
-    unsigned long long key = 0ull;
-    unsigned slotu = 0u;
-    if (e < end) {
-      uint64_t a2, b2;
-      double v;
-      const int kind = gen_entry(L.ham, P, e, hd, a2, b2, v);
-      if (kind != kNone) {
-        // Start the probe at the home slot before the integral value is used
-        // (the diagonal entry's slot is the picked determinant's own).
-        const uint64_t home = e == 0 ? static_cast<uint64_t>(dslot) : det_hash(a2, b2) & L.tab.mask;
-        uint64_t ka = 0, kb = 0;
-        load_key(L.tab.slots + home, ka, kb);
-        long long q1 = 0;
-        if (timed) {
-          q1 = clock64();
-          t_gen += q1 - q0;
-        }
-        if (kind == kKeep || v != 0.0) {
-          ++emit;
-          const double dz = v * dxc;
-          bool inserted;
-          const long long slot =
-              table_probe_from(L.tab, a2, b2, home, ka, kb, above_threshold(scale, dz, zt.hi), inserted);
-          ins += inserted ? 1u : 0u;
-          long long q2 = 0;
-          if (timed) {
-            q2 = clock64();
-            t_probe += q2 - q1;
-          }
-          if (slot >= 0) {
-            Slot* sp = L.tab.slots + slot;
-            const double x = sp->x;
-            const double znew = atomicAdd(&sp->z, dz) + dz;
-            ++upd;
-            acc_newz += v * x;
-            acc_dot += dz * x;
-            key = static_cast<unsigned long long>(__double_as_longlong(score_of(x, znew, xss))) + 1ull;
-            slotu = static_cast<unsigned>(slot);
-            if (timed) t_upd += clock64() - q2;
-          }
-        }
-      }
-    }
-    const long long q3 = timed ? clock64() : 0;
-    toplist_offer<R>(T, key, slotu);
-    if (timed) t_off += clock64() - q3;
-  }
-  const long long c_post = timed ? clock64() : 0;
-  if (timed) {
-    atomicAdd(L.sect + 0, t_gen);
-    atomicAdd(L.sect + 1, t_probe);
-    atomicAdd(L.sect + 2, t_upd);
-    atomicAdd(L.sect + 3, t_off);
-    atomicAdd(L.sect + 4, static_cast<unsigned long long>(nrounds));
-    atomicAdd(L.sect + 5, static_cast<unsigned long long>(c_rounds - c_start));
-    atomicAdd(L.sect + 8, 1ull);
-  }
-
-  acc_newz = warp_sum(acc_newz);
-  acc_dot = warp_sum(acc_dot);
-  emit = __reduce_add_sync(~0u, emit);
-  upd = __reduce_add_sync(~0u, upd);
-  ins = __reduce_add_sync(~0u, ins);
-  if (lane == 0) {
-    w_newz[warp] = acc_newz;
-    w_dot[warp] = acc_dot;
-    w_emit[warp] = emit;
-    w_upd[warp] = upd;
-    w_ins[warp] = ins;
-  }
-  toplist_cta_merge<R>(T, &s_key[0][0], &s_pay[0][0]);
-
-  // This CTA's list and partial sums to global memory, then a ticket: the
-  // last CTA of the column merges all of them.
+  long long c_merge = 0;
+  const int M = L.list;
   const size_t part = static_cast<size_t>(col) * G + g;
-  if (warp == 0) toplist_store<R>(T, L.part_key + part * M, L.part_slot + part * M);
-  if (threadIdx.x == 0) {
-    double nz = 0.0, dt = 0.0;
-    unsigned long long e2 = 0, u2 = 0, i2 = 0;
-    for (int w = 0; w < kW; ++w) {
-      nz += w_newz[w];
-      dt += w_dot[w];
-      e2 += w_emit[w];
-      u2 += w_upd[w];
-      i2 += w_ins[w];
+  // Blocks of this CTA's entries, and after them, in the column's last CTA,
+  // blocks of the G lists (`merging`).
+  bool merging = false;
+  int at = beg, stop = end;
+#pragma unroll 1
+  while (true) {
+    unsigned long long k[kRounds + 1];
+    unsigned p[kRounds + 1];
+    if (at >= stop) {
+      if (merging) break;
+      // This CTA's list and partial sums to global memory, then a ticket: the
+      // last CTA of the column merges all of them.
+      const long long c_post = timed ? clock64() : 0;
+      if (timed) {
+        atomicAdd(L.sect + 5, static_cast<unsigned long long>(c_rounds - c_start));
+        atomicAdd(L.sect + 8, 1ull);
+      }
+      if (tid < M) {
+        L.part_key[part * M + tid] = tid < n_list ? S.list_key[tid] : 0ull;
+        L.part_slot[part * M + tid] = tid < n_list ? S.list_slot[tid] : 0u;
+        __threadfence();  // before the ticket
+      }
+      // The counters travel with the sums (exact in a double) and are added
+      // once per column by its last CTA, not by every CTA into the same words.
+      const double v[kPartSum] = {warp_sum(acc_newz), warp_sum(acc_dot),
+                                  static_cast<double>(__reduce_add_sync(~0u, emit)),
+                                  static_cast<double>(__reduce_add_sync(~0u, upd)),
+                                  static_cast<double>(__reduce_add_sync(~0u, ins))};
+      if (lane == 0) {
+#pragma unroll
+        for (int j = 0; j < kPartSum; ++j) S.w_sum[j][warp] = v[j];
+      }
+      __syncthreads();
+      if (tid < kPartSum) {
+        double t = 0.0;
+#pragma unroll 1
+        for (int w = 0; w < kW; ++w) t += S.w_sum[tid][w];
+        L.part_sum[kPartSum * part + tid] = t;
+        __threadfence();
+      }
+      __syncwarp();
+      if (tid == 0) {
+        if (bound != 0ull) atomicMax(L.bound + col, bound);
+        __threadfence();
+        S.last = (atomicAdd(L.done + col, 1u) == static_cast<unsigned>(G - 1));
+      }
+      __syncthreads();
+      c_merge = timed ? clock64() : 0;
+      if (timed) atomicAdd(L.sect + 6, static_cast<unsigned long long>(c_merge - c_post));
+      if (!S.last) return;
+      __threadfence();
+      merging = true;
+      at = 0;
+      stop = G * M;
+      n_list = 0;
+      bound = __ldcg(L.bound + col);
+      continue;
     }
-    // The counters travel with the sums (exact in a double) and are added
-    // once per column by its last CTA, not by every CTA into the same words.
-    double* ps = L.part_sum + kPartSum * part;
-    ps[0] = nz;
-    ps[1] = dt;
-    ps[2] = static_cast<double>(e2);
-    ps[3] = static_cast<double>(u2);
-    ps[4] = static_cast<double>(i2);
+    if (merging) {
+      // Lists below the best bound of any CTA are left out.
+      const size_t base = static_cast<size_t>(col) * G * M;
+#pragma unroll
+      for (int r = 0; r < kRounds; ++r) {
+        const int i = at + r * kNT + tid;
+        k[r] = i < stop ? __ldcg(L.part_key + base + i) : 0ull;
+        p[r] = i < stop ? __ldcg(L.part_slot + base + i) : 0u;
+      }
+    } else {
+      column_block(L, S, at, stop, hd, dslot, col, dxc, scale, xss, zt, acc_newz, acc_dot, emit, upd, ins, timed);
+      const int nr = min(kRounds, (stop - at + kNT - 1) / kNT);
+      const unsigned long long shared_bound = __ldcg(L.bound + col);
+      if (shared_bound > bound) bound = shared_bound;
+#pragma unroll
+      for (int r = 0; r < kRounds; ++r) {
+        k[r] = r < nr ? S.val[r][tid] : 0ull;
+        p[r] = r < nr ? static_cast<unsigned>(S.rec[r][tid]) : 0u;
+      }
+      if (timed) atomicAdd(L.sect + 4, static_cast<unsigned long long>(nr));
+    }
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r)
+      if (k[r] < bound) k[r] = 0ull;
+    const long long q3 = timed ? clock64() : 0;
+    n_list = cta_select(S, k, p, n_list, L.m, bound);
+    if (timed && !merging) atomicAdd(L.sect + 3, static_cast<unsigned long long>(clock64() - q3));
+    at += kBlock;
   }
-  // Only warp 0 wrote what the column's last CTA reads (the list and the
-  // partial sums); its fence orders those writes before the ticket.
-  if (warp == 0) __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = (atomicAdd(L.done + col, 1u) == static_cast<unsigned>(G - 1));
-  __syncthreads();
-  const long long c_merge = timed ? clock64() : 0;
-  if (timed) atomicAdd(L.sect + 6, static_cast<unsigned long long>(c_merge - c_post));
-  if (!s_last) return;
-  __threadfence();
-
-  // Last CTA of the column: merge the G CTA lists (warp w takes w, w+kW, ...).
-  TopList<R> U;
-  toplist_clear<R>(U);
-  const size_t base = static_cast<size_t>(col) * G;
-  {
-    // A warp's first kPre lists are all requested before the first merge, so
-    // their L2 round trips overlap; the merge order stays w, w+kW, ...
-    constexpr int kPre = 3;
-    TopList<R> T[kPre];
-#pragma unroll
-    for (int t = 0; t < kPre; ++t) {
-      const int gg = warp + t * kW;
-      if (gg < G) toplist_load_global<R>(T[t], L.part_key + (base + gg) * M, L.part_slot + (base + gg) * M);
-    }
-#pragma unroll
-    for (int t = 0; t < kPre; ++t)
-      if (warp + t * kW < G) toplist_merge_loaded<R>(U, T[t]);
-    for (int gg = warp + kPre * kW; gg < G; gg += kW)
-      toplist_merge_global<R>(U, L.part_key + (base + gg) * M, L.part_slot + (base + gg) * M);
+  if (tid < n_list) L.cand_slot[static_cast<size_t>(col) * L.m + tid] = S.list_slot[tid];
+  if (warp < kPartSum) {
+    // Column sums in a fixed order, one per warp: lane-strided partials, then a fixed tree.
+    double t = 0.0;
+#pragma unroll 1
+    for (int gg = lane; gg < G; gg += 32) t += __ldcg(L.part_sum + kPartSum * (static_cast<size_t>(col) * G + gg) + warp);
+    t = warp_sum(t);
+    if (lane == 0) S.w_sum[0][warp] = t;
   }
-  toplist_cta_merge<R>(U, &s_key[0][0], &s_pay[0][0]);
-  if (warp == 0) {
-    int n = 0;
-#pragma unroll
-    for (int j = 0; j < R; ++j) {
-      const int i = j * 32 + lane;
-      const bool ok = i < L.m && U.k[j] != 0ull;
-      if (ok) {
-        L.cand_score[static_cast<size_t>(col) * L.m + i] = __longlong_as_double(static_cast<long long>(U.k[j] - 1ull));
-        L.cand_slot[static_cast<size_t>(col) * L.m + i] = U.p[j];
-      }
-      n += __popc(__ballot_sync(~0u, ok));
+  __syncthreads();
+  if (tid == 0) {
+    const unsigned long long ce = static_cast<unsigned long long>(S.w_sum[0][2]);
+    const unsigned long long cu = static_cast<unsigned long long>(S.w_sum[0][3]);
+    const unsigned long long ci = static_cast<unsigned long long>(S.w_sum[0][4]);
+    if (ce) {
+      atomicAdd(&St->emitted, ce);
+      atomicAdd(&St->emitted_total, ce);
     }
-    // Column sums in a fixed order: lane-strided partials, then a fixed tree.
-    double nz = 0.0, dt = 0.0;
-    unsigned long long ce = 0, cu = 0, ci = 0;
-    for (int gg = lane; gg < G; gg += 32) {
-      const double* ps = L.part_sum + kPartSum * (base + gg);
-      nz += __ldcg(ps);
-      dt += __ldcg(ps + 1);
-      ce += static_cast<unsigned long long>(__ldcg(ps + 2));
-      cu += static_cast<unsigned long long>(__ldcg(ps + 3));
-      ci += static_cast<unsigned long long>(__ldcg(ps + 4));
+    if (cu) {
+      atomicAdd(&St->updates, cu);
+      atomicAdd(&St->updates_total, cu);
     }
-    nz = warp_sum(nz);
-    dt = warp_sum(dt);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      ce += __shfl_xor_sync(~0u, ce, o);
-      cu += __shfl_xor_sync(~0u, cu, o);
-      ci += __shfl_xor_sync(~0u, ci, o);
+    if (ci) {
+      atomicAdd(&St->z_size, ci);
+      atomicAdd(L.tab.n_occupied, ci);
     }
-    if (lane == 0) {
-      if (ce) {
-        atomicAdd(&S->emitted, ce);
-        atomicAdd(&S->emitted_total, ce);
-      }
-      if (cu) {
-        atomicAdd(&S->updates, cu);
-        atomicAdd(&S->updates_total, cu);
-      }
-      if (ci) atomicAdd(&S->z_size, ci);
-      S->newz[col] = nz;
-      S->dot[col] = dt;
-      S->cand_n[col] = n;
-      L.done[col] = 0u;
-    }
+    St->newz[col] = S.w_sum[0][0];
+    St->dot[col] = S.w_sum[0][1];
+    St->cand_n[col] = n_list;
+    L.done[col] = 0u;
+    L.bound[col] = 0ull;
   }
   if (timed) {
     atomicAdd(L.sect + 7, static_cast<unsigned long long>(clock64() - c_merge));
@@ -493,15 +699,11 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
   }
 }
 
-template <int R>
-__global__ void __launch_bounds__(kNT, 3) column_kernel(ColumnLaunch L) {
-  column_body<R>(L, blockIdx.x);
-}
+__global__ void __launch_bounds__(kNT, kColumnCtasPerSm) column_kernel(ColumnLaunch L) { column_body(L, blockIdx.x); }
 
 // Several instances in one grid: CTAs [cta_begin[i], cta_begin[i+1]) belong
 // to instance i and keep the layout of its own launch.
-template <int R>
-__global__ void __launch_bounds__(kNT, 3) column_kernel_batch(ColumnBatch B) {
+__global__ void __launch_bounds__(kNT, kColumnCtasPerSm) column_kernel_batch(ColumnBatch B) {
   int lo = 0, hi = B.n;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -510,7 +712,7 @@ __global__ void __launch_bounds__(kNT, 3) column_kernel_batch(ColumnBatch B) {
     else
       hi = mid;
   }
-  column_body<R>(B.L[lo], static_cast<int>(blockIdx.x) - B.cta_begin[lo]);
+  column_body(B.L[lo], static_cast<int>(blockIdx.x) - B.cta_begin[lo]);
 }
 
 __global__ void __launch_bounds__(kNT) debug_column_kernel(HamDev h, Det d, double hd, uint64_t* ao,
@@ -519,9 +721,10 @@ __global__ void __launch_bounds__(kNT) debug_column_kernel(HamDev h, Det d, doub
   if ((threadIdx.x >> 5) == 0) build_prelude(P, d, h.norb);
   __syncthreads();
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < P.total; e += gridDim.x * blockDim.x) {
+    unsigned x;
     uint64_t a2, b2;
     double v;
-    const int kind = gen_entry(h, P, e, hd, a2, b2, v);
+    const int kind = gen_entry(h, P, e, hd, x, a2, b2, v);
     if (kind == kKeep || (kind == kIfNonzero && v != 0.0)) {
       const int pos = atomicAdd(nout, 1);
       if (pos < cap) {
@@ -531,12 +734,6 @@ __global__ void __launch_bounds__(kNT) debug_column_kernel(HamDev h, Det d, doub
       }
     }
   }
-}
-
-template <int R>
-cudaError_t launch_column_r(const ColumnLaunch& a, cudaStream_t s) {
-  column_kernel<R><<<a.k_grid * a.groups, kNT, 0, s>>>(a);
-  return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
@@ -745,12 +942,12 @@ int column_entries(int norb, int na, int nb) {
 int column_list_size(int m) { return m <= 32 ? 32 : (m <= 64 ? 64 : 128); }
 
 int column_groups(int entries, int k, int resident) {
-  // About three rounds of kNT entries per CTA ...
-  int g = (entries + 3 * kNT - 1) / (3 * kNT);
+  // One block of kRounds rounds per CTA ...
+  int g = (entries + kBlock - 1) / kBlock;
   // ... or, when k columns of such CTAs leave resident CTA slots empty, as
   // many CTAs as fill them, down to one round each.
   if (resident > 0 && k > 0) {
-    const int fill = (resident + k - 1) / k;
+    const int fill = resident / k;
     const int one_round = (entries + kNT - 1) / kNT;
     g = std::max(g, std::min(fill, one_round));
   }
@@ -764,21 +961,13 @@ int column_groups(int entries, int k, int resident) {
 }
 
 cudaError_t launch_column(const ColumnLaunch& a, cudaStream_t s) {
-  if (a.m <= 32) return launch_column_r<1>(a, s);
-  if (a.m <= 64) return launch_column_r<2>(a, s);
-  return launch_column_r<4>(a, s);
+  column_kernel<<<a.k_grid * a.groups, kNT, 0, s>>>(a);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_column_batch(const ColumnBatch& b, cudaStream_t s) {
   if (b.n < 1 || b.n > kMaxBatch) return cudaErrorInvalidValue;
-  const int ctas = b.cta_begin[b.n];
-  const int m = b.L[0].m;
-  if (m <= 32)
-    column_kernel_batch<1><<<ctas, kNT, 0, s>>>(b);
-  else if (m <= 64)
-    column_kernel_batch<2><<<ctas, kNT, 0, s>>>(b);
-  else
-    column_kernel_batch<4><<<ctas, kNT, 0, s>>>(b);
+  column_kernel_batch<<<b.cta_begin[b.n], kNT, 0, s>>>(b);
   return cudaGetLastError();
 }
 

@@ -118,6 +118,19 @@ __device__ __forceinline__ void load_key(const Slot* s, uint64_t& a, uint64_t& b
       : "l"(s)
       : "memory");
 }
+// A slot's key and x in one 32-byte load (relaxed per 64-bit word): a key word
+// changes once, from the empty key's, so a key caught between its two words
+// has exactly one of them empty, and is read again whole.  x is not written
+// while keys are inserted.
+__device__ __forceinline__ void load_slot(const Slot* s, uint64_t& a, uint64_t& b, double& x) {
+  uint64_t xb, zb;
+  asm volatile("ld.relaxed.gpu.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(a), "=l"(b), "=l"(xb), "=l"(zb)
+               : "l"(s)
+               : "memory");
+  x = __longlong_as_double(static_cast<long long>(xb));
+  if ((a == kEmptyKey) != (b == kEmptyKey)) load_key(s, a, b);
+}
 __device__ __forceinline__ void cas_key(Slot* s, uint64_t na, uint64_t nb, uint64_t& oa, uint64_t& ob) {
   const uint64_t ea = kEmptyKey, eb = kEmptyKey;
   asm volatile(

@@ -596,7 +596,7 @@ GpuSolver::GpuSolver(const Fcidump& fci, const SolverOptions& opt) : opt_(opt) {
   }
   int sms = 0;
   check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "cudaDeviceGetAttribute");
-  groups_rule_ = column_groups(entries_, opt_.k, opt_.fill_gpu ? 3 * sms : 0);
+  groups_rule_ = column_groups(entries_, opt_.k, opt_.fill_gpu ? kColumnCtasPerSm * sms : 0);
   groups_ = opt_.groups > 0 ? opt_.groups : groups_rule_;
   if (opt_.autotune && opt_.groups == 0 && groups_ > kMaxGroups) groups_ = kMaxGroups;
   list_ = column_list_size(opt_.m);
@@ -658,12 +658,13 @@ GpuSolver::GpuSolver(const Fcidump& fci, const SolverOptions& opt) : opt_(opt) {
       mo = align_up(mo + bytes, 256);
       return o;
     };
-    const size_t o_state = carve(sizeof(IterState)), o_cs = carve(mk * sizeof(double)),
+    const size_t o_state = carve(sizeof(IterState)),
                  o_cl = carve(mk * sizeof(unsigned)), o_h = carve((static_cast<size_t>(kMaxK) * kMaxK + 2 * kMaxK + 4) * sizeof(double)),
                  o_err = carve(sizeof(unsigned)), o_occ = carve(sizeof(unsigned long long)),
                  o_sect = carve((kLeaderSections + kColumnSections) * sizeof(unsigned long long)),
                  o_pk = carve(parts * list_ * sizeof(unsigned long long)), o_ps = carve(parts * list_ * sizeof(unsigned)),
-                 o_psum = carve(parts * kPartSum * sizeof(double)), o_done = carve(kMaxK * sizeof(unsigned));
+                 o_psum = carve(parts * kPartSum * sizeof(double)), o_done = carve(kMaxK * sizeof(unsigned)),
+                 o_bound = carve(kMaxK * sizeof(unsigned long long));
     d_tables_ = device_alloc<unsigned char>(mo, "hamiltonian tables and iteration buffers");
     unsigned char* base = static_cast<unsigned char*>(d_tables_);
     auto up = [&](size_t o, const void* src, size_t bytes) {
@@ -692,7 +693,6 @@ GpuSolver::GpuSolver(const Fcidump& fci, const SolverOptions& opt) : opt_(opt) {
     }
     unsigned char* mb = static_cast<unsigned char*>(d_tables_);
     d_state_ = reinterpret_cast<IterState*>(mb + o_state);
-    d_cand_score_ = reinterpret_cast<double*>(mb + o_cs);
     d_cand_slot_ = reinterpret_cast<unsigned*>(mb + o_cl);
     d_hsub_ = reinterpret_cast<double*>(mb + o_h);
     d_err_ = reinterpret_cast<unsigned*>(mb + o_err);
@@ -702,9 +702,11 @@ GpuSolver::GpuSolver(const Fcidump& fci, const SolverOptions& opt) : opt_(opt) {
     d_part_slot_ = reinterpret_cast<unsigned*>(mb + o_ps);
     d_part_sum_ = reinterpret_cast<double*>(mb + o_psum);
     d_done_ = reinterpret_cast<unsigned*>(mb + o_done);
+    d_bound_ = reinterpret_cast<unsigned long long*>(mb + o_bound);
     check(cudaMemsetAsync(d_sect_, 0, (kLeaderSections + kColumnSections) * sizeof(unsigned long long), stream_),
           "memset");
     check(cudaMemsetAsync(d_done_, 0, kMaxK * sizeof(unsigned), stream_), "memset");
+    check(cudaMemsetAsync(d_bound_, 0, kMaxK * sizeof(unsigned long long), stream_), "memset");
     h_occ_ = pinned_words_acquire();
     for (auto& e : ev_occ_) check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
 
@@ -771,13 +773,14 @@ GpuSolver::GpuSolver(const Fcidump& fci, const SolverOptions& opt) : opt_(opt) {
   cl_.ham = hd_;
   cl_.tab = td_;
   cl_.st = d_state_;
-  cl_.cand_score = d_cand_score_;
   cl_.cand_slot = d_cand_slot_;
   cl_.part_key = d_part_key_;
   cl_.part_slot = d_part_slot_;
   cl_.part_sum = d_part_sum_;
   cl_.done = d_done_;
+  cl_.bound = d_bound_;
   cl_.m = opt_.m;
+  cl_.list = list_;
   cl_.groups = groups_;
   cl_.k_grid = opt_.k;
   cl_.na = na_;
@@ -786,7 +789,6 @@ GpuSolver::GpuSolver(const Fcidump& fci, const SolverOptions& opt) : opt_(opt) {
   ll_.ham = hd_;
   ll_.tab = td_;
   ll_.st = d_state_;
-  ll_.cand_score = d_cand_score_;
   ll_.cand_slot = d_cand_slot_;
   ll_.hsub_out = d_hsub_;
   ll_.sect = d_sect_;
@@ -817,10 +819,10 @@ void GpuSolver::release() {
   d_part_slot_ = nullptr;
   d_part_sum_ = nullptr;
   d_done_ = nullptr;
+  d_bound_ = nullptr;
   d_tables_ = nullptr;
   d_slots_ = nullptr;
   d_state_ = nullptr;
-  d_cand_score_ = nullptr;
   d_cand_slot_ = nullptr;
   d_hsub_ = nullptr;
   d_err_ = nullptr;

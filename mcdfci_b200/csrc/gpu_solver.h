@@ -217,7 +217,6 @@ class GpuSolver {
   void* d_misc_ = nullptr;  // unused: the buffers from d_state_ to d_done_ follow the tables in d_tables_
   Slot* d_slots_ = nullptr;
   IterState* d_state_ = nullptr;
-  double* d_cand_score_ = nullptr;
   unsigned* d_cand_slot_ = nullptr;
   double* d_hsub_ = nullptr;
   unsigned* d_err_ = nullptr;
@@ -227,6 +226,7 @@ class GpuSolver {
   unsigned* d_part_slot_ = nullptr;
   double* d_part_sum_ = nullptr;
   unsigned* d_done_ = nullptr;
+  unsigned long long* d_bound_ = nullptr;
   HamDev hd_{};
   TableDev td_{};
   ColumnLaunch cl_{};

@@ -80,14 +80,15 @@ struct ColumnLaunch {
   HamDev ham;
   TableDev tab;
   IterState* st;
-  double* cand_score;     // [kMaxK][m] score of each column's candidates
   unsigned* cand_slot;    // [kMaxK][m] their hash slots (tables have at most 2^32 slots)
-  unsigned long long* part_key;  // [kMaxK][groups][list] per-CTA candidate lists
+  unsigned long long* part_key;  // [kMaxK][groups][list] per-CTA candidate lists (key 0: no candidate)
   unsigned* part_slot;           // [kMaxK][groups][list]
   double* part_sum;              // [kMaxK][groups][kPartSum] per-CTA new_z, dot and entry counters
   unsigned* done;                // [kMaxK] CTAs finished per column (reset by the last one)
+  unsigned long long* bound;     // [kMaxK] a lower bound of the column's m-th largest candidate key (likewise)
   unsigned long long* sect;  // [kColumnSections] SM cycles per phase of thread 0's rounds, or null
   int m;
+  int list;               // stride of the per-CTA lists (column_list_size(m))
   int groups;             // CTAs per column
   int k_grid;             // columns launched (>= k_cur)
   int na, nb;             // electrons per spin (fixed by the starting determinant)
@@ -97,7 +98,6 @@ struct LeaderLaunch {
   HamDev ham;
   TableDev tab;
   IterState* st;
-  const double* cand_score;
   const unsigned* cand_slot;
   double* hsub_out;       // [kMaxK*kMaxK] last H_sub (row-major, k_cur x k_cur), then the last eig
                           // update's other inputs: x[kMaxK], z[kMaxK], xx (hi, lo), xz (hi, lo)
@@ -161,9 +161,9 @@ struct RdmLaunch {
 constexpr int kLeaderSections = 25;
 
 // Phases of the column kernel timed into ColumnLaunch::sect (thread 0 of each
-// CTA, summed): 0 entry decode and integral value, 1 slot probe, 2 x load,
-// z atomic and score, 3 candidate offer, 4 rounds counted, 5 prelude (CTA
-// start to the first round), 6 CTA list merge, store and ticket, 7 the
+// CTA, summed): 0 entry decode and integral value, 1 that and the slot probe,
+// 2 z atomic and score, 3 candidate selection, 4 rounds counted, 5 prelude (CTA
+// start to the first round), 6 CTA list store and ticket, 7 the
 // column's final merge (last CTA), 8 CTAs counted, 9 final merges counted.
 constexpr int kColumnSections = 10;
 
@@ -171,10 +171,10 @@ constexpr int kColumnSections = 10;
 int column_entries(int norb, int na, int nb);
 // Length of the per-CTA candidate lists for `estimate` m (32, 64 or 128).
 int column_list_size(int m);
-// CTAs per column for a column of `entries` entries.
-// CTAs per column: about three rounds of 256 entries each, or more when k
-// such columns would leave some of `resident` CTA slots of the GPU empty
-// (resident = 0: never more); at most 96.
+// CTAs per column for a column of `entries` entries: one block of 1024
+// entries each, or more when k such columns would leave some of `resident` CTA
+// slots of the GPU empty (resident = 0: never more); at most 96.
+constexpr int kColumnCtasPerSm = 4;
 int column_groups(int entries, int k, int resident);
 // The most CTAs per column the autotuner tries, and its iterations per trial.
 constexpr int kMaxGroups = 96;
