@@ -307,7 +307,9 @@ int mcd_debug_eig_method(int32_t k, const double* hsub, const double* x, const d
                          const double xz[2], int32_t method, double drop, double* dx, double new_xx[2],
                          double new_scale[2], int32_t* branch, int32_t* steps);
 /* mcd_debug_eig without any allocation: no counterpart in the reference.
- * The same kernel and results, but its device buffers are a file-scope
+ * The same update, solved as the leader solves it by default (method 2 at
+ * every k, with the full reduction when it does not certify its result: the
+ * same results to rounding), but its device buffers are a file-scope
  * static device array of 134 KB (k <= 128; a larger k returns
  * MCD_ERR_UNSUPPORTED) instead of cudaMalloc/cudaFree per call, for callers
  * that cannot allocate: a host whose device memory is committed to the hash

@@ -57,6 +57,7 @@
 #include <algorithm>
 
 #include "kernels.h"
+#include "select.cuh"
 
 namespace mcd {
 namespace {
@@ -178,19 +179,6 @@ __device__ __forceinline__ void apply_x(unsigned x, uint64_t& a, uint64_t& b) {
   b ^= (beta1 ? m1 : 0ull) ^ (beta2 ? m2 : 0ull);
 }
 
-// Parity of the occupied spin-orbitals between p and r in the interleaved
-// order (sign_alpha, sign_beta), for spin beta or alpha.
-__device__ __forceinline__ unsigned sign_one(bool beta, uint64_t a, uint64_t b, int p, int r) {
-  const int lo = min(p, r), hi = max(p, r);
-  const uint64_t below_hi = (1ull << hi) - 1ull, upto_lo = (2ull << lo) - 1ull;
-  // own string: (lo, hi); the other's: [lo, hi) for alpha, (lo, hi] for beta
-  const uint64_t open = below_hi & ~upto_lo;
-  const uint64_t other = open | (beta ? 1ull << hi : 1ull << lo);
-  const uint64_t own_bits = beta ? b : a, other_bits = beta ? a : b;
-  // lo = hi (no excitation) counts nothing
-  return lo == hi ? 0u : static_cast<unsigned>(__popcll((own_bits & open) ^ (other_bits & other))) & 1u;
-}
-
 // Entry e of the column of P's determinant: the packed excitation, (a2, b2)
 // and the signed value.  Returns kNone when the reference stores no such
 // excitation, kKeep for the diagonal and singles (kept whatever their value,
@@ -296,129 +284,45 @@ struct alignas(16) ColumnShared {
   double x[kRounds][kNT];  // x of the entries found
   unsigned long long list_key[kMaxM];    // the CTA's candidates so far
   unsigned list_slot[kMaxM];
-  alignas(16) unsigned hist[3][256];
-  unsigned w_cnt[kW], w_max[kW];
+  SelectScratch sel;
   double w_sum[kPartSum][kW];
   unsigned out, ties;
   int last;
 };
 
 // Reduces the CTA's candidates, S.list's n_list and the keys k[0..kRounds) (0:
-// none) with payloads p, to the m largest in S.list, in no particular order,
-// by radix selection on bits(score) + 1: scores are +0 or positive, so their
-// bit patterns order like their values.  Returns how many there are, and
-// raises `bound` to the smallest value a kept key can have when some were
-// left out.  k[kRounds], p[kRounds] are scratch.  A pass counts the keys by
-// their distance below `ref` in units of 2^lo: first the top 15 bits (the
-// exponent and three mantissa bits) down from the largest key, with all keys
-// 255 or more steps below it in the last bin, then eight bits at a time within
-// the bin that holds the m-th largest, until the keys at and above a bin are
-// exactly m.  One barrier per pass: every warp scans the histogram itself, and
-// three histograms rotate so that the one cleared was last read before the
-// previous barrier.  Called by the whole CTA; ends with a barrier.
+// none) with payloads p, to the m largest in S.list, in no particular order.
+// Returns how many there are, and raises `bound` to the smallest value a kept
+// key can have when some were left out.  k[kRounds], p[kRounds] are scratch.
+// Called by the whole CTA; ends with a barrier.
 __device__ __forceinline__ int cta_select(ColumnShared& S, unsigned long long (&k)[kRounds + 1],
                                           unsigned (&p)[kRounds + 1], int n_list, int m, unsigned long long& bound) {
-  constexpr int N = kRounds + 1;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x;
   bool any = false;
 #pragma unroll
   for (int j = 0; j < kRounds; ++j) any |= k[j] != 0ull;
   if (!__syncthreads_or(any)) return n_list;  // nothing new above the bound
   k[kRounds] = tid < n_list ? S.list_key[tid] : 0ull;
   p[kRounds] = tid < n_list ? S.list_slot[tid] : 0u;
-  unsigned cnt = 0, mx = 0;
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    cnt += k[j] != 0ull ? 1u : 0u;
-    mx = max(mx, static_cast<unsigned>(k[j] >> 49));
-  }
-  cnt = __reduce_add_sync(~0u, cnt);
-  mx = __reduce_max_sync(~0u, mx);
-  if (lane == 0) {
-    S.w_cnt[warp] = cnt;
-    S.w_max[warp] = mx;
-  }
-  S.hist[0][tid] = 0u;
   if (tid == 0) {
     S.out = 0u;
     S.ties = 0u;
   }
-  __syncthreads();
-  const unsigned total = __reduce_add_sync(~0u, lane < kW ? S.w_cnt[lane] : 0u);
   const unsigned want = static_cast<unsigned>(m);
-  unsigned long long edge = 1ull;  // keep k >= edge, of the keys equal to it only `need` when tied
-  unsigned need = want;
-  bool tied = false;
-  if (total > want) {
-    unsigned long long ref = __reduce_max_sync(~0u, lane < kW ? S.w_max[lane] : 0u);
-    unsigned long long limit = ~0ull;  // distances counted (the first passes: all)
-    int lo = 49, buf = 0;
-#pragma unroll 1
-    while (true) {
+  const SelectEdge E = select_edge(S.sel, want, [&](auto f) {
 #pragma unroll
-      for (int j = 0; j < N; ++j) {
-        const unsigned long long d = ref - (k[j] >> lo);  // wraps above ref
-        if (k[j] != 0ull && (k[j] >> lo) <= ref && d < limit)
-          atomicAdd(&S.hist[buf][d < 255ull ? static_cast<unsigned>(d) : 255u], 1u);
-      }
-      const int nxt = buf == 2 ? 0 : buf + 1;
-      S.hist[nxt][tid] = 0u;
-      __syncthreads();
-      // The bin of the need-th largest: lane l holds bins 8l .. 8l+7.
-      const uint4 u0 = *reinterpret_cast<const uint4*>(&S.hist[buf][8 * lane]);
-      const uint4 u1 = *reinterpret_cast<const uint4*>(&S.hist[buf][8 * lane + 4]);
-      buf = nxt;
-      const unsigned c[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
-      const unsigned t = ((c[0] + c[1]) + (c[2] + c[3])) + ((c[4] + c[5]) + (c[6] + c[7]));
-      unsigned run = t;
+    for (int j = 0; j <= kRounds; ++j) f(k[j]);
+  });
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned v = __shfl_up_sync(~0u, run, o);
-        if (lane >= o) run += v;
-      }
-      const int src = __ffs(__ballot_sync(~0u, run >= need)) - 1;
-      run -= t;
-      unsigned bin = 8u * lane, in_bin = c[0];
-#pragma unroll
-      for (int j = 0; j < 7; ++j) {
-        if (run + in_bin < need) {
-          run += in_bin;
-          in_bin = c[j + 1];
-          ++bin;
-        }
-      }
-      bin = __shfl_sync(~0u, bin, src);
-      in_bin = __shfl_sync(~0u, in_bin, src);
-      need -= __shfl_sync(~0u, run, src);
-      const bool rest = limit == ~0ull && bin == 255u;  // the bin of everything further down
-      if (!rest) edge = (ref - bin) << lo;
-      if (in_bin == need) break;
-      if (rest) {
-        ref -= 255ull;
-        continue;
-      }
-      if (lo == 0) {
-        tied = true;
-        break;
-      }
-      const int w = lo < 8 ? lo : 8;
-      lo -= w;
-      limit = 1ull << w;
-      ref = ((ref - bin) << w) | (limit - 1ull);
-    }
-    if (edge == 0ull) edge = 1ull;
-  }
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    if (k[j] == 0ull || k[j] < edge) continue;
-    if (tied && k[j] == edge && atomicAdd(&S.ties, 1u) >= need) continue;
+  for (int j = 0; j <= kRounds; ++j) {
+    if (k[j] < E.edge || (E.tied && k[j] == E.edge && atomicAdd(&S.ties, 1u) >= E.need)) continue;
     const unsigned pos = atomicAdd(&S.out, 1u);
     S.list_key[pos] = k[j];
     S.list_slot[pos] = p[j];
   }
-  if (total > want && edge > bound) bound = edge;
+  if (E.total > want && E.edge > bound) bound = E.edge;
   __syncthreads();
-  return static_cast<int>(min(total, want));
+  return static_cast<int>(min(E.total, want));
 }
 
 // Continues a probe at slot i, which was empty when the first phase ended
@@ -526,7 +430,7 @@ __device__ __forceinline__ void column_block(const ColumnLaunch& L, ColumnShared
         ++upd;
         acc_newz += v * x;
         acc_dot += dz * x;
-        key = static_cast<unsigned long long>(__double_as_longlong(score_of(x, znew, xss))) + 1ull;
+        key = score_key(score_of(x, znew, xss));
         S.rec[r][tid] = static_cast<unsigned long long>(slot);
       }
     }
@@ -661,7 +565,7 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
     if (timed && !merging) atomicAdd(L.sect + 3, static_cast<unsigned long long>(clock64() - q3));
     at += kBlock;
   }
-  if (tid < n_list) L.cand_slot[static_cast<size_t>(col) * L.m + tid] = S.list_slot[tid];
+  if (tid < L.m) L.cand_slot[static_cast<size_t>(col) * L.m + tid] = tid < n_list ? S.list_slot[tid] : kNoSlot;
   if (warp < kPartSum) {
     // Column sums in a fixed order, one per warp: lane-strided partials, then a fixed tree.
     double t = 0.0;

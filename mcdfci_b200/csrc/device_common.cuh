@@ -42,6 +42,19 @@ __device__ __forceinline__ int sign_beta(uint64_t a, uint64_t b, int p, int r) {
   return (__popcll(b & mask_open(lo, hi)) + __popcll(a & mask_right_closed(lo, hi))) & 1;
 }
 
+// Parity of the occupied spin-orbitals between p and r in the interleaved
+// order (sign_alpha, sign_beta), for spin beta or alpha.
+__device__ __forceinline__ unsigned sign_one(bool beta, uint64_t a, uint64_t b, int p, int r) {
+  const int lo = min(p, r), hi = max(p, r);
+  const uint64_t below_hi = (1ull << hi) - 1ull, upto_lo = (2ull << lo) - 1ull;
+  // own string: (lo, hi); the other's: [lo, hi) for alpha, (lo, hi] for beta
+  const uint64_t open = below_hi & ~upto_lo;
+  const uint64_t other = open | (beta ? 1ull << hi : 1ull << lo);
+  const uint64_t own_bits = beta ? b : a, other_bits = beta ? a : b;
+  // lo = hi (no excitation) counts nothing
+  return lo == hi ? 0u : static_cast<unsigned>(__popcll((own_bits & open) ^ (other_bits & other))) & 1u;
+}
+
 // Sequential sign of a double excitation: first (p->r) on the determinant, then
 // (q->s) on the result (src/hamiltonian.h:397-403).  For an alpha-beta double
 // the two excitations commute, so alpha-first gives the reference's sign
@@ -123,7 +136,8 @@ __device__ __forceinline__ void load_key(const Slot* s, uint64_t& a, uint64_t& b
 // has exactly one of them empty, and is read again whole.  x is not written
 // while keys are inserted.
 __device__ __forceinline__ void load_slot(const Slot* s, uint64_t& a, uint64_t& b, double& x) {
-  uint64_t xb, zb;
+  uint64_t xb;
+  [[maybe_unused]] uint64_t zb;
   asm volatile("ld.relaxed.gpu.global.v4.b64 {%0, %1, %2, %3}, [%4];"
                : "=l"(a), "=l"(b), "=l"(xb), "=l"(zb)
                : "l"(s)
@@ -147,6 +161,11 @@ __device__ __forceinline__ double load_relaxed(const double* p) {
   double v;
   asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
   return v;
+}
+
+// x and z of a slot in one 16-byte load.
+__device__ __forceinline__ void load_xz(const Slot* s, double& x, double& z) {
+  asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(x), "=d"(z) : "l"(&s->x) : "memory");
 }
 
 // Linear probing, continuing from the home slot i whose key (ka, kb) the

@@ -33,10 +33,9 @@
 // The caller forms the Rayleigh quotient from the original matrix, the
 // quantity that the reference's refined step approximates
 // (rq = v'Bv + 2 dv'Bv, src/solver.h:516-521).
-// Two faster solvers that fall back to the reduction follow: 5, shifted
-// inverse iteration from a certified shift, and 6, the bordered fixed point
-// (the default), a one-warp iteration on the structure of the subspace matrix
-// whose result is certified as the lowest eigenpair by interlacing.
+// A faster solver that falls back to the reduction follows: 5, shifted
+// inverse iteration from a certified shift.  The default solver, the bordered
+// fixed point, is part of the update itself (eig_update_bordered).
 #pragma once
 
 #include "device_common.cuh"
@@ -1128,205 +1127,6 @@ __device__ bool eig_lowest_shifted_warp(double* A, int lda, int n, const EigVecs
   *steps = s_steps;
   *diff = s_diff;
   return s_ok;
-}
-
-// ---------------------------------------------------------------------------
-// 6. The lowest eigenpair of the bordered matrix B = [[a, b'], [b, C]] (n = k + 1
-//    rows, k <= kBorderMaxK) when it lies below the Gershgorin bound of C,
-//    g = min_i (C_ii - sum_{j != i} |C_ij|).  By Cauchy interlacing B has exactly
-//    one eigenvalue below lambda_1(C) >= g, so an approximate eigenpair (lambda,
-//    v) with lambda + ||B v - lambda v|| / ||v|| < g belongs to the lowest
-//    eigenvalue (some eigenvalue lies within the residual norm of lambda).  With
-//    v = (1, y), D the diagonal of C and E the rest, the last k rows of
-//    (B - lambda I) v = 0 read (D - lambda I) y = -(b + E y), and the first row
-//    lambda = a + b'y.  One warp iterates
-//        y <- -(b + E y) / (d - lambda),   lambda <- a + b'y,
-//    which contracts by about max_i sum_j |E_ij| / (d_i - lambda) per step, less
-//    than 1 whenever lambda < g (C is strongly diagonal in a subspace of picked
-//    determinants, most of which are not connected by a single or double
-//    excitation).  The product E y of a step also gives the residual of the
-//    current iterate, r_i = (b + E y)_i + (d_i - lambda) y_i (row 0's residual
-//    is zero by the choice of lambda), so a step costs one matrix-vector
-//    product, a reciprocal per row and one warp reduction of three values, with
-//    no block barrier.  The reciprocal of d_i - lambda is one Newton-Raphson
-//    step, r <- r + r e with e = 1 - (d_i - lambda) r, from the last step's r,
-//    while |e| < 1e-3 (lambda moves less every step, so the error falls
-//    quadratically), and a division otherwise (the first steps); an inexact r
-//    changes only the step, not the fixed point.  E is sparse (most picked determinants are not
-//    connected), so each lane first packs its rows' nonzero entries of E into
-//    `pack`, 2 (k + 1) lda doubles of scratch (values of row i from i lda on;
-//    after the k rows of values, their columns as 4-byte ints, row i from
-//    i (2 lda + 1) on), and a step's product runs over those only.  The
-//    iteration stops when ||r|| / ||v|| reaches
-//    1e-15 max_i sum_j |B_ij| (or stalls within 16 times that), and gives up
-//    when it stops contracting or lambda is not below g; A is only read.
-//    Returns true (uniform over the block) with V.y = (1, y) when the pair is
-//    certified; *iters receives the steps taken and *resid the final residual
-//    norm.  All threads call it.
-constexpr int kBorderMaxK = 64;
-constexpr int kBorderIters = 64;
-
-__device__ bool eig_lowest_bordered(const double* A, int lda, int n, const EigVecs& V, double* pack, int* iters,
-                                    double* resid, SectionClock& clk) {
-  __shared__ int s_ok, s_it;
-  __shared__ double s_rn;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int k = n - 1;
-  if (warp == 0) {
-    double* ys = V.y + 1;  // y_j at ys[j]
-    const double a = A[0];
-    double d[2], b[2], y[2];
-    bool own[2];
-    int cnt[2];
-    double gl = 1e300, nb = 0.0, babs = 0.0;
-    // Row i's nonzero off-diagonal entries of C: values at pv + i lda, their
-    // columns at pc + i (2 lda + 1) (an odd stride in 4-byte words).
-    double* const pv = pack;
-    int* const pc = reinterpret_cast<int*>(pack + static_cast<size_t>(k) * lda);
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int i = lane + 32 * q;
-      own[q] = i < k;
-      const double* row = A + (i + 1) * lda + 1;
-      d[q] = own[q] ? row[i] : 0.0;
-      b[q] = own[q] ? A[i + 1] : 0.0;
-      double off = 0.0;
-      int c = 0;
-      if (own[q])
-        for (int j0 = 0; j0 < k; j0 += 8) {
-          double v8[8];  // eight loads in flight before the dependent stores
-#pragma unroll
-          for (int jj = 0; jj < 8; ++jj) v8[jj] = j0 + jj < k ? row[j0 + jj] : 0.0;
-#pragma unroll
-          for (int jj = 0; jj < 8; ++jj) {
-            const int j = j0 + jj;
-            if (j != i && v8[jj] != 0.0) {
-              off += fabs(v8[jj]);
-              pv[i * lda + c] = v8[jj];
-              pc[i * (2 * lda + 1) + c] = j;
-              ++c;
-            }
-          }
-        }
-      cnt[q] = c;
-      y[q] = 0.0;
-      if (own[q]) {
-        gl = fmin(gl, d[q] - off);
-        nb = fmax(nb, fabs(d[q]) + off + fabs(b[q]));
-        babs += fabs(b[q]);
-        ys[i] = 0.0;
-      }
-    }
-    int cmax = max(cnt[0], cnt[1]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      gl = fmin(gl, __shfl_xor_sync(~0u, gl, o));
-      nb = fmax(nb, __shfl_xor_sync(~0u, nb, o));
-      babs += __shfl_xor_sync(~0u, babs, o);
-      cmax = max(cmax, __shfl_xor_sync(~0u, cmax, o));
-    }
-    nb = fmax(nb, fabs(a) + babs);
-    if (lane == 0) V.y[0] = 1.0;
-    __syncwarp();
-    clk.mark(17);
-    const double tol = 1e-15 * nb;
-    const double tol2 = tol * tol;
-    double lam = fmin(a, gl) - 1e-3 * (1.0 + fabs(a));
-    double rcp[2];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) rcp[q] = own[q] ? 1.0 / (d[q] - lam) : 0.0;
-    // The tests compare squared residual norms |r|^2 / |v|^2 cross-multiplied,
-    // so that no division or square root sits on a step's chain.
-    double rrp = 1e300, vvp = 1.0;  // |r|^2 and |v|^2 of the previous step
-    bool ok = false;
-    int t = 0;
-    for (; t < kBorderIters; ++t) {
-      // s = b + E y_t for this lane's rows, over their packed nonzeros.
-      double s[2], yn[2];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int i = lane + 32 * q;
-        const double* rv = pv + i * lda;
-        const int* rc = pc + i * (2 * lda + 1);
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-        if (q == 0 || k > 32) {
-          const int c = cnt[q];
-          int e = 0;
-          for (; e + 3 < cmax; e += 4) {
-            if (e < c) s0 = fma(rv[e], ys[rc[e]], s0);
-            if (e + 1 < c) s1 = fma(rv[e + 1], ys[rc[e + 1]], s1);
-            if (e + 2 < c) s2 = fma(rv[e + 2], ys[rc[e + 2]], s2);
-            if (e + 3 < c) s3 = fma(rv[e + 3], ys[rc[e + 3]], s3);
-          }
-          for (; e < cmax; ++e)
-            if (e < c) s0 = fma(rv[e], ys[rc[e]], s0);
-          s[q] = b[q] + ((s0 + s1) + (s2 + s3));
-          if (t > 0) {
-            const double x = d[q] - lam;
-            const double e = fma(-x, rcp[q], 1.0);  // relative error of rcp as 1 / x
-            if (fabs(e) < 1e-3)
-              rcp[q] = fma(rcp[q], e, rcp[q]);
-            else
-              rcp[q] = 1.0 / x;
-          }
-          yn[q] = own[q] ? -s[q] * rcp[q] : 0.0;
-        } else {
-          s[q] = 0.0;
-          yn[q] = 0.0;
-        }
-      }
-      clk.mark(18);
-      // Residual of (lambda_t, v_t), |y_t|^2 and b'y_{t+1}, in one reduction.
-      double rr = 0.0, yy = 0.0, by = 0.0;
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        if (!own[q]) continue;
-        const double ri = fma(d[q] - lam, y[q], s[q]);
-        rr = fma(ri, ri, rr);
-        yy = fma(y[q], y[q], yy);
-        by = fma(b[q], yn[q], by);
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        rr += __shfl_xor_sync(~0u, rr, o);
-        yy += __shfl_xor_sync(~0u, yy, o);
-        by += __shfl_xor_sync(~0u, by, o);
-      }
-      const double vv = 1.0 + yy;
-      if (!isfinite(rr) || !isfinite(vv)) break;
-      // rn <= tol, or rn > rn_prev / 2 and rn <= 16 tol (stalled at rounding)
-      const bool small =
-          rr <= tol2 * vv || (t >= 2 && rr * vvp > 0.25 * rrp * vv && rr <= 256.0 * tol2 * vv);
-      if (t > 0 && small) {
-        const double rn = sqrt(rr / vv);
-        ok = lam + rn < gl;
-        if (lane == 0) s_rn = rn;
-        break;
-      }
-      // not contracting (rn > 0.9 rn_prev), or lambda not below g
-      if ((t >= 8 && rr * vvp > 0.81 * rrp * vv) || (t >= 4 && !(lam < gl))) break;
-      clk.mark(19);
-      rrp = rr;
-      vvp = vv;
-      __syncwarp();  // every lane has read y_t
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        y[q] = yn[q];
-        if (own[q]) ys[lane + 32 * q] = yn[q];
-      }
-      lam = a + by;
-      __syncwarp();
-      clk.mark(20);
-    }
-    if (lane == 0) {
-      s_ok = ok;
-      s_it = t + 1;
-    }
-  }
-  __syncthreads();
-  *iters = s_it;
-  if (resid) *resid = s_ok ? s_rn : 0.0;
-  return s_ok != 0;
 }
 
 }  // namespace mcd

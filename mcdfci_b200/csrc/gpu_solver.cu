@@ -365,7 +365,10 @@ __global__ void compact_cand_restore_kernel(TableDev t, const IterState* st, con
                                             int m) {
   const int col = blockIdx.x;
   for (int i = threadIdx.x; i < m; i += blockDim.x) {
-    if (!(col < st->k_cur && i < st->cand_n[col])) continue;
+    if (!(col < st->k_cur && i < st->cand_n[col])) {
+      cand_slot[col * m + i] = kNoSlot;
+      continue;
+    }
     const Slot s = saved[col * m + i];
     bool inserted;
     const long long j = table_upsert(t, s.a, s.b, inserted);

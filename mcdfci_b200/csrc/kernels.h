@@ -80,7 +80,7 @@ struct ColumnLaunch {
   HamDev ham;
   TableDev tab;
   IterState* st;
-  unsigned* cand_slot;    // [kMaxK][m] their hash slots (tables have at most 2^32 slots)
+  unsigned* cand_slot;    // [kMaxK][m] hash slots of each column's candidates, then kNoSlot (tables have at most 2^32 slots)
   unsigned long long* part_key;  // [kMaxK][groups][list] per-CTA candidate lists (key 0: no candidate)
   unsigned* part_slot;           // [kMaxK][groups][list]
   double* part_sum;              // [kMaxK][groups][kPartSum] per-CTA new_z, dot and entry counters

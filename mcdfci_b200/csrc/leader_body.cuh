@@ -23,11 +23,22 @@
 //                          (WaveFunctionCuckoo::update_x, src/wavefunction.h:425-451)
 //   publish                the k picked determinants, dx, H_cc, xx*scale^2
 //                          and scale for the column kernel.
+//
+// What bounds it: a serial chain on one SM, so the cycles of its phases, and
+// of those the instructions that 16 warps issue on four schedulers as much as
+// the loads they wait for.  The candidate and H_sub phases keep four to
+// sixteen loads per thread in flight, and nothing of the iteration state that
+// is not needed is copied.  Cycles per iteration before and after (12 orbitals
+// 6a5b, k = 32, m = 64): candidates and scores 16,900 and 10,100, selection
+// 10,100 and 5,700, H_sub 9,800 and 6,500, eig update 34,300 and 14,500, all
+// 86,700 and 46,500; 24 orbitals, k = 96, m = 128: the update by the bordered
+// form instead of the full reduction, 380 us and 107 us for the whole kernel.
 #pragma once
 
 #include "eig.cuh"
 #include "device_common.cuh"
 #include "kernels.h"
+#include "select.cuh"
 
 namespace mcd {
 namespace {
@@ -39,107 +50,110 @@ constexpr int kLW = kLT / 32;     // warps
 // ---------------------------------------------------------------------------
 // Matrix elements between two determinants.
 
+__device__ __forceinline__ int lowest_bit(uint64_t x) { return __ffsll(static_cast<long long>(x)) - 1; }
+
 // Single p->r of spin s summed over the occupied spin-orbitals of (a, b) in
-// interleaved order.
-__device__ double single_value_det(const HamDev& h, int s, int p, int r, uint64_t a, uint64_t b) {
-  const int n = h.norb;
-  const size_t base = (static_cast<size_t>(s) * n + p) * n + r;
+// interleaved order, sixteen loads in flight.
+__device__ __forceinline__ double single_value_det(const HamDev& h, int s, int p, int r, uint64_t a, uint64_t b) {
+  const size_t base = (static_cast<size_t>(s) * h.norb + p) * h.norb + r;
   const double* st = h.st + base * h.nso;
-  double v = h.sh[base];
-  uint64_t u = a | b;
-  while (u) {
-    const int q = __ffsll(static_cast<long long>(u)) - 1;
-    u &= u - 1;
-    if ((a >> q) & 1ull) v += st[2 * q];
-    if ((b >> q) & 1ull) v += st[2 * q + 1];
+  double v = __ldg(h.sh + base);
+#pragma unroll 1
+  while (a | b) {
+    double t[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      t[j] = 0.0;
+      const uint64_t u = a | b, bit = u & (0ull - u);
+      if (u == 0ull) continue;
+      const bool alpha = (a & bit) != 0ull;
+      t[j] = __ldg(st + 2 * lowest_bit(u) + (alpha ? 0 : 1));
+      if (alpha)
+        a ^= bit;
+      else
+        b ^= bit;
+    }
+    // Adding 0.0 past the last orbital changes nothing but the sign of a zero.
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v += t[j];
   }
   return v;
 }
 
-__device__ __forceinline__ int lowest_bit(uint64_t x) { return __ffsll(static_cast<long long>(x)) - 1; }
-
 // <d2|H|d1> computed from d1's side, as HamiltonianMolecule::get_off_diagonal(d1, d2).
-__device__ double off_diagonal(const HamDev& h, Det d1, Det d2) {
+__device__ __forceinline__ double off_diagonal(const HamDev& h, Det d1, Det d2) {
   const uint64_t da = d1.a ^ d2.a, db = d1.b ^ d2.b;
   const int na = __popcll(da), nb = __popcll(db);
+  const bool single = na + nb == 2;
+  if ((!single && na + nb != 4) || (na & 1)) return 0.0;
+  // The excitation p -> r, and q -> s for a double: alpha before beta, lower
+  // orbitals first; beta1 and beta2 are their spins.
+  const bool beta1 = na == 0, beta2 = na != 4;
+  uint64_t o1 = beta1 ? db & d1.b : da & d1.a, v1 = beta1 ? db & d2.b : da & d2.a;
+  const int p = lowest_bit(o1), r = lowest_bit(v1);
+  int q = 0, s = 0;
   const int n = h.norb;
-  if (na + nb == 2) {
-    if (na == 2) {
-      const int p = lowest_bit(da & d1.a), r = lowest_bit(da & d2.a);
-      if (!((h.spres[p] >> r) & 1ull)) return 0.0;
-      double v = single_value_det(h, 0, p, r, d1.a, d1.b);
-      return sign_alpha(d1.a, d1.b, p, r) ? -v : v;
-    }
-    if (nb == 2) {
-      const int p = lowest_bit(db & d1.b), r = lowest_bit(db & d2.b);
-      if (!((h.spres[n + p] >> r) & 1ull)) return 0.0;
-      double v = single_value_det(h, 1, p, r, d1.a, d1.b);
-      return sign_beta(d1.a, d1.b, p, r) ? -v : v;
-    }
-    return 0.0;
-  }
-  if (na + nb == 4) {
+  double val;
+  if (single) {
+    const uint64_t stored = __ldg(h.spres + (beta1 ? n : 0) + p);
+    val = single_value_det(h, beta1 ? 1 : 0, p, r, d1.a, d1.b);
+    if (!((stored >> r) & 1ull)) return 0.0;
+  } else {
     const size_t np = static_cast<size_t>(h.npair);
-    if (na == 4) {
-      uint64_t o = da & d1.a, v = da & d2.a;
-      const int p = lowest_bit(o);
-      o &= o - 1;
-      const int q = lowest_bit(o);
-      const int r = lowest_bit(v);
-      v &= v - 1;
-      const int s = lowest_bit(v);
-      const double val = h.vss[static_cast<size_t>(pair_index(p, q)) * np + pair_index(r, s)];
-      return sign_aa(d1.a, d1.b, p, q, r, s) ? -val : val;
+    const double* at;
+    if (na == 2) {
+      q = lowest_bit(db & d1.b);
+      s = lowest_bit(db & d2.b);
+      at = h.wab + ((static_cast<size_t>(p) * n + q) * n + r) * n + s;
+    } else {
+      q = lowest_bit(o1 & (o1 - 1));
+      s = lowest_bit(v1 & (v1 - 1));
+      at = h.vss + ((beta1 ? np : 0) + pair_index(p, q)) * np + pair_index(r, s);
     }
-    if (nb == 4) {
-      uint64_t o = db & d1.b, v = db & d2.b;
-      const int p = lowest_bit(o);
-      o &= o - 1;
-      const int q = lowest_bit(o);
-      const int r = lowest_bit(v);
-      v &= v - 1;
-      const int s = lowest_bit(v);
-      const double val = h.vss[(np + pair_index(p, q)) * np + pair_index(r, s)];
-      return sign_bb(d1.a, d1.b, p, q, r, s) ? -val : val;
-    }
-    if (na == 2 && nb == 2) {
-      const int pa = lowest_bit(da & d1.a), ra = lowest_bit(da & d2.a);
-      const int pb = lowest_bit(db & d1.b), sb = lowest_bit(db & d2.b);
-      const double val = h.wab[((static_cast<size_t>(pa) * n + pb) * n + ra) * n + sb];
-      return sign_ab(d1.a, d1.b, pa, ra, pb, sb) ? -val : val;
-    }
+    val = __ldg(at);
   }
-  return 0.0;
+  uint64_t a = d1.a, b = d1.b;
+  unsigned neg = sign_one(beta1, a, b, p, r);
+  (beta1 ? b : a) ^= (1ull << p) ^ (1ull << r);
+  if (!single) neg ^= sign_one(beta2, a, b, q, s);
+  return neg ? -val : val;
 }
 
-// Diagonal element by one warp (lane-partial sums, fixed reduction order).
-// occ: 128-byte per-warp scratch.
-__device__ double diagonal_warp(const HamDev& h, Det d, unsigned char* occ) {
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = lanemask_lt();
-  int nocc = 0;
-  for (int j = 0; j < 4; ++j) {
-    const int s = lane + 32 * j;
+// Diagonal element of d by half a warp (16 lanes, the whole warp calling; d
+// may differ between the halves): <i|h|i> over the occupied i and <ij||ij>
+// over the occupied pairs i < j, row x of the pairs on lane x mod 16 with
+// eight loads in flight, then a fixed reduction order.  occ: 128 bytes of
+// scratch for each half.
+__device__ __forceinline__ double diagonal_half(const HamDev& h, Det d, unsigned char* occ) {
+  const int sub = threadIdx.x & 15;
+  const int nocc = __popcll(d.a) + __popcll(d.b);
+  // The occupied spin-orbitals in interleaved order, each at its rank.
+  for (int s = sub; s < h.nso; s += 16) {
     const int p = s >> 1;
-    const bool o = p < h.norb && ((((s & 1) ? d.b : d.a) >> p) & 1ull);
-    const unsigned m = __ballot_sync(~0u, o);
-    if (o) occ[nocc + __popc(m & lt)] = static_cast<unsigned char>(s);
-    nocc += __popc(m);
+    const uint64_t below = (1ull << p) - 1ull;
+    if ((((s & 1) ? d.b : d.a) >> p) & 1ull) {
+      const int rank = __popcll(d.a & below) + __popcll(d.b & below) + ((s & 1) ? static_cast<int>((d.a >> p) & 1ull) : 0);
+      occ[rank] = static_cast<unsigned char>(s);
+    }
   }
   __syncwarp();
-  // <i|h|i> over the occupied i and <ij||ij> over the occupied pairs i < j,
-  // the (i, j) terms spread over the lanes (independent loads).
   double v = 0.0;
-  for (int x = lane; x < nocc; x += 32) v += h.hdiag[occ[x]];
-  const int nn = nocc * nocc;
-#pragma unroll 4
-  for (int t = lane; t < nn; t += 32) {
-    const int x = t / nocc, y = t - x * nocc;
-    if (y > x) v += h.d2[static_cast<size_t>(occ[x]) * h.nso + occ[y]];
+#pragma unroll 1
+  for (int x = sub; x < nocc; x += 16) {
+    const double* row = h.d2 + static_cast<size_t>(occ[x]) * h.nso;
+    v += __ldg(h.hdiag + occ[x]);
+#pragma unroll 1
+    for (int y0 = x + 1; y0 < nocc; y0 += 8) {
+      double t[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) t[j] = y0 + j < nocc ? __ldg(row + occ[y0 + j]) : 0.0;
+      v += ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
+    }
   }
-  v = warp_sum(v);
+#pragma unroll
+  for (int o = 1; o < 16; o <<= 1) v += __shfl_xor_sync(~0u, v, o);
   __syncwarp();
-  return __shfl_sync(~0u, v, 0) + h.ecore;
+  return v + h.ecore;
 }
 
 // ---------------------------------------------------------------------------
@@ -151,10 +165,11 @@ __device__ double diagonal_warp(const HamDev& h, Det d, unsigned char* occ) {
 
 struct EigResult {
   dd xx, scale;
+  dd rq;              // the eigenvalue (Rayleigh quotient of the vector)
   int branch;
   bool ok;
   double resid;
-  double lambda;     // the eigenvalue (Rayleigh quotient of the vector)
+  double lambda;     // rq rounded
   double max_evec;   // max |v_i| over i >= 1 (branch 1) or i >= 0 (branch 2)
   int shift_steps;   // steps of the shifted solver, 0 when the reduction ran
   double shift_diff; // change made by its last refinement step
@@ -177,12 +192,16 @@ __host__ __device__ constexpr size_t eig_work_doubles(int k) {
 // (an upper bound of lambda_1: the current vector lies in the subspace, and
 // its Rayleigh quotient there is xz/xx) and the current vector as the start;
 // the reduction runs when that fails or its residual is not below 1e-11
-// (1 + |lambda|).  method 2: the bordered fixed point (eig_lowest_bordered)
-// runs first for k <= kBorderMaxK, the reduction when it does not certify its
-// result or the residual check fails.  The first iteration's problem (branch
-// 2, no bordering row) always takes the reduction.
-__device__ EigResult eig_update(const double* H, int k, const double* x, const double* z, dd xx, dd xz,
-                                double* dx, double* work, SectionClock& clk, double drop, int method) {
+// (1 + |lambda|).  Out of line, with the reduction itself: the usual update
+// takes eig_update_bordered, and its code should be what the instruction
+// cache holds.  x, z, dx and work are in shared memory.
+__device__ __noinline__ EigResult eig_update_full(const double* H, int k, const double* x, const double* z, dd xx,
+                                                  dd xz, double* dx, double* work, SectionClock& clk, double drop) {
+  // (a function of its own does not see where its callers' arrays are)
+  __builtin_assume(__isShared(x));
+  __builtin_assume(__isShared(z));
+  __builtin_assume(__isShared(dx));
+  __builtin_assume(__isShared(work));
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   __shared__ double s_b00, s_y1, s_res;
   __shared__ dd s_sum3[3];
@@ -306,21 +325,13 @@ __device__ EigResult eig_update(const double* H, int k, const double* x, const d
       __syncthreads();
     }
   }
-  bool bordered = false;
-  if (!shifted && method == 2 && branch == 1 && k <= kBorderMaxK) {
-    int iters = 0;
-    double rn = 0.0;
-    bordered = eig_lowest_bordered(A, lda, n, V, Li, &iters, &rn, clk);  // Li and Ci as its scratch
-    res.shift_steps = bordered ? iters : 0;
-    res.shift_diff = rn;
-    res.fallback = !bordered;
-  }
   clk.mark(16);
-  if (!shifted && !bordered) eig_lowest(Ae, lda, n, V, clk);
-  clk.mark(13);
-  shifted = shifted || bordered;  // a fast solve, checked below
 
+  bool reduce = !shifted;
+#pragma unroll 1
   for (int attempt = 0; attempt < 2; ++attempt) {
+  if (reduce) eig_lowest(Ae, lda, n, V, clk);
+  clk.mark(13);
   // B v in double, one row per warp (H is symmetric, so its rows are read).
   const double* y = V.y;
   for (int r = warp; r < n; r += kLW) {
@@ -390,6 +401,7 @@ __device__ EigResult eig_update(const double* H, int k, const double* x, const d
   // A shifted solve whose residual is not small runs the reduction instead.
   if (!shifted || s_res <= 1e-11 * (1.0 + fabs(dd_to_d(s_rq)))) break;
   shifted = false;
+  reduce = true;
   res.shift_steps = 0;
   res.shift_diff = 0.0;
   res.fallback = true;
@@ -399,7 +411,6 @@ __device__ EigResult eig_update(const double* H, int k, const double* x, const d
     A[i * lda] = bvec[i];
   }
   __syncthreads();
-  eig_lowest(Ae, lda, n, V, clk);
   }
   clk.mark(14);
   const dd rq = s_rq;
@@ -408,6 +419,7 @@ __device__ EigResult eig_update(const double* H, int k, const double* x, const d
   res.branch = branch;
   res.ok = true;
   res.lambda = lam;
+  res.rq = rq;
   {
     double mv = 0.0;
     if (warp == 0)
@@ -446,6 +458,410 @@ __device__ EigResult eig_update(const double* H, int k, const double* x, const d
 }
 
 // ---------------------------------------------------------------------------
+// The eig update by the bordered fixed point, for every k: the lowest
+// eigenpair of B = [[a, b'], [b, C]] (C = H, n = k + 1 rows) when it lies
+// below the Gershgorin bound of C, g = min_i (C_ii - sum_{j != i} |C_ij|).  By
+// Cauchy interlacing B has exactly one eigenvalue below lambda_1(C) >= g, so an
+// approximate eigenpair (lambda, v) with lambda + ||B v - lambda v|| / ||v|| < g
+// belongs to the lowest eigenvalue (some eigenvalue lies within the residual
+// norm of lambda).  With v = (1, y), D the diagonal of C and E the rest, the
+// last k rows of (B - lambda I) v = 0 read (D - lambda I) y = -(b + E y), and
+// the first row lambda = a + b'y.  A step is
+//     y <- -(b + E y) / (d - lambda),   lambda <- a + b'y,
+// which contracts by about max_i sum_j |E_ij| / (d_i - lambda), less than 1
+// whenever lambda < g (C is strongly diagonal in a subspace of picked
+// determinants, most of which are not connected by a single or double
+// excitation).  The product E y also gives the residual of the current
+// iterate, r_i = (b + E y)_i + (d_i - lambda) y_i (row 0's is zero by the choice
+// of lambda).  The start is the current vector, y = x / y1, which is within
+// the update itself of the solution.  The reciprocal of d_i - lambda is a
+// Newton-Raphson step from the last one, r <- r + r e with e = 1 - (d_i -
+// lambda) r, while |e| < 1e-3, and a division otherwise; an inexact r changes
+// only the step, not the fixed point.  The iteration stops when ||r|| / ||v||
+// reaches 1e-15 max_i sum_j |B_ij| (or stalls within 16 times that), and gives
+// up when it stops contracting or lambda is not below g.
+//
+// Bound by the latency of a step's chain.  One warp issues a shared-memory load
+// about every ten cycles and a shuffle every six, so the row products are
+// spread: row i of E is held in registers by four lanes (NJ values each), and
+// ceil(k/8) warps take part.  A step has one named barrier, after the new y is
+// in shared memory (two buffers in turn); then every warp forms b'y over all
+// rows itself, from one load per 32 rows, beside the product for the step
+// after.  The residual is tested at every second step, from successive y
+// (r = (d - lambda) (y_t - y_{t+1}) but for the error of the reciprocal, at
+// most 1e-3); the one that certifies is taken from the exact r.
+// Cycles per step at k = 32: one warp over packed nonzeros 1,500; a row per
+// lane and y read uniformly 1,340; four lanes per row with per-warp sums of
+// b'y, rr and yy exchanged at every step 900; this form 700.
+//
+// With y_0 = 1 the update's formulas (src/solver.h:516-538: gamma = v_0 / y1,
+// scale = gamma sqrt(-rq), xx = -rq / scale^2, dx_i = v_{i+1} / gamma - x_i,
+// for the normalised v) become dx_i = y_i y1 - x_i, xx = |v|^2 y1^2 and
+// scale = sqrt(-rq / xx), with rq = v'Bv / v'v; |v|^2 and v'Bv are summed in
+// double-double, the rows of B v taken from the last step's products.
+
+constexpr int kBorderIters = 64;
+
+constexpr int kBorderWarps = kMaxK / 8;
+
+struct BorderShared {
+  double y[2][kMaxK];
+  double b[kMaxK], d[kMaxK];
+  double part[kBorderWarps][4];
+  dd vv[kBorderWarps], vbv[kBorderWarps];  // (vv holds x'Hx before)
+  dd xtx, xtz;
+  double ymax[kBorderWarps];
+  double lam, y1, resid;
+  int ok, steps;
+};
+
+// Two double-double sums over the lanes whose numbers differ in the bits
+// from `first` up to, not including, `last`, side by side: the high parts by
+// exact two-sums, their errors and the low parts in one running sum, put
+// together at the end (half the chain of normalised additions; the low sum's
+// own rounding is 2^-53 of it).
+__device__ __forceinline__ void lanes_sum_dd(dd& v, dd& w, int first, int last) {
+#pragma unroll 1
+  for (int o = first; o < last; o <<= 1) {
+    const dd v2{__shfl_xor_sync(~0u, v.hi, o), __shfl_xor_sync(~0u, v.lo, o)};
+    const dd w2{__shfl_xor_sync(~0u, w.hi, o), __shfl_xor_sync(~0u, w.lo, o)};
+    const dd vs = dd_two_sum(v.hi, v2.hi), ws = dd_two_sum(w.hi, w2.hi);
+    v = dd{vs.hi, (v.lo + v2.lo) + vs.lo};
+    w = dd{ws.hi, (w.lo + w2.lo) + ws.lo};
+  }
+  v = dd_fast_two_sum(v.hi, v.lo);
+  w = dd_fast_two_sum(w.hi, w.lo);
+}
+
+// x'x and x'z by one warp.
+__device__ __forceinline__ void dots_dd(const double* x, const double* z, int k, dd& xtx, dd& xtz) {
+  xtx = xtz = dd{0.0, 0.0};
+#pragma unroll 1
+  for (int i = threadIdx.x & 31; i < k; i += 32) {
+    xtx = dd_add(xtx, dd_two_prod(x[i], x[i]));
+    xtz = dd_add(xtz, dd_two_prod(x[i], z[i]));
+  }
+  lanes_sum_dd(xtx, xtz, 1, 32);
+}
+
+// A sum over the rows of a warp (a row's four lanes hold the same value).
+__device__ __forceinline__ double rows_sum(double v) {
+  v += __shfl_xor_sync(~0u, v, 4);
+  v += __shfl_xor_sync(~0u, v, 8);
+  return v + __shfl_xor_sync(~0u, v, 16);
+}
+
+// The sum of the four lanes of a row.
+__device__ __forceinline__ double quad_sum(double v) {
+  v += __shfl_xor_sync(~0u, v, 1);
+  return v + __shfl_xor_sync(~0u, v, 2);
+}
+
+// Threads [0, 32 ceil(k/8)), k <= 4 NJ.  S.xtx and S.xtz hold x'x and x'z.
+// Leaves dx, the partial sums for bordered_scalars and S.ok: 1, 0 when the
+// pair is not certified, -1 when its eigenvalue is not negative.
+template <int NJ>
+__device__ __forceinline__ void eig_bordered(BorderShared& S, const double* H, int k, const double* x, const double* z,
+                                             dd xx, dd xz, double* dx) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int row = tid >> 2, q = tid & 3;
+  const int nw = (k + 7) >> 3, T = 32 * nw;
+  const bool own = row < k;
+  // Columns q, q + 4, ...; H is symmetric: element (j, row) of row-major H.
+  double e[NJ], d = 0.0, off = 0.0, hx = 0.0;
+#pragma unroll
+  for (int jj = 0; jj < NJ; ++jj) {
+    const int j = q + 4 * jj;
+    const double v = own && j < k ? H[static_cast<size_t>(j) * k + row] : 0.0;
+    hx = fma(v, j < k ? x[j] : 0.0, hx);
+    if (j == row) d = v;
+    e[jj] = j == row ? 0.0 : v;
+    off += fabs(e[jj]);
+  }
+  for (int i = tid; i < 2 * kMaxK; i += T) (&S.y[0][0])[i] = 0.0;  // rows that no thread has stay zero
+  d = quad_sum(d);
+  off = quad_sum(off);
+  hx = quad_sum(hx);
+  const double xi = own ? x[row] : 0.0;
+  {
+    dd part = dd_two_prod(xi, hx), none{0.0, 0.0};
+    lanes_sum_dd(part, none, 4, 32);
+    if (lane == 0) S.vv[warp] = part;
+  }
+  bar_named(1, T);
+  // x'Hx, |rest|^2 and B's first row; x'Hx, x'z and x'x rounded to double
+  // where the reference works in double.
+  dd sum = lane < nw ? S.vv[lane] : dd{0.0, 0.0}, none{0.0, 0.0};
+  lanes_sum_dd(sum, none, 1, nw);
+  const double xtx = dd_to_d(S.xtx), xtz = dd_to_d(S.xtz);
+  const double xthx = __shfl_sync(~0u, dd_to_d(sum), 0);
+  const double yy0 = dd_to_d(dd_add_d(xx, -xtx));
+  if (!(yy0 > 1e-14)) {  // no rest vector to border with
+    if (tid == 0) S.ok = 0;
+    return;
+  }
+  const double y1 = sqrt(yy0);
+  // The quotient of a double-double and a double, rounded once: a double
+  // quotient and its remainder.
+  const dd num = dd_add_d(dd_add_d(xz, -2.0 * xtz), xthx);
+  const double q0 = num.hi / yy0;
+  const double a = q0 + (fma(-q0, yy0, num.hi) + num.lo) / yy0;
+  const double b = own ? (z[row] - hx) / y1 : 0.0;
+
+  // The start, and the sums and bounds over all rows that the tests need.
+  double y = own ? xi / y1 : 0.0;
+  double gl = own ? d - off : 1e300, nb = own ? fabs(d) + off + fabs(b) : 0.0;
+  {
+    const double by = rows_sum(b * y), babs = rows_sum(fabs(b));
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+      const double g2 = __shfl_xor_sync(~0u, gl, o), n2 = __shfl_xor_sync(~0u, nb, o);
+      gl = g2 < gl ? g2 : gl;
+      nb = n2 > nb ? n2 : nb;
+    }
+    if (lane == 0) {
+      S.part[warp][0] = by;
+      S.part[warp][1] = babs;
+      S.part[warp][2] = gl;
+      S.part[warp][3] = nb;
+    }
+    if (q == 0) {
+      S.y[0][row] = y;
+      S.b[row] = b;
+      S.d[row] = d;
+    }
+  }
+  bar_named(1, T);
+  double babs = 0.0, lam = a;
+  gl = 1e300;
+  nb = 0.0;
+#pragma unroll 1
+  for (int w = 0; w < nw; ++w) {
+    lam += S.part[w][0];
+    babs += S.part[w][1];
+    const double g2 = S.part[w][2], n2 = S.part[w][3];
+    gl = g2 < gl ? g2 : gl;
+    nb = n2 > nb ? n2 : nb;
+  }
+  const double top = fabs(a) + babs, tol = 1e-15 * (nb > top ? nb : top), tol2 = tol * tol;
+  const bool cold = !(lam < gl);
+  if (cold) {  // a start from below instead; lambda is then not yet a + b'y
+    bar_named(1, T);
+    y = 0.0;
+    if (q == 0) S.y[0][row] = 0.0;
+    lam = (a < gl ? a : gl) - 1e-3 * (1.0 + fabs(a));
+    bar_named(1, T);
+  }
+  // Rows lane, lane + 32, ... for the sums over all rows.
+  constexpr int R = NJ <= 8 ? 1 : NJ / 8;
+  double bl[R], dl[R], yl[R];
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int j = lane + 32 * i;
+    bl[i] = j < k ? S.b[j] : 0.0;
+    dl[i] = j < k ? S.d[j] : 0.0;
+    yl[i] = j < k ? S.y[0][j] : 0.0;
+  }
+  // E y over this thread's columns, then the row.
+  auto product = [&](int buf) {
+    const double* ys = S.y[buf] + q;
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int jj = 0; jj < NJ; jj += 2) {
+      s0 = fma(e[jj], ys[4 * jj], s0);
+      s1 = fma(e[jj + 1], ys[4 * jj + 4], s1);
+    }
+    return b + quad_sum(s0 + s1);
+  };
+  double rcp = own ? 1.0 / (d - lam) : 0.0;
+  double rrp = 1e300, vvp = 1.0;  // |r|^2 and |v|^2 at the previous test
+  double s = product(0);
+  int done = 0, t = 0;
+  // y_t -> y_{t+1}: s, lambda and the reciprocal follow; with `test`, whether
+  // (lambda_t, y_t) ends the iteration (1 converged, -1 given up), before
+  // anything of it is replaced.
+  auto step = [&](int buf, bool test) {
+    const double yn = -s * rcp;  // rows beyond k: rcp = 0
+    if (q == 0) S.y[buf ^ 1][row] = yn;
+    bar_named(1, T);
+    double by = 0.0, rr = 0.0, vv = 0.0, yn_l[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      yn_l[i] = lane + 32 * i < k ? S.y[buf ^ 1][lane + 32 * i] : 0.0;
+      by = fma(bl[i], yn_l[i], by);
+      const double ri = (dl[i] - lam) * (yl[i] - yn_l[i]);
+      rr = fma(ri, ri, rr);
+      vv = fma(yl[i], yl[i], vv);
+    }
+    const double sn = product(buf ^ 1);
+    by = warp_sum(by);
+    if (test) {
+      rr = warp_sum(rr);
+      vv = 1.0 + warp_sum(vv);
+      // rn <= tol, or rn > rn_prev / 4 (two steps before) and rn <= 16 tol
+      // (stalled at rounding); squared norms cross-multiplied, no division
+      const bool small = rr <= tol2 * vv || (t >= 2 && rr * vvp > 0.0625 * rrp * vv && rr <= 256.0 * tol2 * vv);
+      if (small && !(cold && t == 0)) {
+        done = 1;
+        return;
+      }
+      // not finite, not contracting (rn > 0.8 rn_prev), or lambda not below g
+      if (!(rr < 1e290 && vv < 1e290) || (t >= 8 && rr * vvp > 0.64 * rrp * vv) || (t >= 4 && !(lam < gl))) {
+        done = -1;
+        return;
+      }
+      rrp = rr;
+      vvp = vv;
+    }
+    y = yn;
+    s = sn;
+    lam = a + by;
+#pragma unroll
+    for (int i = 0; i < R; ++i) yl[i] = yn_l[i];
+    const double den = d - lam, err = fma(-den, rcp, 1.0);  // relative error of rcp as 1 / den
+    if (__any_sync(~0u, own && fabs(err) >= 1e-3))
+      rcp = own ? 1.0 / den : 0.0;
+    else
+      rcp = fma(rcp, err, rcp);
+  };
+#pragma unroll 1
+  for (; t < kBorderIters; t += 2) {
+    step(0, true);
+    if (done != 0) break;
+    step(1, false);
+  }
+  int ok = 0;
+  double rn = 0.0;
+  if (done == 1) {  // (uniform over the threads: all sums are formed the same way)
+    const double ri = own && q == 0 ? fma(d - lam, y, s) : 0.0, yi = q == 0 ? y : 0.0;
+    const double rr = rows_sum(quad_sum(ri * ri)), vv = rows_sum(quad_sum(yi * yi));
+    if (lane == 0) {
+      S.part[warp][0] = rr;
+      S.part[warp][1] = vv;
+    }
+    bar_named(1, T);
+    double rrs = 0.0, vvs = 1.0;
+#pragma unroll 1
+    for (int w = 0; w < nw; ++w) {
+      rrs += S.part[w][0];
+      vvs += S.part[w][1];
+    }
+    rn = sqrt(rrs / vvs);
+    // (the exact residual may be a little above what the test saw)
+    ok = rn <= 32.0 * tol && lam + rn < gl ? 1 : 0;
+  }
+  if (!ok) {
+    if (tid == 0) S.ok = 0;
+    return;
+  }
+  // dx, and |v|^2 and v'Bv over the rows; row 0 of B v is lambda.
+  if (own && q == 0) dx[row] = dd_to_d(dd_add_d(dd_two_prod(y, y1), -xi));
+  dd vv = dd_two_prod(y, y), vbv = dd_two_prod(y, own ? fma(d, y, s) : 0.0);
+  lanes_sum_dd(vv, vbv, 4, 32);
+  double ym = fabs(y);
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) {
+    const double m2 = __shfl_xor_sync(~0u, ym, o);
+    ym = m2 > ym ? m2 : ym;
+  }
+  if (lane == 0) {
+    S.vv[warp] = vv;
+    S.vbv[warp] = vbv;
+    S.ymax[warp] = ym;
+  }
+  if (tid == 0) {
+    S.ok = lam < 0.0 ? 1 : -1;
+    S.steps = t + 1;
+    S.resid = rn;
+    S.lam = lam;
+    S.y1 = y1;
+  }
+}
+
+// The update's scalars from what eig_bordered left in S, by one warp, after a
+// barrier: lane 0 returns them.
+__device__ __forceinline__ EigResult bordered_scalars(const BorderShared& S, int k) {
+  const int lane = threadIdx.x & 31, nw = (k + 7) >> 3;
+  dd vv = lane < nw ? S.vv[lane] : dd{0.0, 0.0}, vbv = lane < nw ? S.vbv[lane] : dd{0.0, 0.0};
+  lanes_sum_dd(vv, vbv, 1, nw < 2 ? 2 : nw);  // lanes 0 and 1 both
+  double ym = 0.0;
+#pragma unroll 1
+  for (int w = 0; w < nw; ++w) ym = S.ymax[w] > ym ? S.ymax[w] : ym;
+  const dd nrm = dd_add_d(vv, 1.0), num = dd_add_d(vbv, S.lam);
+  const dd nxx = dd_mul(nrm, dd_two_prod(S.y1, S.y1));
+  // Lane 0: rq = num / nrm.  Lane 1: the root of -rq / xx = -num / (nrm xx).
+  const dd quo = dd_div(lane == 0 ? num : dd_neg(num), lane == 0 ? nrm : dd_mul(nrm, nxx));
+  const dd root = dd_sqrt(dd_abs(quo));
+  EigResult r;
+  r.xx = nxx;
+  r.scale = dd{__shfl_sync(~0u, root.hi, 1), __shfl_sync(~0u, root.lo, 1)};
+  r.rq = quo;
+  r.lambda = dd_to_d(quo);
+  r.branch = 1;
+  r.ok = true;
+  r.resid = S.resid;
+  r.max_evec = ym * rsqrt(nrm.hi);
+  r.shift_steps = S.steps;
+  r.shift_diff = S.resid;
+  r.fallback = false;
+  return r;
+}
+
+// The bordered update of a whole CTA; S.xtx and S.xtz are set, after a
+// barrier.  Returns S.ok, in every thread.
+__device__ __forceinline__ int eig_update_bordered(BorderShared& S, const double* H, int k, const double* x,
+                                                   const double* z, dd xx, dd xz, double* dx) {
+  if (static_cast<int>(threadIdx.x >> 5) < (k + 7) >> 3) {
+    if (k <= 16)
+      eig_bordered<4>(S, H, k, x, z, xx, xz, dx);
+    else if (k <= 32)
+      eig_bordered<8>(S, H, k, x, z, xx, xz, dx);
+    else if (k <= 64)
+      eig_bordered<16>(S, H, k, x, z, xx, xz, dx);
+    else
+      eig_bordered<32>(S, H, k, x, z, xx, xz, dx);
+  }
+  __syncthreads();
+  return S.ok;
+}
+
+// The eig update on its own (the debug entry points): the bordered fixed
+// point first with method 2, eig_update_full otherwise or when it does not
+// certify its result (and for the first iteration, which has no bordering
+// row).  Block-wide; every thread gets the result.
+__device__ __forceinline__ EigResult eig_update(const double* H, int k, const double* x, const double* z, dd xx, dd xz,
+                                                double* dx, double* work, SectionClock& clk, double drop, int method) {
+  __shared__ BorderShared S;
+  __shared__ EigResult s_res;
+  bool tried = false;
+  if (method == 2) {
+    if (threadIdx.x < 32) {
+      dd xtx, xtz;
+      dots_dd(x, z, k, xtx, xtz);
+      if (threadIdx.x == 0) {
+        S.xtx = xtx;
+        S.xtz = xtz;
+      }
+    }
+    __syncthreads();
+    const int ok = eig_update_bordered(S, H, k, x, z, xx, xz, dx);
+    if (ok != 0) {
+      if (threadIdx.x < 32) {
+        EigResult r = bordered_scalars(S, k);
+        r.ok = ok > 0;
+        if (threadIdx.x == 0) s_res = r;
+      }
+      __syncthreads();
+      return s_res;
+    }
+    tried = true;
+  }
+  EigResult res = eig_update_full(H, k, x, z, xx, xz, dx, work, clk, drop);
+  if (tried && res.branch == 1) res.fallback = true;
+  return res;
+}
+
+// ---------------------------------------------------------------------------
 // End of iteration t (src/wavefunction.h:557-565,583): z[D_c] = new_z_c for
 // the picked determinants, then xz += sum_c dot_c.  Block-wide, on a state
 // copy `S` (shared or global); table stores go to global memory.
@@ -480,167 +896,68 @@ __device__ __forceinline__ unsigned hash32(unsigned x) {
   return x;
 }
 
-// Block-wide exclusive position of a kept element within one chunk of
-// blockDim.x elements; returns the chunk's kept count through *chunk_total.
-__device__ __forceinline__ int block_rank(bool keep, int* wsum, int* chunk_total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned b = __ballot_sync(~0u, keep);
-  if (lane == 0) wsum[warp] = __popc(b);
-  __syncthreads();
-  if (warp == 0) {
-    const int v = lane < static_cast<int>(blockDim.x >> 5) ? wsum[lane] : 0;
-    int incl = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(~0u, incl, o);
-      if (lane >= o) incl += t;
-    }
-    wsum[lane] = incl - v;  // exclusive
-    if (lane == 31) wsum[32] = incl;
+// The candidates of one iteration, in dynamic shared memory: the slots of up
+// to PR candidates (kNoSlot for one seen before), and a hash set of 2 PR words
+// that the candidates' keys replace once it has served.
+struct Candidates {
+  unsigned* slot;
+  unsigned* set;
+  unsigned long long* key;
+  int n;   // entries in use
+  int pr;  // a power of two
+};
+
+// Full sort by decreasing key, equal keys in the reference's determinant
+// order (rare: the k-th and (k+1)-th keys are equal); the first k slots to out.
+__device__ __noinline__ void sort_candidates(const Candidates& C, int k, const Slot* slots, int nwords, unsigned* out) {
+  int P = 1;
+  while (P < C.n) P <<= 1;
+  for (int u = C.n + threadIdx.x; u < P; u += kLT) {
+    C.key[u] = 0ull;
+    C.slot[u] = kNoSlot;
   }
   __syncthreads();
-  const int pos = wsum[warp] + __popc(b & lanemask_lt());
-  *chunk_total = wsum[32];
-  __syncthreads();
-  return pos;
-}
-
-constexpr unsigned kNoSlot = 0xFFFFFFFFu;
-
-// The k best (score, slot) pairs among n candidates (us, sc in shared
-// memory) by radix selection on the 64-bit keys bits(score) + 1: scores are
-// +0 or positive, so their bit patterns order like their values.  Eight-bit
-// digits from the top, one 256-bin shared histogram per pass (warp-aggregated
-// counts: the leading digits of nearby scores coincide), until the bin that
-// holds the k-th largest key holds exactly the keys still to choose.  The
-// chosen keys are then ranked among themselves, in decreasing score and equal
-// scores in the reference's determinant order (detComp_global,
-// src/wavefunction.h:30-36), and their slots written to out[0..k) in that
-// order.  Returns false, writing nothing, when the k-th and (k+1)-th keys are
-// equal, so that the caller can choose the set by determinant order.
-__device__ bool topk_radix(const unsigned* us, const double* sc, int n, int k, const Slot* slots, int nwords,
-                           unsigned* out) {
-  __shared__ unsigned s_hist[256];
-  __shared__ unsigned long long s_sel_key[kMaxK];
-  __shared__ unsigned s_sel_slot[kMaxK];
-  __shared__ unsigned long long s_prefix;
-  __shared__ unsigned s_need;
-  __shared__ int s_state, s_count;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < 256) s_hist[tid] = 0u;
-  if (tid == 0) {
-    s_need = static_cast<unsigned>(k);
-    s_count = 0;
-    s_state = 0;
-    s_prefix = 0ull;
-  }
-  __syncthreads();
-  unsigned long long prefix = 0ull;  // the digits chosen so far, lower bits 0
-  int state = 0;                     // 0 more digits, 1 set found, 2 tie at the k-th key
-  for (int pass = 0; pass < 8 && state == 0; ++pass) {
-    const int shift = 56 - 8 * pass;
-    const unsigned long long himask = pass == 0 ? 0ull : (~0ull << (shift + 8));
-    for (int base = warp * 32; base < n; base += blockDim.x) {
-      const int u = base + lane;
-      const unsigned long long key =
-          u < n ? static_cast<unsigned long long>(__double_as_longlong(sc[u])) + 1ull : 0ull;
-      const bool match = u < n && ((key ^ prefix) & himask) == 0ull;
-      const unsigned act = __ballot_sync(~0u, match);
-      if (match) {
-        const unsigned d = static_cast<unsigned>(key >> shift) & 255u;
-        const unsigned peers = __match_any_sync(act, d);
-        if (lane == __ffs(peers) - 1) atomicAdd(&s_hist[d], static_cast<unsigned>(__popc(peers)));
-      }
-    }
-    __syncthreads();
-    if (warp == 0) {
-      // Lane l holds bins 255-8l .. 248-8l, in decreasing order.
-      const unsigned need = s_need;
-      unsigned c[8], t = 0u;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        c[j] = s_hist[255 - 8 * lane - j];
-        s_hist[255 - 8 * lane - j] = 0u;
-        t += c[j];
-      }
-      unsigned incl = t;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned v = __shfl_up_sync(~0u, incl, o);
-        if (lane >= o) incl += v;
-      }
-      unsigned run = incl - t;  // keys in higher bins
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (run < need && run + c[j] >= need) {
-          const unsigned long long d = static_cast<unsigned long long>(255 - 8 * lane - j);
-          s_prefix = prefix | (d << shift);
-          s_need = need - run;
-          s_state = (c[j] == need - run) ? 1 : (pass == 7 ? 2 : 0);
+  for (int size = 2; size <= P; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int t = threadIdx.x; t < (P >> 1); t += kLT) {
+        const int i = 2 * stride * (t / stride) + (t % stride);
+        const int j = i + stride;
+        const unsigned long long ki = C.key[i], kj = C.key[j];
+        bool jfirst = kj > ki;
+        if (ki == kj && ki != 0ull) {
+          uint64_t ia, ib, ja, jb;
+          load_key(slots + C.slot[i], ia, ib);
+          load_key(slots + C.slot[j], ja, jb);
+          jfirst = det_ref_compare(ja, jb, ia, ib, nwords) > 0;
         }
-        run += c[j];
+        const bool up = (i & size) == 0;
+        if (jfirst == up && (ki != kj || ki != 0ull)) {
+          C.key[i] = kj;
+          C.key[j] = ki;
+          const unsigned tmp = C.slot[i];
+          C.slot[i] = C.slot[j];
+          C.slot[j] = tmp;
+        }
       }
-    }
-    __syncthreads();
-    prefix = s_prefix;
-    state = s_state;
-  }
-  if (state != 1) return false;
-  // The chosen keys are those >= prefix: exactly k of them.
-  for (int base = warp * 32; base < n; base += blockDim.x) {
-    const int u = base + lane;
-    const unsigned long long key =
-        u < n ? static_cast<unsigned long long>(__double_as_longlong(sc[u])) + 1ull : 0ull;
-    const bool keep = u < n && key >= prefix;
-    const unsigned b = __ballot_sync(~0u, keep);
-    if (b == 0u) continue;
-    int pos = 0;
-    if (lane == 0) pos = atomicAdd(&s_count, __popc(b));
-    pos = __shfl_sync(~0u, pos, 0) + __popc(b & lanemask_lt());
-    if (keep) {
-      s_sel_key[pos] = key;
-      s_sel_slot[pos] = us[u];
+      __syncthreads();
     }
   }
+  if (threadIdx.x < k) out[threadIdx.x] = C.slot[threadIdx.x];
   __syncthreads();
-  if (tid < k) {
-    const unsigned long long mine = s_sel_key[tid];
-    const unsigned slot = s_sel_slot[tid];
-    int rank = 0;
-    bool equal = false;
-    for (int j = 0; j < k; ++j) {
-      const unsigned long long o = s_sel_key[j];
-      rank += o > mine;
-      equal |= (o == mine) && j != tid;
-    }
-    if (equal) {  // equal scores: the reference's determinant order
-      uint64_t ia, ib;
-      load_key(slots + slot, ia, ib);
-      for (int j = 0; j < k; ++j) {
-        if (j == tid || s_sel_key[j] != mine) continue;
-        uint64_t ja, jb;
-        load_key(slots + s_sel_slot[j], ja, jb);
-        rank += det_ref_compare(ja, jb, ia, ib, nwords) > 0;
-      }
-    }
-    out[rank] = slot;
-  }
-  __syncthreads();
-  return true;
 }
-
 
 __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ __align__(16) IterState sS;
-  __shared__ int s_off[kMaxK + 1];
-  __shared__ int s_wsum[33];
-  __shared__ int s_R, s_U;
-  __shared__ unsigned s_err;
-  __shared__ unsigned s_slot[kMaxK];
+  __shared__ __align__(16) IterState sS;  // the scalars; the per-column arrays stay in global memory
+  __shared__ SelectScratch s_sel;
+  __shared__ unsigned s_err, s_out, s_newx;
+  __shared__ dd s_xz;
+  __shared__ unsigned s_slot[kMaxK], s_sel_slot[kMaxK];
+  __shared__ unsigned long long s_sel_key[kMaxK];
   __shared__ Det s_det[kMaxK];
   __shared__ double s_x[kMaxK], s_z[kMaxK], s_dx[kMaxK];
-  __shared__ unsigned char s_occ[kLW][128];
-  __shared__ unsigned long long s_newx;
+  __shared__ unsigned char s_occ[2 * kLW][128];
+  __shared__ BorderShared s_border;
 
   IterState* G = L.st;
   const TableDev& T = L.tab;
@@ -649,214 +966,173 @@ __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
   SectionClock clk{L.sect, 0};
   clk.start();
 
-  // 0. Iteration state into shared memory.
+  Candidates C;
+  C.pr = 4;
+  while (C.pr < L.k_req * m) C.pr <<= 1;
+  C.slot = reinterpret_cast<unsigned*>(smem);
+  C.set = C.slot + C.pr;
+  C.key = reinterpret_cast<unsigned long long*>(C.set);
+  for (int i = tid; i < C.pr / 2; i += kLT)
+    reinterpret_cast<uint4*>(C.set)[i] = make_uint4(kNoSlot, kNoSlot, kNoSlot, kNoSlot);
+  if (tid == 0) s_out = s_newx = 0u;
+
+  // 1. The scalars into shared memory, and the end of the previous iteration
+  //    (src/wavefunction.h:557-565,583; unless finish_kernel already did):
+  //    z[D_c] = new_z_c for the picked determinants, xz += sum_c dot_c.
+  const int kprev = __ldcg(&G->k_cur);
+  const int pending = __ldcg(&G->pending);
+  unsigned cand[4];  // the first candidates, whatever kprev is
+#pragma unroll
+  for (int j = 0; j < 4; ++j) cand[j] = tid + j * kLT < L.k_req * m ? __ldcg(L.cand_slot + tid + j * kLT) : kNoSlot;
   {
+    constexpr int kHead = offsetof(IterState, k_cur) / 8, kTail = offsetof(IterState, x_size) / 8;
+    constexpr int kWords = sizeof(IterState) / 8;
     const unsigned long long* src = reinterpret_cast<const unsigned long long*>(G);
     unsigned long long* dst = reinterpret_cast<unsigned long long*>(&sS);
-    for (int i = tid; i < static_cast<int>(sizeof(IterState) / 8); i += kLT) dst[i] = src[i];
+    const int i = tid < kHead ? tid : kTail + tid - kHead;
+    if (i < kWords) dst[i] = src[i];
   }
-  if (tid == 0) {
+  if (tid == kLT - 1) {
     s_err = *reinterpret_cast<volatile unsigned*>(T.err);
     if (*T.n_occupied > L.st->occupancy_limit) {
       atomicOr(T.err, kErrOverflow);
       s_err |= kErrOverflow;
     }
-    s_newx = 0;
   }
+  if (pending && tid < kprev) T.slots[__ldcg(&G->slot[tid])].z = __ldcg(&G->newz[tid]);
+  C.n = kprev * m;
   __syncthreads();
   clk.mark(0);
 
-  // 1. Finish the previous iteration (unless finish_kernel already did).
-  const int kprev = sS.k_cur;
-  finish_iteration(&sS, T);
-  if (warp == 0) {
-    int run = 0;
-    for (int base = 0; base < kMaxK; base += 32) {
-      const int cc = (base + lane < kprev) ? sS.cand_n[base + lane] : 0;
-      int incl = cc;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(~0u, incl, o);
-        if (lane >= o) incl += t;
-      }
-      s_off[base + lane] = run + incl - cc;
-      run += __shfl_sync(~0u, incl, 31);
+  // 2. Candidate slots, with duplicates (one determinant in several columns)
+  //    removed through a shared-memory hash set: the first copy stays.
+  if (warp == kLW - 1) {
+    dd acc{0.0, 0.0}, none{0.0, 0.0};
+    if (pending)
+      for (int c = lane; c < kprev; c += 32) acc = dd_add_d(acc, __ldcg(&G->dot[c]));
+    lanes_sum_dd(acc, none, 1, 32);
+    if (lane == 0) s_xz = dd_add(sS.xz, acc);
+  }
+#pragma unroll 1
+  for (int r0 = tid; r0 < C.n; r0 += 4 * kLT) {
+    if (r0 != tid) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) cand[j] = r0 + j * kLT < C.n ? __ldcg(L.cand_slot + r0 + j * kLT) : kNoSlot;
     }
-    if (lane == 0) {
-      s_off[kMaxK] = run;
-      s_R = run;
+    const unsigned mask = static_cast<unsigned>(2 * C.pr - 1);
+    unsigned old[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (r0 + j * kLT >= C.n) cand[j] = kNoSlot;
+      old[j] = kNoSlot;
+      if (cand[j] != kNoSlot) old[j] = atomicCAS(&C.set[hash32(cand[j]) & mask], kNoSlot, cand[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      unsigned h = hash32(cand[j]);
+#pragma unroll 1
+      while (old[j] != kNoSlot && old[j] != cand[j]) old[j] = atomicCAS(&C.set[++h & mask], kNoSlot, cand[j]);
+      if (r0 + j * kLT < C.n) C.slot[r0 + j * kLT] = old[j] == kNoSlot ? cand[j] : kNoSlot;
     }
   }
   __syncthreads();
   clk.mark(1);
-  if (s_err != 0u || s_R == 0) {
+
+  // 3. Their scores |x*xx*scale^2 + z|, refetched from the table
+  //    (src/wavefunction.h:567-575), and the k largest by radix selection.
+  {
+    const dd xss = sS.xss;
+#pragma unroll 1
+    for (int r0 = tid; r0 < C.n; r0 += 4 * kLT) {
+      double x[4], z[4];
+      bool some[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const unsigned s = r0 + j * kLT < C.n ? C.slot[r0 + j * kLT] : kNoSlot;
+        some[j] = s != kNoSlot;
+        x[j] = z[j] = 0.0;
+        if (some[j]) load_xz(T.slots + s, x[j], z[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const double g = score_of(x[j], z[j], xss);
+        // (a non-finite gradient must not reorder the rest)
+        if (r0 + j * kLT < C.n) C.key[r0 + j * kLT] = some[j] ? score_key(g >= 0.0 ? g : 0.0) : 0ull;
+      }
+    }
+  }
+  __syncthreads();
+  clk.mark(2);
+  const SelectEdge E = select_edge(s_sel, static_cast<unsigned>(L.k_req), [&](auto f) {
+#pragma unroll 1
+    for (int r0 = tid; r0 < C.n; r0 += 4 * kLT) {
+      unsigned long long key[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) key[j] = r0 + j * kLT < C.n ? C.key[r0 + j * kLT] : 0ull;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) f(key[j]);
+    }
+  });
+  if (s_err != 0u || E.total == 0u) {
     if (tid == 0) {
-      if (s_R == 0 && s_err == 0u) atomicOr(T.err, kErrCandidates);
-      G->xz = sS.xz;
+      if (E.total == 0u && s_err == 0u) atomicOr(T.err, kErrCandidates);
+      G->xz = s_xz;
       G->pending = 0;
       G->k_cur = 0;
     }
     return;
   }
+  const int k = static_cast<int>(min(E.total, static_cast<unsigned>(L.k_req)));
 
-  // 2-3. Candidate slots, with duplicates (one determinant in several
-  //      columns) removed through a shared-memory hash set, and their scores
-  //      |x*xx*scale^2 + z| refetched from the table.
-  const int R = s_R;
-  int PR = 2;  // >= 2 keeps the score array (which reuses the hash set) 8-byte aligned
-  while (PR < R) PR <<= 1;
-  unsigned* us = reinterpret_cast<unsigned*>(smem);  // [PR] slots, compacted in place
-  unsigned* hs = us + PR;                             // [2*PR] hash set; then scores (double[PR])
-  double* sc = reinterpret_cast<double*>(hs);
-  const int H = 2 * PR;
-  const dd xss = sS.xss;
-  auto slot_of = [&](int r) {  // candidate r: s_off[lo] <= r < s_off[lo+1]
-    int lo = 0, hi = kprev;
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (s_off[mid] <= r) lo = mid; else hi = mid;
-    }
-    return L.cand_slot[lo * m + (r - s_off[lo])];
-  };
-  auto score_at = [&](unsigned slot) {
-    const Slot* sp = T.slots + slot;
-    const double x = load_relaxed(&sp->x), z = load_relaxed(&sp->z);
-    const double g = score_of(x, z, xss);
-    return (g >= 0.0) ? g : 0.0;  // a non-finite gradient must not reorder the padding
-  };
-  auto hash_keep = [&](unsigned s) {  // true for the first copy of slot s
-    unsigned h = hash32(s) & static_cast<unsigned>(H - 1);
-    for (int probe = 0; probe < H; ++probe) {
-      const unsigned old = atomicCAS(&hs[h], kNoSlot, s);
-      if (old == kNoSlot) return true;
-      if (old == s) return false;
-      h = (h + 1) & static_cast<unsigned>(H - 1);
-    }
-    return false;
-  };
-  // With at most two candidates per thread (the usual case), each thread
-  // fetches its candidates' slots and scores in one go, before the duplicate
-  // removal, and the scores are written once the hash set is done with.
-  auto gather = [&]() {
-    for (int i = tid; i < H; i += kLT) hs[i] = kNoSlot;
-    int total = 0;
-    if (R <= 2 * kLT) {
-      const int r0 = tid, r1 = kLT + tid;
-      const unsigned s0 = r0 < R ? slot_of(r0) : kNoSlot;
-      const unsigned s1 = r1 < R ? slot_of(r1) : kNoSlot;
-      // The candidates' (x, z) loads are issued here and consumed after the
-      // duplicate removal, which needs only the slots, so that their latency
-      // overlaps it.
-      double x0 = 0.0, z0 = 0.0, x1 = 0.0, z1 = 0.0;
-      if (r0 < R) {
-        x0 = load_relaxed(&T.slots[s0].x);
-        z0 = load_relaxed(&T.slots[s0].z);
-      }
-      if (r1 < R) {
-        x1 = load_relaxed(&T.slots[s1].x);
-        z1 = load_relaxed(&T.slots[s1].z);
-      }
-      __syncthreads();
-      int p0 = -1, p1 = -1, chunk = 0;
-      bool keep = r0 < R && hash_keep(s0);
-      int pos = block_rank(keep, s_wsum, &chunk);
-      if (keep) {
-        us[pos] = s0;
-        p0 = pos;
-      }
-      total = chunk;
-      __syncthreads();
-      if (R > kLT) {
-        keep = r1 < R && hash_keep(s1);
-        pos = block_rank(keep, s_wsum, &chunk);
-        if (keep) {
-          us[total + pos] = s1;
-          p1 = total + pos;
-        }
-        total += chunk;
-        __syncthreads();
-      }
-      // The hash set (which sc overlays) is no longer read.
-      auto score_xz = [&](double x, double z) {
-        const double g = score_of(x, z, xss);
-        return (g >= 0.0) ? g : 0.0;  // as score_at
-      };
-      if (p0 >= 0) sc[p0] = score_xz(x0, z0);
-      if (p1 >= 0) sc[p1] = score_xz(x1, z1);
-    } else {
-      for (int r = tid; r < R; r += kLT) us[r] = slot_of(r);
-      __syncthreads();
-      for (int base = 0; base < R; base += kLT) {
-        const int r = base + tid;
-        const unsigned s = r < R ? us[r] : kNoSlot;
-        const bool keep = r < R && hash_keep(s);
-        int chunk = 0;
-        const int pos = block_rank(keep, s_wsum, &chunk);
-        if (keep) us[total + pos] = s;
-        total += chunk;
-        __syncthreads();
-      }
-      for (int u = tid; u < total; u += kLT) sc[u] = score_at(us[u]);
-    }
-    if (tid == 0) s_U = total;
-    int Pl = 1;
-    while (Pl < total) Pl <<= 1;
-    for (int u = total + tid; u < Pl; u += kLT) {
-      sc[u] = -1.0;
-      us[u] = kNoSlot;
+  // 4. In decreasing score, equal scores in the reference's determinant order
+  //    (detComp_global, src/wavefunction.h:30-36).
+  if (!E.tied) {
+#pragma unroll 4
+    for (int r = tid; r < C.n; r += kLT) {
+      const unsigned long long key = C.key[r];
+      if (key < E.edge) continue;
+      const unsigned pos = atomicAdd(&s_out, 1u);
+      s_sel_key[pos] = key;
+      s_sel_slot[pos] = C.slot[r];
     }
     __syncthreads();
-  };
-  gather();
-  clk.mark(2);
-  const int U = s_U;
-  const int k = U < L.k_req ? U : L.k_req;
-
-  // 4. The k largest scores, by radix selection over the candidates.  Equal
-  //    scores are ordered by the reference's determinant order
-  //    (detComp_global, src/wavefunction.h:30-36); when the k-th and (k+1)-th
-  //    scores are equal that order decides the set, and the whole candidate
-  //    list is sorted instead (rare).
-  const bool fast = topk_radix(us, sc, U, k, T.slots, sS.n_words, s_slot);
-  clk.mark(3);
-  if (!fast) {
-    gather();
-    int P = 1;
-    while (P < U) P <<= 1;
-    const int nwords = sS.n_words;
-    for (int size = 2; size <= P; size <<= 1) {
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        for (int t = tid; t < (P >> 1); t += kLT) {
-          const int i = 2 * stride * (t / stride) + (t % stride);
-          const int j = i + stride;
-          const double si = sc[i], sj = sc[j];
-          bool jfirst;
-          if (si != sj) {
-            jfirst = sj > si;
-          } else {
-            const unsigned a = us[i], b = us[j];
-            if (a == kNoSlot || b == kNoSlot || a == b) {
-              jfirst = false;
-            } else {
-              uint64_t ia, ib, ja, jb;
-              load_key(T.slots + a, ia, ib);
-              load_key(T.slots + b, ja, jb);
-              jfirst = det_ref_compare(ja, jb, ia, ib, nwords) > 0;
-            }
-          }
-          const bool up = (i & size) == 0;
-          if (jfirst == up) {
-            sc[i] = sj;
-            sc[j] = si;
-            const unsigned tmp = us[i];
-            us[i] = us[j];
-            us[j] = tmp;
+    clk.mark(3);
+    // Ranks by counting, 16 lanes per key.
+    const int part = tid & 15;
+#pragma unroll 1
+    for (int i0 = 0; i0 < k; i0 += kLT / 16) {
+      const int i = i0 + (tid >> 4);
+      const unsigned long long mine = i < k ? s_sel_key[i] : 0ull;
+      unsigned rank = 0, equal = 0;
+      for (int j = part; j < k; j += 16) {
+        const unsigned long long o = s_sel_key[j];
+        rank += o > mine ? 1u : 0u;
+        equal += o == mine ? 1u : 0u;
+      }
+#pragma unroll
+      for (int o = 1; o < 16; o <<= 1) {
+        rank += __shfl_xor_sync(~0u, rank, o);
+        equal += __shfl_xor_sync(~0u, equal, o);
+      }
+      if (part == 0 && i < k) {
+        const unsigned slot = s_sel_slot[i];
+        if (equal > 1u) {
+          uint64_t ia, ib;
+          load_key(T.slots + slot, ia, ib);
+          for (int j = 0; j < k; ++j) {
+            if (j == i || s_sel_key[j] != mine) continue;
+            uint64_t ja, jb;
+            load_key(T.slots + s_sel_slot[j], ja, jb);
+            rank += det_ref_compare(ja, jb, ia, ib, sS.n_words) > 0 ? 1u : 0u;
           }
         }
-        __syncthreads();
+        s_slot[rank] = slot;
       }
     }
-    if (tid < k) s_slot[tid] = us[tid];
     __syncthreads();
+  } else {
+    __syncthreads();
+    sort_candidates(C, k, T.slots, sS.n_words, s_slot);
   }
   clk.mark(4);
   if (tid < k) {
@@ -864,8 +1140,7 @@ __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
     uint64_t a, b;
     load_key(sp, a, b);
     s_det[tid] = Det{a, b};
-    s_x[tid] = load_relaxed(&sp->x);
-    s_z[tid] = load_relaxed(&sp->z);
+    load_xz(sp, s_x[tid], s_z[tid]);
   }
   __syncthreads();
   clk.mark(5);
@@ -876,18 +1151,29 @@ __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
   double* Hs = h_in_smem ? reinterpret_cast<double*>(smem) : L.hsub_out;
   double* work = h_in_smem ? Hs + k * k : reinterpret_cast<double*>(smem);
   // One thread per pair i < j (pair t = j(j-1)/2 + i).
+#pragma unroll 1
   for (int t = tid; t < k * (k - 1) / 2; t += kLT) {
     int j = static_cast<int>((1.0f + sqrtf(1.0f + 8.0f * static_cast<float>(t))) * 0.5f);
-    while (j * (j - 1) / 2 > t) --j;
-    while (j * (j + 1) / 2 <= t) ++j;
+    if (j * (j - 1) / 2 > t) --j;
+    if (j * (j + 1) / 2 <= t) ++j;
     const int i = t - j * (j - 1) / 2;
     const double v = off_diagonal(L.ham, s_det[i], s_det[j]);
     Hs[i * k + j] = v;
     Hs[j * k + i] = v;
   }
-  for (int i = warp; i < k; i += kLW) {
-    const double v = diagonal_warp(L.ham, s_det[i], s_occ[warp]);
-    if (lane == 0) Hs[i * k + i] = v;
+#pragma unroll 1
+  for (int i0 = 0; i0 < k; i0 += 2 * kLW) {
+    const int i = i0 + (tid >> 4);
+    const double v = diagonal_half(L.ham, s_det[min(i, k - 1)], s_occ[tid >> 4]);
+    if ((tid & 15) == 0 && i < k) Hs[i * k + i] = v;
+  }
+  if (warp == kLW - 1) {
+    dd xtx, xtz;
+    dots_dd(s_x, s_z, k, xtx, xtz);
+    if (lane == 0) {
+      s_border.xtx = xtx;
+      s_border.xtz = xtz;
+    }
   }
   __threadfence_block();
   __syncthreads();
@@ -903,19 +1189,29 @@ __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
     if (tid == 0) {
       in[2 * kMaxK] = sS.xx.hi;
       in[2 * kMaxK + 1] = sS.xx.lo;
-      in[2 * kMaxK + 2] = sS.xz.hi;
-      in[2 * kMaxK + 3] = sS.xz.lo;
+      in[2 * kMaxK + 2] = s_xz.hi;
+      in[2 * kMaxK + 3] = s_xz.lo;
     }
   }
 
-  // 6. Eig update.
-  const EigResult er =
-      eig_update(Hs, k, s_x, s_z, sS.xx, sS.xz, s_dx, work, clk, L.eig_method == 1 ? sS.eig_drop : 0.0, L.eig_method);
+  // 6. Eig update: the bordered fixed point with method 2, the full solver
+  //    otherwise or when it does not certify its result (and for the first
+  //    iteration, which has no bordering row).
+  int fast = 0;
+  EigResult er;
+  if (L.eig_method == 2) {
+    fast = eig_update_bordered(s_border, Hs, k, s_x, s_z, sS.xx, s_xz, s_dx);
+    clk.mark(16);
+  }
+  if (fast == 0) {
+    er = eig_update_full(Hs, k, s_x, s_z, sS.xx, s_xz, s_dx, work, clk, L.eig_method == 1 ? sS.eig_drop : 0.0);
+    if (L.eig_method == 2 && er.branch == 1) er.fallback = true;
+  }
   clk.mark(15);
-  if (!er.ok) {
+  if (fast < 0 || (fast == 0 && !er.ok)) {
     if (tid == 0) {
       atomicOr(T.err, kErrEig);
-      G->xz = sS.xz;
+      G->xz = s_xz;
       G->pending = 0;
       G->k_cur = 0;
     }
@@ -924,39 +1220,48 @@ __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
 
   // 7. update_x: x[D_i] += dx_i; xz += z_i dx_i; x_size counts dets whose x was 0.
   if (tid < k) {
-    Slot* sp = T.slots + s_slot[tid];
-    const double x0 = s_x[tid];
-    sp->x = x0 + s_dx[tid];
-    if (x0 == 0.0) atomicAdd(&s_newx, 1ull);
+    T.slots[s_slot[tid]].x = s_x[tid] + s_dx[tid];
+    if (s_x[tid] == 0.0) atomicAdd(&s_newx, 1u);
+    G->det[tid] = s_det[tid];
+    G->slot[tid] = s_slot[tid];
+    G->dx[tid] = s_dx[tid];
+    G->hdiag[tid] = Hs[tid * k + tid];
   }
   __syncthreads();
   clk.mark(7);
 
-  // 8. Publish the next iteration.
-  dd zdx{0.0, 0.0};
-  double mx = 0.0;
-  if (warp == 0) {
+  // 8. Publish the next iteration: the eigenvalue's part on warp 0, the sums
+  //    over the picks on warp 1.
+  if (warp == 1) {
+    dd zdx{0.0, 0.0}, none{0.0, 0.0};
+    double mx = 0.0;
+#pragma unroll 1
     for (int i = lane; i < k; i += 32) {
       zdx = dd_add_d(zdx, s_z[i] * s_dx[i]);
       mx = fmax(mx, fabs(s_dx[i]));
     }
-    zdx = warp_sum_dd(zdx);
+    lanes_sum_dd(zdx, none, 1, 32);
+#pragma unroll 1
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(~0u, mx, o));
-  }
-  if (tid == 0) {
-    G->xz = dd_add(sS.xz, zdx);
+    if (lane == 0) {
+      G->xz = dd_add(s_xz, zdx);
+      G->dx_max = mx;
+    }
+  } else if (warp == 0) {
+    if (fast > 0) er = bordered_scalars(s_border, k);
+    if (tid != 0) return;
     G->xx = er.xx;
     G->scale = er.scale;
-    G->xss = dd_mul(er.xx, dd_mul(er.scale, er.scale));
+    G->xss = fast > 0 ? dd_neg(er.rq) : dd_mul(er.xx, dd_mul(er.scale, er.scale));
     G->x_size = sS.x_size + s_newx;
-    G->dx_max = mx;
     G->eig_residual_max = fmax(sS.eig_residual_max, er.resid);
     G->last_branch = er.branch;
     // Energy drop of this update, for the next one's shift: the current
     // energy xz/xx minus the eigenvalue (the energy after the update).
     // (only the shifted solver, eig_method 1, uses it)
-    const double drop = L.eig_method == 1 ? dd_to_d(dd_div(sS.xz, sS.xx)) - er.lambda : 0.0;
-    G->eig_drop = er.branch == 1 && L.eig_method == 1 ? fmax(drop, 1e-300) : 0.0;
+    double drop = 0.0;
+    if (L.eig_method == 1 && er.branch == 1) drop = fmax(dd_to_d(dd_div(s_xz, sS.xx)) - er.lambda, 1e-300);
+    G->eig_drop = drop;
     G->max_abs_evec = er.max_evec;
     G->inv_steps_curr = er.shift_steps;
     G->inv_diff_curr = er.shift_diff;
@@ -972,15 +1277,8 @@ __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
     G->iter = sS.iter + 1;
     G->k_cur = k;
     G->pending = 1;
+    clk.mark(8);
   }
-  if (tid < k) {
-    G->det[tid] = s_det[tid];
-    G->slot[tid] = s_slot[tid];
-    G->dx[tid] = s_dx[tid];
-    G->hdiag[tid] = Hs[tid * k + tid];
-  }
-  __syncthreads();
-  clk.mark(8);
 }
 
 }  // namespace

@@ -69,15 +69,16 @@ __global__ void init_kernel(LeaderLaunch L, Det ref, double ref_diag) {
 }
 
 __global__ void debug_hsub_kernel(HamDev h, const Det* dets, int k, double* H) {
-  __shared__ unsigned char s_occ[kLW][128];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ unsigned char s_occ[2 * kLW][128];
+  const int tid = threadIdx.x;
   for (int t = tid; t < k * k; t += blockDim.x) {
     const int i = t / k, j = t - i * k;
     if (i != j) H[t] = off_diagonal(h, dets[i], dets[j]);
   }
-  for (int i = warp; i < k; i += blockDim.x / 32) {
-    const double v = diagonal_warp(h, dets[i], s_occ[warp]);
-    if (lane == 0) H[i * k + i] = v;
+  for (int i0 = 0; i0 < k; i0 += blockDim.x / 16) {
+    const int i = i0 + (tid >> 4);
+    const double v = diagonal_half(h, dets[min(i, k - 1)], s_occ[tid >> 4]);
+    if ((tid & 15) == 0 && i < k) H[i * k + i] = v;
   }
 }
 
@@ -91,6 +92,8 @@ __device__ void symmetrise_from_upper(double* H, int k) {
   __syncthreads();
 }
 
+constexpr int kDebugBorderMaxK = 64;
+
 __global__ void __launch_bounds__(kLT, 1) debug_eig_kernel(int k, double* H, const double* x, const double* z,
                                                            dd xx, dd xz, double* dx, dd* out, int* branch,
                                                            unsigned* err, double drop, int method, int* steps) {
@@ -102,8 +105,10 @@ __global__ void __launch_bounds__(kLT, 1) debug_eig_kernel(int k, double* H, con
   }
   symmetrise_from_upper(H, k);
   SectionClock clk{nullptr, 0};
-  const EigResult er =
-      eig_update(H, k, s_x, s_z, xx, xz, s_dx, reinterpret_cast<double*>(smem), clk, drop, method);
+  // This entry point keeps method 2 to 64 rows (more take the reduction); the
+  // leader has no such limit.
+  const int use = method == 2 && k > kDebugBorderMaxK ? 0 : method;
+  const EigResult er = eig_update(H, k, s_x, s_z, xx, xz, s_dx, reinterpret_cast<double*>(smem), clk, drop, use);
   for (int i = threadIdx.x; i < k; i += blockDim.x) dx[i] = s_dx[i];
   if (threadIdx.x == 0) {
     out[0] = er.xx;
@@ -220,7 +225,8 @@ constexpr size_t kStaticEigDoubles = kStaticEigFlags + 1;
 
 static __device__ __align__(256) double g_static_eig_scratch[kStaticEigDoubles];
 
-// debug_eig_kernel on the array at `base` (the address of
+// The leader's eig update (the bordered fixed point, certified, or the full
+// reduction) on the array at `base` (the address of
 // g_static_eig_scratch on this device).  A kernel of its own, so that its
 // shared-memory attribute, set once per device, is not changed by debug_eig.
 __global__ void __launch_bounds__(kLT, 1) static_eig_kernel(int k, double* base, dd xx, dd xz) {
@@ -233,7 +239,7 @@ __global__ void __launch_bounds__(kLT, 1) static_eig_kernel(int k, double* base,
   symmetrise_from_upper(base + kStaticEigH, k);
   SectionClock clk{nullptr, 0};
   const EigResult er =
-      eig_update(base + kStaticEigH, k, s_x, s_z, xx, xz, s_dx, reinterpret_cast<double*>(smem), clk, 0.0, 0);
+      eig_update(base + kStaticEigH, k, s_x, s_z, xx, xz, s_dx, reinterpret_cast<double*>(smem), clk, 0.0, 2);
   for (int i = threadIdx.x; i < k; i += blockDim.x) base[kStaticEigDx + i] = s_dx[i];
   if (threadIdx.x == 0) {
     dd* out = reinterpret_cast<dd*>(base + kStaticEigOut);

@@ -30,6 +30,9 @@ constexpr uint64_t kEmptyKey = ~0ull;
 // alpha electrons matches, so every probe passes over it.
 constexpr uint64_t kReservedKeyB = ~0ull - 1ull;
 
+// "No slot" in the candidate lists.
+constexpr unsigned kNoSlot = 0xFFFFFFFFu;
+
 // A slot that holds no determinant: empty, or the reserved last slot.
 MCD_HD bool slot_vacant(uint64_t a, uint64_t b) { return a == kEmptyKey && (b == kEmptyKey || b == kReservedKeyB); }
 
