@@ -42,7 +42,22 @@
 // A block has two phases.  The first needs only the picked determinant: it
 // decodes every entry, reads its matrix element and probes the table for its
 // slot, one record per entry in shared memory.  The second needs dx: it adds
-// to z (inserting where the rule says so), reads x and scores the entry.
+// to z (inserting where the rule says so) and scores the entry.
+//
+// Overlap.  When all CTAs of a launch fit beside the leader's (one SM is its
+// own), they start while it runs (programmatic dependent launch): the leader
+// publishes its picks before it builds and solves the subspace problem, and
+// the CTAs probe their first block meanwhile, then wait for its end.  Keys do
+// not change while the leader runs; x does, on the picked determinants, so the
+// slots that a small filter of these holds have x read again.  What was read
+// before the wait is compared with the final picks after it.  The leader in
+// turn is launched to start when the column CTAs have, and waits for their
+// end, which hides its launch.  Per solve, launched one after the other and
+// overlapped: 7 orbitals, k = 8, 600 iterations 18.6 and 16.8 ms; 12 orbitals,
+// k = 32, 256 iterations 10.7 and 10.3 ms; 24 orbitals, k = 32, 256 iterations
+// 20.8 and 19.3 ms (with the launch overlapped but the probes after the wait,
+// 21.9 ms).  Launches of more CTAs keep the order: the first wave's probes
+// would hide little, and its idle CTAs hold the others back.
 //
 // Candidates.  The keys of a block and the CTA's list so far (at most m) are
 // reduced to the m largest by a radix selection over the whole CTA
@@ -179,17 +194,18 @@ __device__ __forceinline__ void apply_x(unsigned x, uint64_t& a, uint64_t& b) {
   b ^= (beta1 ? m1 : 0ull) ^ (beta2 ? m2 : 0ull);
 }
 
-// Entry e of the column of P's determinant: the packed excitation, (a2, b2)
-// and the signed value.  Returns kNone when the reference stores no such
-// excitation, kKeep for the diagonal and singles (kept whatever their value,
-// as get_single_excitation does), and kIfNonzero for doubles, which the
-// reference stores only with a non-zero table value.  One path for all kinds
-// after the orbitals are decoded: the code stays small, since the leader and
-// this kernel take turns in the instruction caches.
-enum : int { kNone = 0, kKeep = 1, kIfNonzero = 2 };
+// Entry e of the column of P's determinant: the packed excitation with its
+// flags, (a2, b2) and the value, whose sign kXNegative turns.  kXAny: the entry
+// may exist, kXKeep: it is kept whatever its value (the diagonal and singles,
+// as get_single_excitation does; doubles are stored by the reference only with
+// a non-zero table value).  Leaving sign and test to the caller lets it start
+// the hash probe before the table value arrives.  One path for all kinds after
+// the orbitals are decoded: the code stays small, since the leader and this
+// kernel take turns in the instruction caches.
+constexpr unsigned kXNegative = 1u << 29, kXKeep = 1u << 30, kXAny = 1u << 31;
 
-__device__ __forceinline__ int gen_entry(const HamDev& h, const Prelude& P, int e, double hdiag, unsigned& x,
-                                         uint64_t& a2, uint64_t& b2, double& v) {
+__device__ __forceinline__ void gen_entry(const HamDev& h, const Prelude& P, int e, double hdiag, unsigned& x,
+                                          uint64_t& a2, uint64_t& b2, double& v) {
   const int n = h.norb;
   int p = 0, q = 0, r = 0, s = 0;
   unsigned kind = kXDiag;
@@ -232,14 +248,16 @@ __device__ __forceinline__ int gen_entry(const HamDev& h, const Prelude& P, int 
   x = static_cast<unsigned>(p) | (static_cast<unsigned>(q) << 6) | (static_cast<unsigned>(r) << 12) |
       (static_cast<unsigned>(s) << 18) | (kind << 24);
   v = hdiag;
-  int keep = kKeep;
   if (val) {
     v = __ldg(val);
-    keep = kIfNonzero;
+    x |= kXAny;
   } else if (kind != kXDiag) {
     const int sp = kind == kXBeta ? 1 : 0;
-    if (!((__ldg(h.spres + sp * n + p) >> r) & 1ull)) return kNone;
+    const uint64_t stored = __ldg(h.spres + sp * n + p);
     v = single_value(h, P, sp, p, r);
+    if ((stored >> r) & 1ull) x |= kXAny | kXKeep;
+  } else {
+    x |= kXAny | kXKeep;
   }
   // The first excitation on (a, b), the second on the result of the first.
   a2 = P.a;
@@ -255,8 +273,7 @@ __device__ __forceinline__ int gen_entry(const HamDev& h, const Prelude& P, int 
     b2 ^= m2;
   else
     a2 ^= m2;
-  if (neg) v = -v;
-  return keep;
+  if (neg) x |= kXNegative;
 }
 
 // |dz scale| > zt, the insertion rule (src/wavefunction.h:517-528): a double
@@ -286,8 +303,12 @@ struct alignas(16) ColumnShared {
   unsigned list_slot[kMaxM];
   SelectScratch sel;
   double w_sum[kPartSum][kW];
+  double dx, hdiag, zt;  // the column's scalars
+  dd xss, scale;
+  unsigned filter[64];  // of the picked slots
   unsigned out, ties;
-  int last;
+  unsigned slot;        // the picked determinant's
+  int last, some;
 };
 
 // Reduces the CTA's candidates, S.list's n_list and the keys k[0..kRounds) (0:
@@ -350,59 +371,82 @@ __device__ __forceinline__ long long probe_again(const TableDev& t, uint64_t a, 
   return -1;
 }
 
-// One block of entries [at, at + kBlock) of the column, below stop: both
-// phases.  Leaves the candidate keys in S.val and their slots in S.rec.
-__device__ __forceinline__ void column_block(const ColumnLaunch& L, ColumnShared& S, int at, int stop, double hd,
-                                             unsigned dslot, int col, double dxc, dd scale, dd xss, double zt,
-                                             double& acc_newz, double& acc_dot, unsigned& emit, unsigned& upd,
-                                             unsigned& ins, bool timed) {
+// A slot's bit in a 2048-bit filter.
+__device__ __forceinline__ unsigned filter_bit(unsigned slot) { return (slot * 0x9E3779B1u) >> 21; }
+
+// First phase of the block of entries [at, at + kBlock) of the column, below
+// stop: their values (the diagonal's is filled in later), slots and x.
+__device__ __forceinline__ void block_probe(const ColumnLaunch& L, ColumnShared& S, int at, int stop, bool timed) {
   const int tid = threadIdx.x;
   const int nr = min(kRounds, (stop - at + kNT - 1) / kNT);
-  // First phase: the entries' values and slots.
+  // The home slot and matrix element of a thread's next entry are requested before the last one's are
+  // looked at, so that its decoding runs under their latency.
+  const long long q0 = timed ? clock64() : 0;
+  uint64_t na = 0, nb = 0;  // the requested slot's key and x, and the element
+  double nx = 0.0, nv = 0.0;
 #pragma unroll 1
-  for (int r = 0; r < nr; ++r) {
-    const long long q0 = timed ? clock64() : 0;
+  for (int r = 0; r <= nr; ++r) {
+    uint64_t ka = na, kb = nb;
+    double x = nx, v = nv;
     const int e = at + r * kNT + tid;
-    unsigned info = 0u;
-    uint64_t slot = 0;
-    double v = 0.0;
-    if (e < stop) {
-      uint64_t a2, b2, ka = 0, kb = 0;
-      double x = 0.0;
-      const int kind = gen_entry(L.ham, S.P, e, hd, info, a2, b2, v);
-      if (kind != kNone) {
-        // The probe starts at the home slot before the integral value is used
-        // (the diagonal entry's slot is the picked determinant's own).
-        slot = e == 0 ? static_cast<uint64_t>(dslot) : det_hash(a2, b2) & L.tab.mask;
-        load_slot(L.tab.slots + slot, ka, kb, x);
-      }
-      if (timed) atomicAdd(L.sect + 0, static_cast<unsigned long long>(clock64() - q0));
-      if (kind == kKeep || (kind == kIfNonzero && v != 0.0)) {
-#pragma unroll 1
-        for (int q = 1;; ++q) {
-          if (ka == a2 && kb == b2) {
-            info |= kRecFound;
-            S.x[r][tid] = x;
-            break;
-          }
-          if (ka == kEmptyKey && kb == kEmptyKey) {
-            info |= kRecEmpty;
-            break;
-          }
-          if (q >= L.tab.max_probe) {
-            atomicOr(L.tab.err, kErrProbe);
-            break;
-          }
-          slot = (slot + 1) & L.tab.mask;
-          load_slot(L.tab.slots + slot, ka, kb, x);
+    if (r < nr) {
+      unsigned info = 0u;
+      uint64_t slot = 0;
+      if (e < stop) {
+        uint64_t a2, b2;
+        gen_entry(L.ham, S.P, e, 0.0, info, a2, b2, nv);
+        if (info & kXAny) {
+          // (the diagonal entry's slot is the picked determinant's own)
+          slot = e == 0 ? static_cast<uint64_t>(S.slot) : det_hash(a2, b2) & L.tab.mask;
+          load_slot(L.tab.slots + slot, na, nb, nx);
         }
       }
+      S.rec[r][tid] = slot | (static_cast<unsigned long long>(info) << 32);
     }
-    S.rec[r][tid] = slot | (static_cast<unsigned long long>(info) << 32);
-    S.val[r][tid] = static_cast<unsigned long long>(__double_as_longlong(v));
-    if (timed) atomicAdd(L.sect + 1, static_cast<unsigned long long>(clock64() - q0));
+    if (r == 0) continue;
+    const unsigned long long rec = S.rec[r - 1][tid];
+    unsigned info = static_cast<unsigned>(rec >> 32);
+    if (info & kXNegative) v = -v;
+    if ((info & kXKeep) || ((info & kXAny) && v != 0.0)) {
+      uint64_t slot = rec & 0xFFFFFFFFull, a2 = S.P.a, b2 = S.P.b;
+      apply_x(info, a2, b2);
+#pragma unroll 1
+      for (int q = 1;; ++q) {
+        whole_key(L.tab.slots + slot, ka, kb);
+        if (ka == a2 && kb == b2) {
+          info |= kRecFound;
+          S.x[r - 1][tid] = x;
+          break;
+        }
+        if (ka == kEmptyKey && kb == kEmptyKey) {
+          info |= kRecEmpty;
+          break;
+        }
+        if (q >= L.tab.max_probe) {
+          atomicOr(L.tab.err, kErrProbe);
+          break;
+        }
+        slot = (slot + 1) & L.tab.mask;
+        load_slot(L.tab.slots + slot, ka, kb, x);
+      }
+      S.rec[r - 1][tid] = slot | (static_cast<unsigned long long>(info) << 32);
+      S.val[r - 1][tid] = static_cast<unsigned long long>(__double_as_longlong(v));
+    }
   }
-  // Second phase: the z updates and the candidate keys.
+  if (timed) atomicAdd(L.sect + 1, static_cast<unsigned long long>(clock64() - q0));
+}
+
+// Second phase: the z updates and the candidate keys, left in S.val with
+// their slots in S.rec.  kOverlap, and `early`: the first phase may have run
+// before the leader's update of x, so x is read again for the slots that
+// S.filter holds.
+template <bool kOverlap>
+__device__ __forceinline__ void block_update(const ColumnLaunch& L, ColumnShared& S, int nr, bool early, double& acc_newz,
+                                             double& acc_dot, unsigned& emit, unsigned& upd, unsigned& ins,
+                                             bool timed) {
+  const int tid = threadIdx.x;
+  const double dxc = S.dx, zt = S.zt;
+  const dd xss = S.xss, scale = S.scale;
   const long long q2 = timed ? clock64() : 0;
 #pragma unroll 1
   for (int r = 0; r < nr; ++r) {
@@ -410,13 +454,18 @@ __device__ __forceinline__ void column_block(const ColumnLaunch& L, ColumnShared
     const unsigned info = static_cast<unsigned>(rec >> 32);
     unsigned long long key = 0ull;
     if (info & (kRecFound | kRecEmpty)) {
-      const double v = __longlong_as_double(static_cast<long long>(S.val[r][tid]));
+      const bool diagonal = ((info >> 24) & 7u) == kXDiag;
+      const double v = diagonal ? S.hdiag : __longlong_as_double(static_cast<long long>(S.val[r][tid]));
       ++emit;
       const double dz = v * dxc;
       long long slot = static_cast<long long>(rec & 0xFFFFFFFFull);
       double x = 0.0;
       if (info & kRecFound) {
         x = S.x[r][tid];
+        if (kOverlap && early) {
+          const unsigned h = filter_bit(static_cast<unsigned>(slot));
+          if ((S.filter[h >> 5] >> (h & 31u)) & 1u) x = load_relaxed(&L.tab.slots[slot].x);
+        }
       } else {
         bool inserted;
         uint64_t a2 = S.P.a, b2 = S.P.b;
@@ -439,30 +488,61 @@ __device__ __forceinline__ void column_block(const ColumnLaunch& L, ColumnShared
   if (timed) atomicAdd(L.sect + 2, static_cast<unsigned long long>(clock64() - q2));
 }
 
+// The column's picked determinant into S (prelude and slot); false, for the
+// whole CTA, when the iteration has no such column.
+__device__ __forceinline__ bool read_picked(const IterState* St, ColumnShared& S, int col, int norb) {
+  if (threadIdx.x < 32) {
+    const bool some = col < __ldcg(&St->k_cur);
+    if (some) {
+      const Det d{__ldcg(&St->det[col].a), __ldcg(&St->det[col].b)};
+      const unsigned slot = static_cast<unsigned>(__ldcg(&St->slot[col]));
+      build_prelude(S.P, d, norb);
+      if (threadIdx.x == 0) S.slot = slot;
+    }
+    if (threadIdx.x == 0) S.some = some;
+  }
+  __syncthreads();
+  return S.some;
+}
+
+// After the leader's end: whether what read_picked took before it still holds.
+// 1 yes, 0 the iteration has no such column, 2 it was another determinant and
+// has been read again.
+__device__ __forceinline__ int confirm_picked(const IterState* St, ColumnShared& S, int col, int norb) {
+  pdl_wait();
+  if (col >= __ldcg(&St->k_cur)) return 0;
+  if (__ldcg(&St->det[col].a) == S.P.a && __ldcg(&St->det[col].b) == S.P.b &&
+      static_cast<unsigned>(__ldcg(&St->slot[col])) == S.slot)
+    return 1;
+  __syncthreads();
+  read_picked(St, S, col, norb);
+  return 2;
+}
+
 // One CTA's share of one column: CTA `blk` of the launch described by L
-// (column blk / groups, slice blk % groups).
+// (column blk / groups, slice blk % groups).  kOverlap: launched to start
+// beside the leader; the first block is probed from the determinants as the
+// leader publishes them when it has picked, while it solves for dx.
+template <bool kOverlap>
 __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
   const int G = L.groups;
   const int col = blk / G;
   const int g = blk - col * G;
   IterState* St = L.st;
-  const int kcur = St->k_cur;
-  if (col >= kcur) return;
 
   __shared__ __align__(16) ColumnShared S;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool timed = L.sect != nullptr && tid == 0;
   const long long c_start = timed ? clock64() : 0;
-  // The column's scalars are read while warp 0 decodes the determinant.
-  const double dxc = St->dx[col];
-  const double hd = St->hdiag[col];
-  const dd xss = St->xss;
-  const dd scale = St->scale;
-  const double zt = St->zt;
-  const unsigned dslot = static_cast<unsigned>(St->slot[col]);
-  if (warp == 0) build_prelude(S.P, St->det[col], L.ham.norb);
-  __syncthreads();
+  bool early = false;  // probing before the leader has ended
+  if (kOverlap) {
+    if (tid == 0) pdl_trigger();
+    if (tid < 64) S.filter[tid] = 0u;
+    early = read_picked(St, S, col, L.ham.norb);
+    if (!early) pdl_wait();
+  }
+  if (!early && !read_picked(St, S, col, L.ham.norb)) return;
   const int total = S.P.total;
   // CTA g's slice: whole rounds of kNT entries, shared evenly.
   const int chunks = (total + kNT - 1) / kNT;
@@ -488,6 +568,11 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
     unsigned p[kRounds + 1];
     if (at >= stop) {
       if (merging) break;
+      if (kOverlap && early) {  // an empty slice
+        pdl_wait();
+        early = false;
+        if (col >= __ldcg(&St->k_cur)) return;
+      }
       // This CTA's list and partial sums to global memory, then a ticket: the
       // last CTA of the column merges all of them.
       const long long c_post = timed ? clock64() : 0;
@@ -498,7 +583,6 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
       if (tid < M) {
         L.part_key[part * M + tid] = tid < n_list ? S.list_key[tid] : 0ull;
         L.part_slot[part * M + tid] = tid < n_list ? S.list_slot[tid] : 0u;
-        __threadfence();  // before the ticket
       }
       // The counters travel with the sums (exact in a double) and are added
       // once per column by its last CTA, not by every CTA into the same words.
@@ -511,18 +595,21 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
         for (int j = 0; j < kPartSum; ++j) S.w_sum[j][warp] = v[j];
       }
       __syncthreads();
-      if (tid < kPartSum) {
-        double t = 0.0;
-#pragma unroll 1
-        for (int w = 0; w < kW; ++w) t += S.w_sum[tid][w];
-        L.part_sum[kPartSum * part + tid] = t;
-        __threadfence();
-      }
-      __syncwarp();
-      if (tid == 0) {
-        if (bound != 0ull) atomicMax(L.bound + col, bound);
-        __threadfence();
-        S.last = (atomicAdd(L.done + col, 1u) == static_cast<unsigned>(G - 1));
+      if (warp == 0) {
+        if (lane < kPartSum) {
+          double t = 0.0;
+#pragma unroll
+          for (int w = 0; w < kW; ++w) t += S.w_sum[lane][w];
+          L.part_sum[kPartSum * part + lane] = t;
+        }
+        __syncwarp();
+        // One fence for the whole CTA's list and sums (the barriers order
+        // them before it), then the ticket.
+        if (lane == 0) {
+          if (bound != 0ull) atomicMax(L.bound + col, bound);
+          __threadfence();
+          S.last = (atomicAdd(L.done + col, 1u) == static_cast<unsigned>(G - 1));
+        }
       }
       __syncthreads();
       c_merge = timed ? clock64() : 0;
@@ -537,17 +624,41 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
       continue;
     }
     if (merging) {
-      // Lists below the best bound of any CTA are left out.
+      // Keys below the best bound of any CTA are left out.
       const size_t base = static_cast<size_t>(col) * G * M;
 #pragma unroll
       for (int r = 0; r < kRounds; ++r) {
         const int i = at + r * kNT + tid;
         k[r] = i < stop ? __ldcg(L.part_key + base + i) : 0ull;
-        p[r] = i < stop ? __ldcg(L.part_slot + base + i) : 0u;
+        p[r] = i < stop ? static_cast<unsigned>(i) : 0u;
       }
     } else {
-      column_block(L, S, at, stop, hd, dslot, col, dxc, scale, xss, zt, acc_newz, acc_dot, emit, upd, ins, timed);
+      block_probe(L, S, at, stop, timed);
+      if (at == beg) {
+        if (kOverlap && early) {
+          const int state = confirm_picked(St, S, col, L.ham.norb);
+          if (state == 0) return;
+          if (state == 2) {  // read before the leader had published it: probe again
+            early = false;
+            continue;
+          }
+          if (tid < kMaxK && tid < __ldcg(&St->k_cur)) {
+            const unsigned h = filter_bit(static_cast<unsigned>(__ldcg(&St->slot[tid])));
+            atomicOr(&S.filter[h >> 5], 1u << (h & 31u));
+          }
+        }
+        if (tid == 0) {
+          S.dx = __ldcg(&St->dx[col]);
+          S.hdiag = __ldcg(&St->hdiag[col]);
+          S.zt = __ldcg(&St->zt);
+          S.xss = dd{__ldcg(&St->xss.hi), __ldcg(&St->xss.lo)};
+          S.scale = dd{__ldcg(&St->scale.hi), __ldcg(&St->scale.lo)};
+        }
+        __syncthreads();
+      }
       const int nr = min(kRounds, (stop - at + kNT - 1) / kNT);
+      block_update<kOverlap>(L, S, nr, early, acc_newz, acc_dot, emit, upd, ins, timed);
+      early = false;
       const unsigned long long shared_bound = __ldcg(L.bound + col);
       if (shared_bound > bound) bound = shared_bound;
 #pragma unroll
@@ -565,7 +676,9 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
     if (timed && !merging) atomicAdd(L.sect + 3, static_cast<unsigned long long>(clock64() - q3));
     at += kBlock;
   }
-  if (tid < L.m) L.cand_slot[static_cast<size_t>(col) * L.m + tid] = tid < n_list ? S.list_slot[tid] : kNoSlot;
+  if (tid < L.m)
+    L.cand_slot[static_cast<size_t>(col) * L.m + tid] =
+        tid < n_list ? __ldcg(L.part_slot + static_cast<size_t>(col) * G * M + S.list_slot[tid]) : kNoSlot;
   if (warp < kPartSum) {
     // Column sums in a fixed order, one per warp: lane-strided partials, then a fixed tree.
     double t = 0.0;
@@ -603,7 +716,10 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
   }
 }
 
-__global__ void __launch_bounds__(kNT, kColumnCtasPerSm) column_kernel(ColumnLaunch L) { column_body(L, blockIdx.x); }
+template <bool kOverlap>
+__global__ void __launch_bounds__(kNT, kColumnCtasPerSm) column_kernel(ColumnLaunch L) {
+  column_body<kOverlap>(L, blockIdx.x);
+}
 
 // Several instances in one grid: CTAs [cta_begin[i], cta_begin[i+1]) belong
 // to instance i and keep the layout of its own launch.
@@ -616,7 +732,7 @@ __global__ void __launch_bounds__(kNT, kColumnCtasPerSm) column_kernel_batch(Col
     else
       hi = mid;
   }
-  column_body(B.L[lo], static_cast<int>(blockIdx.x) - B.cta_begin[lo]);
+  column_body<false>(B.L[lo], static_cast<int>(blockIdx.x) - B.cta_begin[lo]);
 }
 
 __global__ void __launch_bounds__(kNT) debug_column_kernel(HamDev h, Det d, double hd, uint64_t* ao,
@@ -628,8 +744,9 @@ __global__ void __launch_bounds__(kNT) debug_column_kernel(HamDev h, Det d, doub
     unsigned x;
     uint64_t a2, b2;
     double v;
-    const int kind = gen_entry(h, P, e, hd, x, a2, b2, v);
-    if (kind == kKeep || (kind == kIfNonzero && v != 0.0)) {
+    gen_entry(h, P, e, hd, x, a2, b2, v);
+    if (x & kXNegative) v = -v;
+    if ((x & kXKeep) || ((x & kXAny) && v != 0.0)) {
       const int pos = atomicAdd(nout, 1);
       if (pos < cap) {
         ao[pos] = a2;
@@ -864,8 +981,12 @@ int column_groups(int entries, int k, int resident) {
   return g < 1 ? 1 : g;
 }
 
+bool column_overlaps(int ctas, int sms) { return ctas <= kColumnCtasPerSm * (sms - 1); }
+
 cudaError_t launch_column(const ColumnLaunch& a, cudaStream_t s) {
-  column_kernel<<<a.k_grid * a.groups, kNT, 0, s>>>(a);
+  const dim3 grid(a.k_grid * a.groups), block(kNT);
+  if (a.overlap) return launch_overlapped(column_kernel<true>, grid, block, 0, s, a);
+  column_kernel<false><<<grid, block, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -133,7 +133,8 @@ __device__ __forceinline__ void load_key(const Slot* s, uint64_t& a, uint64_t& b
 }
 // A slot's key and x in one 32-byte load (relaxed per 64-bit word): a key word
 // changes once, from the empty key's, so a key caught between its two words
-// has exactly one of them empty, and is read again whole.  x is not written
+// has exactly one of them empty.  whole_key, on the loaded words, reads such a
+// key again; it is apart so that the load can stay in flight.  x is not written
 // while keys are inserted.
 __device__ __forceinline__ void load_slot(const Slot* s, uint64_t& a, uint64_t& b, double& x) {
   uint64_t xb;
@@ -143,6 +144,8 @@ __device__ __forceinline__ void load_slot(const Slot* s, uint64_t& a, uint64_t& 
                : "l"(s)
                : "memory");
   x = __longlong_as_double(static_cast<long long>(xb));
+}
+__device__ __forceinline__ void whole_key(const Slot* s, uint64_t& a, uint64_t& b) {
   if ((a == kEmptyKey) != (b == kEmptyKey)) load_key(s, a, b);
 }
 __device__ __forceinline__ void cas_key(Slot* s, uint64_t na, uint64_t nb, uint64_t& oa, uint64_t& ob) {
@@ -275,6 +278,30 @@ struct SectionClock {
     }
   }
 };
+
+// ---------------------------------------------------------------------------
+// The two kernels of an iteration overlap at their ends (programmatic
+// dependent launch): a kernel's CTAs may start once every CTA of the one
+// before has called pdl_trigger (or ended), and pdl_wait returns when that
+// kernel has ended and its writes are visible.  Both do nothing in a kernel
+// launched the ordinary way.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename A>
+cudaError_t launch_overlapped(void (*kernel)(A), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A& arg) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, arg);
+}
 
 // ---------------------------------------------------------------------------
 // Warp helpers.

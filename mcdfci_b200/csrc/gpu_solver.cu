@@ -599,7 +599,9 @@ GpuSolver::GpuSolver(const Fcidump& fci, const SolverOptions& opt) : opt_(opt) {
   }
   int sms = 0;
   check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_), "cudaDeviceGetAttribute");
-  groups_rule_ = column_groups(entries_, opt_.k, opt_.fill_gpu ? kColumnCtasPerSm * sms : 0);
+  sms_ = sms;
+  // (the leader's CTA takes one SM to itself)
+  groups_rule_ = column_groups(entries_, opt_.k, opt_.fill_gpu ? kColumnCtasPerSm * (sms - 1) : 0);
   groups_ = opt_.groups > 0 ? opt_.groups : groups_rule_;
   if (opt_.autotune && opt_.groups == 0 && groups_ > kMaxGroups) groups_ = kMaxGroups;
   list_ = column_list_size(opt_.m);
@@ -786,6 +788,7 @@ GpuSolver::GpuSolver(const Fcidump& fci, const SolverOptions& opt) : opt_(opt) {
   cl_.list = list_;
   cl_.groups = groups_;
   cl_.k_grid = opt_.k;
+  cl_.overlap = column_overlaps(opt_.k * groups_, sms_);
   cl_.na = na_;
   cl_.nb = nb_;
 
@@ -1048,6 +1051,7 @@ void GpuSolver::set_groups(int g) {
   if (g == groups_) return;
   groups_ = g;
   cl_.groups = g;
+  cl_.overlap = column_overlaps(opt_.k * g, sms_);
   if (graph_) cudaGraphExecDestroy(graph_);
   graph_ = nullptr;
 }

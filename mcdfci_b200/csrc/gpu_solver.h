@@ -213,6 +213,7 @@ class GpuSolver {
   cudaStream_t stream_ = nullptr;
   bool own_stream_ = false;
   int device_ = 0;
+  int sms_ = 0;
   void* d_tables_ = nullptr;
   void* d_misc_ = nullptr;  // unused: the buffers from d_state_ to d_done_ follow the tables in d_tables_
   Slot* d_slots_ = nullptr;

@@ -12,6 +12,10 @@
 //                            and applies z += H_col * dx to the hash table,
 //                            keeping each column's top-m candidates.
 //
+// The column CTAs may start beside the leader, and the leader beside the last
+// of them (column_kernel.cu); each waits for the other kernel's end before it
+// uses anything that kernel wrote, but for the picked determinants.
+//
 // All scalar solver state lives in IterState in device memory, so iterations
 // run back-to-back without host round trips and can be captured in a graph.
 #pragma once
@@ -91,6 +95,7 @@ struct ColumnLaunch {
   int list;               // stride of the per-CTA lists (column_list_size(m))
   int groups;             // CTAs per column
   int k_grid;             // columns launched (>= k_cur)
+  bool overlap;           // the CTAs may start beside the leader (column_overlaps)
   int na, nb;             // electrons per spin (fixed by the starting determinant)
 };
 
@@ -176,6 +181,9 @@ int column_list_size(int m);
 // slots of the GPU empty (resident = 0: never more); at most 96.
 constexpr int kColumnCtasPerSm = 4;
 int column_groups(int entries, int k, int resident);
+// Whether a launch of `ctas` column CTAs is to start beside the leader: when
+// all of them fit on the SMs that the leader leaves free.
+bool column_overlaps(int ctas, int sms);
 // The most CTAs per column the autotuner tries, and its iterations per trial.
 constexpr int kMaxGroups = 96;
 constexpr int kTuneIters = 16;

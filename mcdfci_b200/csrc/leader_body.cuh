@@ -976,6 +976,8 @@ __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
     reinterpret_cast<uint4*>(C.set)[i] = make_uint4(kNoSlot, kNoSlot, kNoSlot, kNoSlot);
   if (tid == 0) s_out = s_newx = 0u;
 
+  pdl_wait();  // for the column kernel
+
   // 1. The scalars into shared memory, and the end of the previous iteration
   //    (src/wavefunction.h:557-565,583; unless finish_kernel already did):
   //    z[D_c] = new_z_c for the picked determinants, xz += sum_c dot_c.
@@ -1141,8 +1143,15 @@ __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
     load_key(sp, a, b);
     s_det[tid] = Det{a, b};
     load_xz(sp, s_x[tid], s_z[tid]);
+    // The picks go out now, so that the column kernel can enumerate and probe
+    // their columns while the subspace problem is solved here.
+    G->det[tid] = s_det[tid];
+    G->slot[tid] = s_slot[tid];
+    if (tid == 0) G->k_cur = k;
+    __threadfence();
   }
   __syncthreads();
+  if (tid == 0) pdl_trigger();
   clk.mark(5);
 
   // 5. H_sub: in shared memory when it fits beside the eig scratch, else in
@@ -1222,8 +1231,6 @@ __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
   if (tid < k) {
     T.slots[s_slot[tid]].x = s_x[tid] + s_dx[tid];
     if (s_x[tid] == 0.0) atomicAdd(&s_newx, 1u);
-    G->det[tid] = s_det[tid];
-    G->slot[tid] = s_slot[tid];
     G->dx[tid] = s_dx[tid];
     G->hdiag[tid] = Hs[tid * k + tid];
   }
@@ -1275,7 +1282,6 @@ __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
     G->emitted = 0;
     G->updates = 0;
     G->iter = sS.iter + 1;
-    G->k_cur = k;
     G->pending = 1;
     clk.mark(8);
   }

@@ -166,8 +166,7 @@ cudaError_t launch_leader(const LeaderLaunch& a, cudaStream_t s) {
   const size_t bytes = leader_smem_bytes(a.k_req, a.m);
   cudaError_t e = ensure_smem(reinterpret_cast<const void*>(leader_kernel), bytes, g_leader_smem);
   if (e != cudaSuccess) return e;
-  leader_kernel<<<1, kLT, bytes, s>>>(a);
-  return cudaGetLastError();
+  return launch_overlapped(leader_kernel, dim3(1), dim3(kLT), bytes, s, a);
 }
 
 cudaError_t launch_leader_batch(const LeaderBatch& b, cudaStream_t s) {

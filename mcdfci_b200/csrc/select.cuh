@@ -7,8 +7,11 @@
 namespace mcd {
 
 struct SelectScratch {
-  alignas(16) unsigned hist[3][256];
+  alignas(16) unsigned hist[2][256];
   unsigned cnt[32], max[32];
+  unsigned bin, in_bin, need;
+  unsigned long long few[32], edge;  // the keys of a bin with at most 32
+  unsigned n_few, tied;
 };
 
 // What to keep of the CTA's keys: all with key >= edge, but of those equal to
@@ -30,9 +33,9 @@ __device__ __forceinline__ unsigned long long score_key(double score) {
 // bits (the exponent and three mantissa bits) down from the largest key, with
 // all keys 255 or more steps below it in the last bin, then eight bits at a
 // time within the bin that holds the want-th largest, until the keys at and
-// above a bin are exactly `want`.  One barrier per pass: every warp scans the
-// histogram itself, and three histograms rotate so that the one cleared was
-// last read before the previous barrier.  Called by the whole CTA (at least
+// above a bin are exactly `want`.  One warp scans the histogram: with every
+// warp scanning it for itself a pass has one barrier less, but the callers
+// are bound by instruction issue (up to eight warps per scheduler).  Called by the whole CTA (at least
 // 256 threads), with a barrier since the scratch was last used.
 template <class Each>
 __device__ __forceinline__ SelectEdge select_edge(SelectScratch& S, unsigned want, Each each) {
@@ -49,6 +52,7 @@ __device__ __forceinline__ SelectEdge select_edge(SelectScratch& S, unsigned wan
     S.max[warp] = mx;
   }
   if (tid < 256) S.hist[0][tid] = 0u;
+  if (tid == 0) S.n_few = 0u;
   __syncthreads();
   SelectEdge r;
   r.total = __reduce_add_sync(~0u, lane < nw ? S.cnt[lane] : 0u);
@@ -65,41 +69,77 @@ __device__ __forceinline__ SelectEdge select_edge(SelectScratch& S, unsigned wan
       const unsigned long long y = key >> lo, d = ref - y;
       if (key != 0ull && y <= ref && d < limit) atomicAdd(&S.hist[buf][d < 255ull ? static_cast<unsigned>(d) : 255u], 1u);
     });
-    const int nxt = buf == 2 ? 0 : buf + 1;
-    if (tid < 256) S.hist[nxt][tid] = 0u;
+    if (tid < 256) S.hist[buf ^ 1][tid] = 0u;
     __syncthreads();
-    // The bin of the need-th largest: lane l holds bins 8l .. 8l+7.
-    const uint4 u0 = *reinterpret_cast<const uint4*>(&S.hist[buf][8 * lane]);
-    const uint4 u1 = *reinterpret_cast<const uint4*>(&S.hist[buf][8 * lane + 4]);
-    buf = nxt;
-    const unsigned c[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
-    const unsigned t = ((c[0] + c[1]) + (c[2] + c[3])) + ((c[4] + c[5]) + (c[6] + c[7]));
-    unsigned run = t;
+    if (warp == 0) {
+      // The bin of the need-th largest: lane l holds bins 8l .. 8l+7.
+      const uint4 u0 = *reinterpret_cast<const uint4*>(&S.hist[buf][8 * lane]);
+      const uint4 u1 = *reinterpret_cast<const uint4*>(&S.hist[buf][8 * lane + 4]);
+      const unsigned c[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+      const unsigned t = ((c[0] + c[1]) + (c[2] + c[3])) + ((c[4] + c[5]) + (c[6] + c[7]));
+      unsigned run = t;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned v = __shfl_up_sync(~0u, run, o);
-      if (lane >= o) run += v;
-    }
-    const int src = __ffs(__ballot_sync(~0u, run >= r.need)) - 1;
-    run -= t;
-    unsigned bin = 8u * lane, in_bin = c[0];
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned v = __shfl_up_sync(~0u, run, o);
+        if (lane >= o) run += v;
+      }
+      const int src = __ffs(__ballot_sync(~0u, run >= r.need)) - 1;
+      if (lane == src) {
+        run -= t;
+        unsigned bin = 8u * lane, in_bin = c[0];
 #pragma unroll
-    for (int j = 0; j < 7; ++j) {
-      if (run + in_bin < r.need) {
-        run += in_bin;
-        in_bin = c[j + 1];
-        ++bin;
+        for (int j = 0; j < 7; ++j) {
+          if (run + in_bin < r.need) {
+            run += in_bin;
+            in_bin = c[j + 1];
+            ++bin;
+          }
+        }
+        S.bin = bin;
+        S.in_bin = in_bin;
+        S.need = r.need - run;
       }
     }
-    bin = __shfl_sync(~0u, bin, src);
-    in_bin = __shfl_sync(~0u, in_bin, src);
-    r.need -= __shfl_sync(~0u, run, src);
+    __syncthreads();
+    buf ^= 1;
+    const unsigned bin = S.bin, in_bin = S.in_bin;
+    r.need = S.need;
     const bool rest = limit == ~0ull && bin == 255u;  // the bin of everything further down
     if (!rest) r.edge = (ref - bin) << lo;
     if (in_bin == r.need) break;
     if (rest) {
       ref -= 255ull;
       continue;
+    }
+    if (in_bin <= 32u) {
+      // Few keys are left to choose from (often an equal pair, which digits
+      // would separate last or never): rank them by counting.
+      const unsigned long long bin_key = ref - bin;
+      each([&](unsigned long long key) {
+        if (key != 0ull && (key >> lo) == bin_key) S.few[atomicAdd(&S.n_few, 1u)] = key;
+      });
+      __syncthreads();
+      if (warp == 0) {
+        const unsigned long long mine = static_cast<unsigned>(lane) < in_bin ? S.few[lane] : 0ull;
+        unsigned above = 0, equal = 0, rank = 0;
+#pragma unroll 4
+        for (unsigned j = 0; j < in_bin; ++j) {
+          const unsigned long long o = S.few[j];
+          above += o > mine ? 1u : 0u;
+          equal += o == mine ? 1u : 0u;
+          rank += o > mine || (o == mine && j < static_cast<unsigned>(lane)) ? 1u : 0u;
+        }
+        if (static_cast<unsigned>(lane) < in_bin && rank == r.need - 1u) {
+          S.edge = mine;
+          S.need = r.need - above;
+          S.tied = equal > r.need - above ? 1u : 0u;
+        }
+      }
+      __syncthreads();
+      r.edge = S.edge;
+      r.need = S.need;
+      r.tied = S.tied != 0u;
+      break;
     }
     if (lo == 0) {
       r.tied = true;
