@@ -241,9 +241,9 @@ int mcd_batch_result(const mcd_batch* b, double* energies);
  * derivative with respect to the integrals is the reduced density matrices of
  * the wavefunction: dE/dh_PQ = rdm1[P][Q] and dE/d(PR|QS) = rdm2[P][Q][R][S]/2
  * for independent entries of the dense spatial integral arrays.  mcd_rdm
- * computes them from the current wavefunction on the GPU (one pass over the
- * determinants with nonzero coefficients, recomputing their single and double
- * excitations): rdm1[P*n+Q] = sum_s <a+_{Ps} a_{Qs}>, rdm2[((P*n+Q)*n+R)*n+S] =
+ * computes them from the current wavefunction on the GPU (the pairs of
+ * determinants with nonzero coefficients that single and double excitations
+ * connect): rdm1[P*n+Q] = sum_s <a+_{Ps} a_{Qs}>, rdm2[((P*n+Q)*n+R)*n+S] =
  * sum_{s,t} <a+_{Ps} a+_{Qt} a_{St} a_{Rs}>, normalised, n spatial orbitals,
  * so that E = sum h_PQ rdm1[P][Q] + 1/2 sum (PR|QS) rdm2[P][Q][R][S] + E_core.
  * RHF FCIDUMPs only (MCD_ERR_UNSUPPORTED for UHF). */
@@ -306,6 +306,9 @@ int mcd_debug_eig_shifted(int32_t k, const double* hsub, const double* x, const 
 int mcd_debug_eig_method(int32_t k, const double* hsub, const double* x, const double* z, const double xx[2],
                          const double xz[2], int32_t method, double drop, double* dx, double new_xx[2],
                          double new_scale[2], int32_t* branch, int32_t* steps);
+/* mcd_rdm with the pairs found by comparing every two determinants (route 1),
+ * by looking up every excitation in the table (2), or as mcd_rdm does (0). */
+int mcd_debug_rdm(mcd_solver* s, double* rdm1, double* rdm2, int32_t route);
 /* mcd_debug_eig without any allocation: no counterpart in the reference.
  * The same update, solved as the leader solves it by default (method 2 at
  * every k, with the full reduction when it does not certify its result: the

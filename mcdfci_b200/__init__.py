@@ -46,7 +46,7 @@ EXPORTED_SYMBOLS = (
     "mcd_batch_create", "mcd_batch_destroy", "mcd_batch_size", "mcd_batch_solve", "mcd_batch_reset",
     "mcd_batch_run_iterations", "mcd_batch_run_iterations_timed", "mcd_batch_get_report", "mcd_batch_result",
     "mcd_rdm", "mcd_debug_wavefunction", "mcd_debug_compact", "mcd_checkpoint_save", "mcd_checkpoint_load",
-    "mcd_debug_column_sections", "mcd_residual", "mcd_debug_slots", "mcd_debug_eig_shifted", "mcd_debug_eig_method",
+    "mcd_debug_column_sections", "mcd_residual", "mcd_debug_slots", "mcd_debug_rdm", "mcd_debug_eig_shifted", "mcd_debug_eig_method",
     "mcd_debug_table_info", "mcd_debug_setup_times", "mcd_batch_residual", "mcd_debug_scatter_rate_mode",
     "mcd_debug_autotune_info", "mcd_batch_table_sums", "mcd_debug_grow",
 )
@@ -147,6 +147,7 @@ def library() -> ctypes.CDLL:
     L.mcd_debug_eig_method.argtypes = [ctypes.c_int32, _dp, _dp, _dp, _dp, _dp, ctypes.c_int32, ctypes.c_double, _dp,
                                        _dp, _dp, ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(ctypes.c_int32)]
     L.mcd_rdm.argtypes = [vp, _dp, _dp]
+    L.mcd_debug_rdm.argtypes = [vp, _dp, _dp, ctypes.c_int32]
     L.mcd_debug_compact.argtypes = [vp, ctypes.c_double, _u64p]
     L.mcd_debug_grow.argtypes = [vp, ctypes.c_int32, ctypes.POINTER(ctypes.c_int64)]
     L.mcd_debug_column_sections.argtypes = [vp, _u64p, ctypes.c_int32, ctypes.c_int32]
@@ -410,6 +411,16 @@ class CDFCI:
         _check(library().mcd_rdm(self._h, g1.ctypes.data_as(_dp), g2.ctypes.data_as(_dp)))
         return g1.reshape(n, n), g2.reshape(n, n, n, n)
 
+    def debug_rdm(self, route: int):
+        """rdm() with the connected pairs found by comparing determinants
+        (1) or by looking up excitations (2) (mcd_debug_rdm)."""
+        import numpy as np
+
+        n = self.norb
+        g1, g2 = np.zeros((n, n)), np.zeros((n, n, n, n))
+        _check(library().mcd_debug_rdm(self._h, g1.ctypes.data_as(_dp), g2.ctypes.data_as(_dp), route))
+        return g1, g2
+
     COLUMN_SECTIONS = ("decode", "probe", "update", "offer", "rounds", "prelude", "post", "merge", "ctas", "merges")
 
     def column_sections(self, enable: bool = True) -> dict:
@@ -438,15 +449,17 @@ class CDFCI:
         import numpy as np
 
         cnt = ctypes.c_int64()
-        _check(library().mcd_debug_wavefunction(self._h, None, None, None, 0, ctypes.byref(cnt)))
-        n = cnt.value + 16
-        a = np.zeros(n, dtype=np.uint64)
-        b = np.zeros(n, dtype=np.uint64)
-        x = np.zeros(n)
-        _check(library().mcd_debug_wavefunction(self._h, a.ctypes.data_as(_u64p), b.ctypes.data_as(_u64p),
-                                                x.ctypes.data_as(_dp), n, ctypes.byref(cnt)))
-        k = min(cnt.value, n)
-        return a[:k], b[:k], x[:k]
+        n = self.report()["x_size"] + 16
+        while True:
+            a = np.zeros(n, dtype=np.uint64)
+            b = np.zeros(n, dtype=np.uint64)
+            x = np.zeros(n)
+            _check(library().mcd_debug_wavefunction(self._h, a.ctypes.data_as(_u64p), b.ctypes.data_as(_u64p),
+                                                    x.ctypes.data_as(_dp), n, ctypes.byref(cnt)))
+            k = cnt.value
+            if k <= n:
+                return a[:k], b[:k], x[:k]
+            n = k
 
     @property
     def stream(self) -> int:

@@ -613,10 +613,15 @@ int mcd_eig_update_static(int32_t k, const double* hsub, const double* x, const 
 int mcd_rdm(mcd_solver* s, double* rdm1, double* rdm2) {
   return guarded([&] {
     if (!s || !rdm1 || !rdm2) return fail(MCD_ERR_INVALID, "NULL argument.");
-    std::vector<double> g1, g2;
-    s->impl->rdm(g1, g2);
-    std::copy(g1.begin(), g1.end(), rdm1);
-    std::copy(g2.begin(), g2.end(), rdm2);
+    s->impl->rdm(rdm1, rdm2);
+    return MCD_OK;
+  });
+}
+
+int mcd_debug_rdm(mcd_solver* s, double* rdm1, double* rdm2, int32_t route) {
+  return guarded([&] {
+    if (!s || !rdm1 || !rdm2) return fail(MCD_ERR_INVALID, "NULL argument.");
+    s->impl->rdm(rdm1, rdm2, route);
     return MCD_OK;
   });
 }

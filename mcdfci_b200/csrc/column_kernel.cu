@@ -759,133 +759,190 @@ __global__ void __launch_bounds__(kNT) debug_column_kernel(HamDev h, Det d, doub
 
 // ---------------------------------------------------------------------------
 // Reduced density matrices of the wavefunction in the table (the adjoint of
-// the energy with respect to the integrals).  One CTA per determinant D with
-// x_D != 0: the diagonal terms over D's occupied pairs, then every single and
-// double excitation D' of D (all of them: the RDM is a property of the
-// wavefunction, so no integral screening) with x_D' looked up in the table.
-// The operator phases are those of the column generation, i.e. of
-// <D'|a+_r a_p|D> and <D'|a+_r a+_s a_q a_p|D> in the interleaved order.
-// Accumulated unnormalised, in spin blocks (see RdmLaunch).
+// the energy with respect to the integrals): the sum over ordered pairs (D, D')
+// of determinants with x != 0 that differ by at most two electrons, of
+// x_D x_D' <D'|a+_r a_p|D> and <D'|a+_r a+_s a_q a_p|D>, with the phases of
+// the column generation and no integral screening (the RDM is a property of
+// the wavefunction).  Accumulated unnormalised, in spin blocks (see
+// RdmLaunch), folded on the device.  The pairs are found in one of two ways:
+// by comparing every two determinants (rdm_pairs_kernel) or by looking up
+// every excitation of every determinant (rdm_lookup_kernel).  See launch_rdm.
 
-__global__ void rdm_list_kernel(const Slot* slots, size_t n, unsigned* list, unsigned long long* count,
-                                unsigned long long cap) {
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const Slot sl = slots[i];
-    if (slot_vacant(sl.a, sl.b)) continue;
-    if (sl.x == 0.0) continue;
+__global__ void __launch_bounds__(256) collect_x_kernel(const Slot* slots, size_t n, Slot* list,
+                                                        unsigned long long* count, unsigned long long cap) {
+  scan_slots(slots, n, [&](const Slot& sl, size_t i) {
+    if (slot_vacant(sl.a, sl.b) || sl.x == 0.0) return;
     const unsigned long long j = atomicAdd(count, 1ull);
-    if (j < cap) list[j] = static_cast<unsigned>(i);
-  }
-}
-
-// Canonical index of a same-spin pair block element: (p, q) and (r, s) put in
-// increasing order; returns the sign of the reordering.
-__device__ __forceinline__ double pair_canon(int& p, int& q) {
-  if (p < q) return 1.0;
-  const int t = p;
-  p = q;
-  q = t;
-  return -1.0;
+    if (j < cap) list[j] = Slot{sl.a, sl.b, sl.x, static_cast<double>(i)};
+  });
 }
 
 __device__ __forceinline__ size_t idx4(int n, int p, int q, int r, int s) {
   return ((static_cast<size_t>(p) * n + q) * n + r) * n + s;
 }
 
-__global__ void __launch_bounds__(kNT) rdm_kernel(RdmLaunch R) {
+// x of a determinant, 0 when it is absent; key and x in one load per slot.
+__device__ __forceinline__ double find_x(const TableDev& t, uint64_t a, uint64_t b) {
+  uint64_t i = det_hash(a, b) & t.mask;
+#pragma unroll 1
+  for (int p = 0; p < t.max_probe; ++p) {
+    uint64_t ka, kb;
+    double x;
+    load_slot(t.slots + i, ka, kb, x);
+    if (ka == a && kb == b) return x;
+    if (ka == kEmptyKey && kb == kEmptyKey) return 0.0;
+    i = (i + 1) & t.mask;
+  }
+  atomicOr(t.err, kErrProbe);
+  return 0.0;
+}
+
+// Spatial RDMs from the spin blocks: rdm2 is the same-spin block from its
+// canonical p < q, r < s elements, and the
+// opposite spins (alpha, beta) + (beta, alpha) = ab[p][q][r][s] + ab[q][p][s][r].
+__global__ void __launch_bounds__(256) rdm_fold_kernel(RdmLaunch R, double norm, double* rdm1, double* rdm2) {
+  const int n = R.ham.norb;
+  const size_t n2 = static_cast<size_t>(n) * n, n4 = n2 * n2;
+  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n4;
+       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    if (i < n2) rdm1[i] = R.g1[i] * norm;
+    const unsigned pq = static_cast<unsigned>(i / n2), rs = static_cast<unsigned>(i - pq * n2);
+    const int p = pq / n, q = pq - p * n, r = rs / n, s = rs - r * n;
+    double same = 0.0;
+    if (p != q && r != s) {
+      const size_t c = idx4(n, min(p, q), max(p, q), min(r, s), max(r, s));
+      same = ((p < q) == (r < s) ? 1.0 : -1.0) * R.g2ss[c];
+    }
+    rdm2[i] = (same + R.g2ab[i] + R.g2ab[idx4(n, q, p, s, r)]) * norm;
+  }
+}
+
+// The diagonal terms of D: gamma_pp and Gamma_pqpq over its occupied pairs.
+__device__ void rdm_diagonal(const RdmLaunch& R, uint64_t a, uint64_t b, double w) {
+  const int n = R.ham.norb;
+  for (uint64_t u = a; u; u &= u - 1) {
+    const int p = __ffsll(static_cast<long long>(u)) - 1;
+    atomicAdd(R.g1 + static_cast<size_t>(p) * n + p, w);
+    for (uint64_t v = u & (u - 1); v; v &= v - 1) {
+      const int q = __ffsll(static_cast<long long>(v)) - 1;
+      atomicAdd(R.g2ss + idx4(n, p, q, p, q), w);
+    }
+    for (uint64_t v = b; v; v &= v - 1) {
+      const int q = __ffsll(static_cast<long long>(v)) - 1;
+      atomicAdd(R.g2ab + idx4(n, p, q, p, q), w);
+    }
+  }
+  for (uint64_t u = b; u; u &= u - 1) {
+    const int p = __ffsll(static_cast<long long>(u)) - 1;
+    atomicAdd(R.g1 + static_cast<size_t>(p) * n + p, w);
+    for (uint64_t v = u & (u - 1); v; v &= v - 1) {
+      const int q = __ffsll(static_cast<long long>(v)) - 1;
+      atomicAdd(R.g2ss + idx4(n, p, q, p, q), w);
+    }
+  }
+}
+
+// The terms of one connected pair D != D', w = x_D x_D'.  The orbitals that
+// leave (p, q) and come (r, s), in increasing order, are the bits that differ.
+__device__ void rdm_pair(const RdmLaunch& R, uint64_t a, uint64_t b, uint64_t a2, uint64_t b2, double w) {
+  const int n = R.ham.norb;
+  const auto low = [](uint64_t u) { return __ffsll(static_cast<long long>(u)) - 1; };
+  const uint64_t ha = a & ~a2, pa = a2 & ~a, hb = b & ~b2, pb = b2 & ~b;
+  if (ha && hb) {  // <a+_r(alpha) a+_s(beta) a_q(beta) a_p(alpha)>
+    const int p = low(ha), r = low(pa), q = low(hb), s = low(pb);
+    atomicAdd(R.g2ab + idx4(n, r, s, p, q), sign_ab(a, b, p, r, q, s) ? -w : w);
+    return;
+  }
+  const bool beta = hb != 0;
+  const uint64_t h = beta ? hb : ha, c = beta ? pb : pa;
+  const int p = low(h), r = low(c);
+  const uint64_t h2 = h & (h - 1), c2 = c & (c - 1);
+  if (h2) {  // <a+_r a+_s a_q a_p>, p < q, r < s
+    const int q = low(h2), s = low(c2);
+    const int neg = beta ? sign_bb(a, b, p, q, r, s) : sign_aa(a, b, p, q, r, s);
+    atomicAdd(R.g2ss + idx4(n, r, s, p, q), neg ? -w : w);
+    return;
+  }
+  // <a+_r a_p> and the spectators k: <a+_r a+_k a_k a_p>
+  if (beta ? sign_beta(a, b, p, r) : sign_alpha(a, b, p, r)) w = -w;
+  atomicAdd(R.g1 + static_cast<size_t>(r) * n + p, w);
+  for (uint64_t u = (beta ? b : a) & ~h; u; u &= u - 1) {
+    const int k = low(u);
+    const bool flip = (r < k) != (p < k);
+    atomicAdd(R.g2ss + idx4(n, min(r, k), max(r, k), min(p, k), max(p, k)), flip ? -w : w);
+  }
+  for (uint64_t u = beta ? a : b; u; u &= u - 1) {
+    const int k = low(u);
+    atomicAdd(R.g2ab + (beta ? idx4(n, k, r, k, p) : idx4(n, r, k, p, k)), w);
+  }
+}
+
+// Every two determinants of the list: a tile of kPairRows of them in shared
+// memory against one per thread.  Bound by the additions of the pairs that
+// connect (a warp runs them lane after lane).  8 rows a tile: 128 CTAs for the
+// 509 determinants of a short solve, whose matrices then take 20 us instead of
+// the 218 us of 7.4 million lookups.
+constexpr int kPairRows = 8;
+constexpr size_t kL2Bytes = static_cast<size_t>(126) << 20;
+__global__ void __launch_bounds__(256) rdm_pairs_kernel(RdmLaunch R) {
+  __shared__ Slot rows[kPairRows];
+  const long long tj = (R.nlist + 255) / 256, ti = (R.nlist + kPairRows - 1) / kPairRows;
+  for (long long tile = blockIdx.x; tile < ti * tj; tile += gridDim.x) {
+    const long long i0 = tile / tj * kPairRows, j = tile % tj * 256 + threadIdx.x;
+    const int rn = static_cast<int>(R.nlist - i0 < kPairRows ? R.nlist - i0 : kPairRows);
+    __syncthreads();  // the rows of the previous tile are no longer read
+    if (threadIdx.x < rn) rows[threadIdx.x] = R.list[i0 + threadIdx.x];
+    __syncthreads();
+    if (j >= R.nlist) continue;
+    const Slot d = R.list[j];
+    for (int i = 0; i < rn; ++i) {
+      const Slot& e = rows[i];
+      if (__popcll(d.a ^ e.a) + __popcll(d.b ^ e.b) > 4) continue;
+      if (i0 + i == j)
+        rdm_diagonal(R, d.a, d.b, d.x * d.x);
+      else
+        rdm_pair(R, d.a, d.b, e.a, e.b, d.x * e.x);
+    }
+  }
+}
+
+// One CTA per determinant of the list: every single and double excitation of
+// it looked up in the table.  Bound by the scattered loads of the slots.
+__global__ void __launch_bounds__(kNT) rdm_lookup_kernel(RdmLaunch R) {
   __shared__ Prelude P;
   const int n = R.ham.norb;
   const int warp = threadIdx.x >> 5;
   for (long long li = blockIdx.x; li < R.nlist; li += gridDim.x) {
-    const Slot* sd = R.tab.slots + R.list[li];
-    const Det D{sd->a, sd->b};
-    const double xd = sd->x;
+    const Det D{R.list[li].a, R.list[li].b};
+    const double xd = R.list[li].x;
     __syncthreads();  // P of the previous determinant is no longer read
     if (warp == 0) build_prelude(P, D, n);
     __syncthreads();
-    // Diagonal: gamma_pp, Gamma_pqpq over occupied pairs.
-    {
-      const double w = xd * xd;
-      const int na = P.na, nb = P.nb;
-      for (int t = threadIdx.x; t < na + nb; t += blockDim.x) {
-        if (t < na)
-          atomicAdd(R.g1a + static_cast<size_t>(P.occA[t]) * n + P.occA[t], w);
-        else
-          atomicAdd(R.g1b + static_cast<size_t>(P.occB[t - na]) * n + P.occB[t - na], w);
-      }
-      for (int t = threadIdx.x; t < na * na; t += blockDim.x) {
-        const int i = t / na, j = t - i * na;
-        if (i < j) {
-          const int p = P.occA[i], q = P.occA[j];
-          atomicAdd(R.g2aa + idx4(n, p, q, p, q), w);
-        }
-      }
-      for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) {
-        const int i = t / nb, j = t - i * nb;
-        if (i < j) {
-          const int p = P.occB[i], q = P.occB[j];
-          atomicAdd(R.g2bb + idx4(n, p, q, p, q), w);
-        }
-      }
-      for (int t = threadIdx.x; t < na * nb; t += blockDim.x) {
-        const int i = t / nb, j = t - i * nb;
-        const int p = P.occA[i], q = P.occB[j];
-        atomicAdd(R.g2ab + idx4(n, p, q, p, q), w);
-      }
-    }
-    // Excitations.
+    if (threadIdx.x == 0) rdm_diagonal(R, D.a, D.b, xd * xd);
     for (int e = 1 + threadIdx.x; e < P.total; e += blockDim.x) {
-      const uint64_t a = P.a, b = P.b;
-      int kind, p = 0, q = 0, r = 0, s = 0;
-      uint64_t a2, b2;
-      bool neg;
+      uint64_t a2 = D.a, b2 = D.b;
       if (e < P.off2) {
         const int t = e - 1;
         const int i = t / P.va;
-        p = P.occA[i];
-        r = P.virA[t - i * P.va];
-        kind = 1;
-        neg = sign_alpha(a, b, p, r);
-        a2 = a ^ (1ull << p) ^ (1ull << r);
-        b2 = b;
+        a2 ^= (1ull << P.occA[i]) ^ (1ull << P.virA[t - i * P.va]);
       } else if (e < P.off3) {
         const int t = e - P.off2;
         const int i = t / P.vb;
-        p = P.occB[i];
-        r = P.virB[t - i * P.vb];
-        kind = 2;
-        neg = sign_beta(a, b, p, r);
-        a2 = a;
-        b2 = b ^ (1ull << p) ^ (1ull << r);
+        b2 ^= (1ull << P.occB[i]) ^ (1ull << P.virB[t - i * P.vb]);
       } else if (e < P.off4) {
         const int t = e - P.off3;
         const int op = t / P.ca_vir, vp = t - op * P.ca_vir;
         int i, j, ri, sj;
         pair_decode(op, i, j);
         pair_decode(vp, ri, sj);
-        p = P.occA[i];
-        q = P.occA[j];
-        r = P.virA[ri];
-        s = P.virA[sj];
-        kind = 3;
-        neg = sign_aa(a, b, p, q, r, s);
-        a2 = a ^ (1ull << p) ^ (1ull << q) ^ (1ull << r) ^ (1ull << s);
-        b2 = b;
+        a2 ^= (1ull << P.occA[i]) ^ (1ull << P.occA[j]) ^ (1ull << P.virA[ri]) ^ (1ull << P.virA[sj]);
       } else if (e < P.off5) {
         const int t = e - P.off4;
         const int op = t / P.cb_vir, vp = t - op * P.cb_vir;
         int i, j, ri, sj;
         pair_decode(op, i, j);
         pair_decode(vp, ri, sj);
-        p = P.occB[i];
-        q = P.occB[j];
-        r = P.virB[ri];
-        s = P.virB[sj];
-        kind = 4;
-        neg = sign_bb(a, b, p, q, r, s);
-        a2 = a;
-        b2 = b ^ (1ull << p) ^ (1ull << q) ^ (1ull << r) ^ (1ull << s);
+        b2 ^= (1ull << P.occB[i]) ^ (1ull << P.occB[j]) ^ (1ull << P.virB[ri]) ^ (1ull << P.virB[sj]);
       } else {
         int t = e - P.off5;
         const int sbi = t % P.vb;
@@ -894,59 +951,11 @@ __global__ void __launch_bounds__(kNT) rdm_kernel(RdmLaunch R) {
         t /= P.va;
         const int pbi = t % P.nb;
         const int pai = t / P.nb;
-        p = P.occA[pai];  // alpha: p -> r
-        r = P.virA[rai];
-        q = P.occB[pbi];  // beta: q -> s
-        s = P.virB[sbi];
-        kind = 5;
-        neg = sign_ab(a, b, p, r, q, s);
-        a2 = a ^ (1ull << p) ^ (1ull << r);
-        b2 = b ^ (1ull << q) ^ (1ull << s);
+        a2 ^= (1ull << P.occA[pai]) ^ (1ull << P.virA[rai]);
+        b2 ^= (1ull << P.occB[pbi]) ^ (1ull << P.virB[sbi]);
       }
-      const long long slot = table_find(R.tab, a2, b2);
-      if (slot < 0) continue;
-      const double x2 = R.tab.slots[slot].x;
-      if (x2 == 0.0) continue;
-      const double w = neg ? -(xd * x2) : xd * x2;
-      switch (kind) {
-        case 1:  // <a+_r a_p> and the spectators k: <a+_r a+_k a_k a_p>
-          atomicAdd(R.g1a + static_cast<size_t>(r) * n + p, w);
-          for (int x = 0; x < P.na; ++x) {
-            const int k = P.occA[x];
-            if (k == p) continue;
-            int c1 = r, c2 = k, d1 = p, d2 = k;
-            const double sg = pair_canon(c1, c2) * pair_canon(d1, d2);
-            atomicAdd(R.g2aa + idx4(n, c1, c2, d1, d2), sg * w);
-          }
-          for (int x = 0; x < P.nb; ++x) {
-            const int k = P.occB[x];
-            atomicAdd(R.g2ab + idx4(n, r, k, p, k), w);
-          }
-          break;
-        case 2:
-          atomicAdd(R.g1b + static_cast<size_t>(r) * n + p, w);
-          for (int x = 0; x < P.nb; ++x) {
-            const int k = P.occB[x];
-            if (k == p) continue;
-            int c1 = r, c2 = k, d1 = p, d2 = k;
-            const double sg = pair_canon(c1, c2) * pair_canon(d1, d2);
-            atomicAdd(R.g2bb + idx4(n, c1, c2, d1, d2), sg * w);
-          }
-          for (int x = 0; x < P.na; ++x) {
-            const int k = P.occA[x];
-            atomicAdd(R.g2ab + idx4(n, k, r, k, p), w);
-          }
-          break;
-        case 3:  // <a+_r a+_s a_q a_p>, p < q, r < s
-          atomicAdd(R.g2aa + idx4(n, r, s, p, q), w);
-          break;
-        case 4:
-          atomicAdd(R.g2bb + idx4(n, r, s, p, q), w);
-          break;
-        default:  // <a+_r(alpha) a+_s(beta) a_q(beta) a_p(alpha)>
-          atomicAdd(R.g2ab + idx4(n, r, s, p, q), w);
-          break;
-      }
+      const double x2 = find_x(R.tab, a2, b2);
+      if (x2 != 0.0) rdm_pair(R, D.a, D.b, a2, b2, xd * x2);
     }
   }
 }
@@ -996,16 +1005,36 @@ cudaError_t launch_column_batch(const ColumnBatch& b, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_rdm_list(const TableDev& t, size_t capacity, unsigned* list, unsigned long long* count,
-                            unsigned long long cap, cudaStream_t s) {
-  rdm_list_kernel<<<148 * 8, 256, 0, s>>>(t.slots, capacity, list, count, cap);
+cudaError_t launch_collect_x(const TableDev& t, size_t capacity, Slot* list, unsigned long long* count,
+                             unsigned long long cap, cudaStream_t s) {
+  collect_x_kernel<<<148 * 8, 256, 0, s>>>(t.slots, capacity, list, count, cap);
   return cudaGetLastError();
 }
 
+cudaError_t launch_rdm_fold(const RdmLaunch& r, double norm, double* rdm1, double* rdm2, cudaStream_t s) {
+  rdm_fold_kernel<<<148 * 8, 256, 0, s>>>(r, norm, rdm1, rdm2);
+  return cudaGetLastError();
+}
+
+// N determinants with C excitations each take N^2 comparisons or N C lookups.
+// A comparison with the additions it leads to costs 8 to 13 ps of the chip, a
+// lookup 26 to 32 ps in a table in HBM, less in one the L2 holds.  Measured,
+// comparisons against lookups: 24 orbitals (C 14,469, 4.3 GB) N 509 0.55 and
+// 0.71 ms, N 9,700 1.7 and 4.9 ms, N 20,998 3.0 and 10.1 ms; 16 orbitals (C
+// 3,690, 1.1 GB) N 3,582 0.39 and 0.48 ms, N 14,647 1.83 and 1.62 ms; 10
+// orbitals (C 840, in L2) N 986 0.15 and 0.14 ms, N 5,740 0.53 and 0.29 ms.
+// Hence up to 3 C determinants are compared, up to C where the L2 holds the
+// table.
 cudaError_t launch_rdm(const RdmLaunch& r, cudaStream_t s) {
   if (r.nlist <= 0) return cudaSuccess;
-  const long long blocks = r.nlist < 148LL * 16 ? r.nlist : 148LL * 16;
-  rdm_kernel<<<static_cast<unsigned>(blocks), kNT, 0, s>>>(r);
+  const bool pairs = r.route ? r.route == 1 : r.nlist <= (r.tab.mask * sizeof(Slot) > kL2Bytes ? 3 : 1) * r.excitations;
+  if (pairs) {
+    const long long tiles = ((r.nlist + 255) / 256) * ((r.nlist + kPairRows - 1) / kPairRows);
+    rdm_pairs_kernel<<<static_cast<unsigned>(tiles < 148LL * 8 ? tiles : 148LL * 8), 256, 0, s>>>(r);
+  } else {
+    const long long blocks = r.nlist < 148LL * 16 ? r.nlist : 148LL * 16;
+    rdm_lookup_kernel<<<static_cast<unsigned>(blocks), kNT, 0, s>>>(r);
+  }
   return cudaGetLastError();
 }
 

@@ -34,14 +34,13 @@ __global__ void table_sums_kernel(const Slot* slots, size_t n, dd* partial, unsi
   __shared__ dd sxx[32], sxz[32];
   dd axx{0, 0}, axz{0, 0};
   unsigned long long c = 0;
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const Slot s = slots[i];
-    if (slot_vacant(s.a, s.b)) continue;
+  scan_slots(slots, n, [&](const Slot& s, size_t) {
+    if (slot_vacant(s.a, s.b)) return;
     ++c;
+    if (s.x == 0.0) return;
     axx = dd_add(axx, dd_two_prod(s.x, s.x));
     axz = dd_add(axz, dd_two_prod(s.x, s.z));
-  }
+  });
   axx = warp_sum_dd(axx);
   axz = warp_sum_dd(axz);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -66,17 +65,16 @@ __global__ void table_sums_kernel(const Slot* slots, size_t n, dd* partial, unsi
 // (z - e x)^2 and x^2 in double-double.  With z = H x (z_threshold = 0 keeps
 // every connected determinant), sqrt(sum (z - e x)^2 / sum x^2) with e =
 // x'z / x'x is ||H c - E c|| / ||c|| for the coefficients c = scale x.
+// Bound by the read of the table.
 __global__ void table_resid_kernel(const Slot* slots, size_t n, dd e, dd* partial) {
   __shared__ dd srr[32], sxx[32];
   dd arr{0, 0}, axx{0, 0};
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const Slot s = slots[i];
-    if (slot_vacant(s.a, s.b)) continue;
+  scan_slots(slots, n, [&](const Slot& s, size_t) {
+    if (slot_vacant(s.a, s.b)) return;
     const dd r = dd_add_d(dd_neg(dd_mul_d(e, s.x)), s.z);
     arr = dd_add(arr, dd_mul(r, r));
-    axx = dd_add(axx, dd_two_prod(s.x, s.x));
-  }
+    if (s.x != 0.0) axx = dd_add(axx, dd_two_prod(s.x, s.x));
+  });
   arr = warp_sum_dd(arr);
   axx = warp_sum_dd(axx);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -669,7 +667,8 @@ GpuSolver::GpuSolver(const Fcidump& fci, const SolverOptions& opt) : opt_(opt) {
                  o_sect = carve((kLeaderSections + kColumnSections) * sizeof(unsigned long long)),
                  o_pk = carve(parts * list_ * sizeof(unsigned long long)), o_ps = carve(parts * list_ * sizeof(unsigned)),
                  o_psum = carve(parts * kPartSum * sizeof(double)), o_done = carve(kMaxK * sizeof(unsigned)),
-                 o_bound = carve(kMaxK * sizeof(unsigned long long));
+                 o_bound = carve(kMaxK * sizeof(unsigned long long)),
+                 o_scan = carve(2 * kScanBlocks * sizeof(dd) + sizeof(unsigned long long));
     d_tables_ = device_alloc<unsigned char>(mo, "hamiltonian tables and iteration buffers");
     unsigned char* base = static_cast<unsigned char*>(d_tables_);
     auto up = [&](size_t o, const void* src, size_t bytes) {
@@ -708,6 +707,7 @@ GpuSolver::GpuSolver(const Fcidump& fci, const SolverOptions& opt) : opt_(opt) {
     d_part_sum_ = reinterpret_cast<double*>(mb + o_psum);
     d_done_ = reinterpret_cast<unsigned*>(mb + o_done);
     d_bound_ = reinterpret_cast<unsigned long long*>(mb + o_bound);
+    d_scan_ = mb + o_scan;
     check(cudaMemsetAsync(d_sect_, 0, (kLeaderSections + kColumnSections) * sizeof(unsigned long long), stream_),
           "memset");
     check(cudaMemsetAsync(d_done_, 0, kMaxK * sizeof(unsigned), stream_), "memset");
@@ -818,6 +818,9 @@ void GpuSolver::release() {
   if (stream_) cudaStreamSynchronize(stream_);
   cudaFree(d_tables_);
   if (own_table_) cudaFree(d_slots_);
+  cudaFree(d_read_);
+  d_read_ = nullptr;
+  read_bytes_ = 0;
   cudaFree(d_misc_);
   d_misc_ = nullptr;
   d_sect_ = nullptr;
@@ -826,6 +829,7 @@ void GpuSolver::release() {
   d_part_sum_ = nullptr;
   d_done_ = nullptr;
   d_bound_ = nullptr;
+  d_scan_ = nullptr;
   d_tables_ = nullptr;
   d_slots_ = nullptr;
   d_state_ = nullptr;
@@ -1202,111 +1206,109 @@ mcd_report GpuSolver::report() {
   return r;
 }
 
-void GpuSolver::wavefunction(std::vector<Det>& dets, std::vector<double>& x) {
-  read_state();
-  const unsigned long long cap = h_state_.x_size + 64;
-  unsigned* d_list = device_alloc<unsigned>(cap, "x list");
-  unsigned long long* d_count = nullptr;
-  try {
-    d_count = device_alloc<unsigned long long>(1, "x count");
-    check(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), stream_), "memset");
-    check(launch_rdm_list(td_, capacity_, d_list, d_count, cap, stream_), "x list");
-    unsigned long long cnt = 0;
-    check(cudaMemcpyAsync(&cnt, d_count, sizeof(cnt), cudaMemcpyDeviceToHost, stream_), "count read");
-    check(cudaStreamSynchronize(stream_), "synchronize");
-    if (cnt > cap) throw McdError(MCD_ERR_CUDA, "more nonzero coefficients than x_size counted");
-    std::vector<unsigned> list(cnt);
-    if (cnt) check(cudaMemcpy(list.data(), d_list, cnt * sizeof(unsigned), cudaMemcpyDeviceToHost), "list read");
-    std::sort(list.begin(), list.end());
-    dets.resize(cnt);
-    x.resize(cnt);
-    for (size_t i = 0; i < cnt; ++i) {
-      Slot sl;
-      check(cudaMemcpy(&sl, d_slots_ + list[i], sizeof(Slot), cudaMemcpyDeviceToHost), "slot read");
-      dets[i] = Det{sl.a, sl.b};
-      x[i] = sl.x;
-    }
-  } catch (...) {
-    cudaFree(d_list);
-    if (d_count) cudaFree(d_count);
-    throw;
+// Device scratch of the calls that read the wavefunction out, kept between them
+// up to kReadScratch (a device allocation and its release take 0.6 ms beside a
+// large table, as long as a scan of 4 GB).
+unsigned char* GpuSolver::read_scratch(size_t bytes) {
+  if (bytes > read_bytes_) {
+    cudaFree(d_read_);
+    d_read_ = nullptr;
+    read_bytes_ = 0;
+    const size_t want = std::max(bytes, static_cast<size_t>(2) << 20);
+    d_read_ = device_alloc<unsigned char>(want, "read-out scratch");
+    read_bytes_ = want;
   }
-  cudaFree(d_list);
-  cudaFree(d_count);
+  return d_read_;
 }
 
-void GpuSolver::rdm(std::vector<double>& rdm1, std::vector<double>& rdm2) {
+void GpuSolver::trim_read_scratch() {
+  if (read_bytes_ <= kReadScratch) return;
+  cudaFree(d_read_);
+  d_read_ = nullptr;
+  read_bytes_ = 0;
+}
+
+// The occupied slots with x != 0 into read_scratch: one scan of the table,
+// which writes each as {alpha, beta, x, slot index in z's place}.  *extra_at
+// (if given): `extra` bytes of the caller's behind the list, 256-byte aligned.
+Slot* GpuSolver::collect_x(unsigned long long* n, size_t extra, unsigned char** extra_at) {
+  for (unsigned long long cap = h_state_.x_size + 64;;) {
+    const size_t list_bytes = align_up(cap * sizeof(Slot), 256);
+    unsigned char* base = read_scratch(list_bytes + 256 + extra);
+    auto* d_count = reinterpret_cast<unsigned long long*>(base + list_bytes);
+    if (extra_at) *extra_at = base + list_bytes + 256;
+    check(cudaMemsetAsync(d_count, 0, sizeof(*n), stream_), "memset");
+    check(launch_collect_x(td_, capacity_, reinterpret_cast<Slot*>(base), d_count, cap, stream_), "x list");
+    check(cudaMemcpyAsync(n, d_count, sizeof(*n), cudaMemcpyDeviceToHost, stream_), "count read");
+    check(cudaStreamSynchronize(stream_), "synchronize");
+    if (*n <= cap) return reinterpret_cast<Slot*>(base);
+    cap = *n;
+  }
+}
+
+void GpuSolver::wavefunction(std::vector<Det>& dets, std::vector<double>& x) {
+  read_state();
+  unsigned long long n = 0;
+  const Slot* d_list = collect_x(&n, 0, nullptr);
+  std::vector<Slot> list(n);
+  if (n) {
+    check(cudaMemcpyAsync(list.data(), d_list, n * sizeof(Slot), cudaMemcpyDeviceToHost, stream_), "list read");
+    check(cudaStreamSynchronize(stream_), "synchronize");
+  }
+  trim_read_scratch();
+  // In slot order (the index, as a double, is exact).
+  std::sort(list.begin(), list.end(), [](const Slot& p, const Slot& q) { return p.z < q.z; });
+  dets.resize(n);
+  x.resize(n);
+  for (size_t i = 0; i < n; ++i) {
+    dets[i] = Det{list[i].a, list[i].b};
+    x[i] = list[i].x;
+  }
+}
+
+void GpuSolver::rdm(double* rdm1, double* rdm2, int route) {
   if (uhf_) throw McdError(MCD_ERR_UNSUPPORTED, "RDMs are implemented for RHF FCIDUMPs.");
   read_state();
   const int n = ham_.norb;
   const size_t n2 = static_cast<size_t>(n) * n, n4 = n2 * n2;
-  const unsigned long long cap = h_state_.x_size + 64;
-  std::vector<void*> owned;
-  auto alloc = [&](size_t bytes, const char* what) {
-    void* p = nullptr;
-    const cudaError_t e = cudaMalloc(&p, bytes);
-    if (e != cudaSuccess) {
-      for (void* q : owned) cudaFree(q);
-      throw McdError(MCD_ERR_CUDA, std::string("cudaMalloc(") + what + "): " + cudaGetErrorString(e));
-    }
-    owned.push_back(p);
-    return p;
-  };
+  const size_t out = n2 + n4, acc = n2 + 2 * n4;
+  unsigned long long cnt = 0;
+  unsigned char* extra = nullptr;
+  RdmLaunch r{};
+  r.list = collect_x(&cnt, (acc + out) * sizeof(double), &extra);
+  r.ham = hd_;
+  r.tab = td_;
+  r.nlist = static_cast<long long>(cnt);
+  r.excitations = static_cast<long long>(entries_);
+  r.route = route;
+  r.g1 = reinterpret_cast<double*>(extra);
+  r.g2ss = r.g1 + n2;
+  r.g2ab = r.g2ss + n4;
+  double* d_out = r.g2ab + n4;
+  // Out through a pinned block (a copy into pageable memory runs at a third of
+  // its rate), or straight when none is had.
+  const StagingBlock stage = staging_acquire(out * sizeof(double));
   try {
-    auto* d_list = static_cast<unsigned*>(alloc(cap * sizeof(unsigned), "rdm list"));
-    auto* d_count = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long), "rdm count"));
-    auto* d_g = static_cast<double*>(alloc((2 * n2 + 3 * n4) * sizeof(double), "rdm"));
-    check(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), stream_), "memset");
-    check(cudaMemsetAsync(d_g, 0, (2 * n2 + 3 * n4) * sizeof(double), stream_), "memset");
-    check(launch_rdm_list(td_, capacity_, d_list, d_count, cap, stream_), "rdm list");
-    unsigned long long cnt = 0;
-    check(cudaMemcpyAsync(&cnt, d_count, sizeof(cnt), cudaMemcpyDeviceToHost, stream_), "count read");
-    check(cudaStreamSynchronize(stream_), "synchronize");
-    if (cnt > cap) throw McdError(MCD_ERR_CUDA, "more nonzero coefficients than x_size counted");
-    RdmLaunch r{};
-    r.ham = hd_;
-    r.tab = td_;
-    r.list = d_list;
-    r.nlist = static_cast<long long>(cnt);
-    r.g1a = d_g;
-    r.g1b = d_g + n2;
-    r.g2aa = d_g + 2 * n2;
-    r.g2bb = r.g2aa + n4;
-    r.g2ab = r.g2bb + n4;
+    check(cudaMemsetAsync(r.g1, 0, acc * sizeof(double), stream_), "memset");
     check(launch_rdm(r, stream_), "rdm");
-    std::vector<double> g(2 * n2 + 3 * n4);
-    check(cudaMemcpyAsync(g.data(), d_g, g.size() * sizeof(double), cudaMemcpyDeviceToHost, stream_), "rdm read");
-    check(cudaStreamSynchronize(stream_), "synchronize");
-    for (void* q : owned) cudaFree(q);
-    owned.clear();
-    const double norm = 1.0 / dd_to_d(h_state_.xx);
-    const double* g1a = g.data();
-    const double* g1b = g1a + n2;
-    const double* aa = g1b + n2;
-    const double* bb = aa + n4;
-    const double* ab = bb + n4;
-    rdm1.assign(n2, 0.0);
-    rdm2.assign(n4, 0.0);
-    for (size_t i = 0; i < n2; ++i) rdm1[i] = (g1a[i] + g1b[i]) * norm;
-    auto I = [n](int p, int q, int r, int s) { return ((static_cast<size_t>(p) * n + q) * n + r) * n + s; };
-    for (int p = 0; p < n; ++p)
-      for (int q = 0; q < n; ++q)
-        for (int r = 0; r < n; ++r)
-          for (int s2 = 0; s2 < n; ++s2) {
-            // Same-spin blocks from their canonical p < q, r < s elements.
-            double same = 0.0;
-            if (p != q && r != s2) {
-              const int cp = p < q ? p : q, cq = p < q ? q : p, cr = r < s2 ? r : s2, cs = r < s2 ? s2 : r;
-              const double sg = ((p < q) ? 1.0 : -1.0) * ((r < s2) ? 1.0 : -1.0);
-              same = sg * (aa[I(cp, cq, cr, cs)] + bb[I(cp, cq, cr, cs)]);
-            }
-            // Opposite spins: (alpha, beta) + (beta, alpha) = ab[p][q][r][s] + ab[q][p][s][r].
-            rdm2[I(p, q, r, s2)] = (same + ab[I(p, q, r, s2)] + ab[I(q, p, s2, r)]) * norm;
-          }
+    check(launch_rdm_fold(r, 1.0 / dd_to_d(h_state_.xx), d_out, d_out + n2, stream_), "rdm fold");
+    if (stage.p) {
+      check(cudaMemcpyAsync(stage.p, d_out, out * sizeof(double), cudaMemcpyDeviceToHost, stream_), "rdm read");
+      check(cudaStreamSynchronize(stream_), "synchronize");
+      std::memcpy(rdm1, stage.p, n2 * sizeof(double));
+      std::memcpy(rdm2, static_cast<double*>(stage.p) + n2, n4 * sizeof(double));
+    } else {
+      check(cudaMemcpyAsync(rdm1, d_out, n2 * sizeof(double), cudaMemcpyDeviceToHost, stream_), "rdm read");
+      check(cudaMemcpyAsync(rdm2, d_out + n2, n4 * sizeof(double), cudaMemcpyDeviceToHost, stream_), "rdm read");
+      check(cudaStreamSynchronize(stream_), "synchronize");
+    }
   } catch (...) {
-    for (void* q : owned) cudaFree(q);
+    cudaStreamSynchronize(stream_);
+    staging_release(stage);
     throw;
   }
+  staging_release(stage);
+  trim_read_scratch();
 }
 
 unsigned long long GpuSolver::compact(double z_threshold) {
@@ -1737,9 +1739,9 @@ std::vector<double> GpuSolver::hsub(const std::vector<Det>& dets) {
 
 void GpuSolver::table_sums(dd* xx, dd* xz, unsigned long long* occupied) {
   read_state();
-  const int nb = 148 * 4;
-  dd* dp = device_alloc<dd>(2 * nb, "debug");
-  unsigned long long* dc = device_alloc<unsigned long long>(1, "debug");
+  const int nb = kScanBlocks;
+  auto* dp = reinterpret_cast<dd*>(d_scan_);
+  auto* dc = reinterpret_cast<unsigned long long*>(dp + 2 * nb);
   std::vector<dd> hp(2 * nb);
   unsigned long long c = 0;
   check(cudaMemsetAsync(dc, 0, 8, stream_), "memset");
@@ -1747,8 +1749,6 @@ void GpuSolver::table_sums(dd* xx, dd* xz, unsigned long long* occupied) {
   check(cudaMemcpyAsync(hp.data(), dp, hp.size() * sizeof(dd), cudaMemcpyDeviceToHost, stream_), "copy");
   check(cudaMemcpyAsync(&c, dc, 8, cudaMemcpyDeviceToHost, stream_), "copy");
   check(cudaStreamSynchronize(stream_), "sync");
-  cudaFree(dp);
-  cudaFree(dc);
   dd a{0, 0}, b{0, 0};
   for (int i = 0; i < nb; ++i) {
     a = dd_add(a, hp[2 * i]);
@@ -1761,8 +1761,8 @@ void GpuSolver::table_sums(dd* xx, dd* xz, unsigned long long* occupied) {
 
 double GpuSolver::residual() {
   read_state();
-  const int nb = 148 * 4;
-  dd* dp = device_alloc<dd>(2 * nb, "residual");
+  const int nb = kScanBlocks;
+  auto* dp = reinterpret_cast<dd*>(d_scan_);
   std::vector<dd> hp(2 * nb);
   const dd e = dd_div(h_state_.xz, h_state_.xx);
   table_resid_kernel<<<nb, 256, 0, stream_>>>(d_slots_, capacity_, e, dp);
@@ -1770,7 +1770,6 @@ double GpuSolver::residual() {
   if (err == cudaSuccess)
     err = cudaMemcpyAsync(hp.data(), dp, hp.size() * sizeof(dd), cudaMemcpyDeviceToHost, stream_);
   if (err == cudaSuccess) err = cudaStreamSynchronize(stream_);
-  cudaFree(dp);
   check(err, "residual");
   dd rr{0, 0}, xx{0, 0};
   for (int i = 0; i < nb; ++i) {

@@ -100,7 +100,8 @@ class GpuSolver {
   // (rdm1[P*n+Q] = sum_s <a+_{Ps} a_{Qs}>, rdm2[((P*n+Q)*n+R)*n+S] =
   // sum_{s,t} <a+_{Ps} a+_{Qt} a_{St} a_{Rs}>, n spatial orbitals), so that
   // E = sum h_PQ rdm1 + 1/2 sum (PR|QS) rdm2 + E_core.
-  void rdm(std::vector<double>& rdm1, std::vector<double>& rdm2);
+  // rdm1 and rdm2: n^2 and n^4 doubles; route as RdmLaunch::route.
+  void rdm(double* rdm1, double* rdm2, int route = 0);
   // Raise z_threshold to `z_threshold` and remove the entries with x = 0 and
   // |z scale| <= z_threshold, rebuilding the table; returns the occupied slots.
   unsigned long long compact(double z_threshold);
@@ -162,6 +163,9 @@ class GpuSolver {
   void read_state();
   void raise_device_error();
   void build_graph();
+  unsigned char* read_scratch(size_t bytes);
+  void trim_read_scratch();
+  Slot* collect_x(unsigned long long* n, size_t extra, unsigned char** extra_at);
   void gather_slots(double zlim, std::vector<Slot>& out);  // occupied slots kept by zlim, in slot order
   // Table growth: before `upcoming` iterations are enqueued, make sure that
   // the table keeps its load below 3/4 even if every one of them inserts a
@@ -228,6 +232,11 @@ class GpuSolver {
   double* d_part_sum_ = nullptr;
   unsigned* d_done_ = nullptr;
   unsigned long long* d_bound_ = nullptr;
+  static constexpr int kScanBlocks = 148 * 4;  // of the whole-table scans
+  unsigned char* d_scan_ = nullptr;            // their partial sums
+  static constexpr size_t kReadScratch = static_cast<size_t>(128) << 20;
+  unsigned char* d_read_ = nullptr;
+  size_t read_bytes_ = 0;
   HamDev hd_{};
   TableDev td_{};
   ColumnLaunch cl_{};

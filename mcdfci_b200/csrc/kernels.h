@@ -136,16 +136,18 @@ static_assert(sizeof(LeaderBatch) <= 32000 && sizeof(ColumnBatch) <= 32000, "ker
 
 // Reduced density matrices of the wavefunction in the table, unnormalised
 // (divide by sum x^2), in spin blocks over spatial orbitals (n = ham.norb):
-//   g1a[r*n+p]          = sum <a+_{r alpha} a_{p alpha}>           (g1b: beta)
-//   g2aa[((p*n+q)*n+r)*n+s], p < q, r < s only
-//                       = sum <a+_p a+_q a_s a_r> (all alpha)      (g2bb: beta)
+//   g1[r*n+p] = sum <a+_r a_p>, both spins
+//   g2ss[((p*n+q)*n+r)*n+s], p < q, r < s only
+//             = sum <a+_p a+_q a_s a_r>, all alpha and all beta
 //   g2ab[((p*n+q)*n+r)*n+s] = sum <a+_{p alpha} a+_{q beta} a_{s beta} a_{r alpha}>
 struct RdmLaunch {
   HamDev ham;
   TableDev tab;
-  const unsigned* list;  // slots of the determinants with x != 0
+  const Slot* list;  // the determinants with x != 0, and their x
   long long nlist;
-  double *g1a, *g1b, *g2aa, *g2bb, *g2ab;
+  long long excitations;  // of each determinant
+  int route;              // 0 by launch_rdm's rule, 1 all pairs, 2 lookups
+  double *g1, *g2ss, *g2ab;
 };
 
 // Phases of the leader kernel timed into LeaderLaunch::sect: 0 state load,
@@ -211,10 +213,13 @@ cudaError_t launch_table_fill(Slot* slots, size_t n, cudaStream_t s);
 cudaError_t launch_table_sums(const Slot* slots, size_t n, dd* partial, unsigned long long* count, int nblocks,
                               cudaStream_t s);
 
-// Slots with x != 0 into list (up to cap; *count receives the total).
-cudaError_t launch_rdm_list(const TableDev& t, size_t capacity, unsigned* list, unsigned long long* count,
-                            unsigned long long cap, cudaStream_t s);
+// Slots with x != 0 into list (up to cap; *count receives the total), with
+// their index, as a double, in z's place.
+cudaError_t launch_collect_x(const TableDev& t, size_t capacity, Slot* list, unsigned long long* count,
+                             unsigned long long cap, cudaStream_t s);
 cudaError_t launch_rdm(const RdmLaunch& r, cudaStream_t s);
+// The spin-summed spatial RDMs times norm, from r's spin blocks.
+cudaError_t launch_rdm_fold(const RdmLaunch& r, double norm, double* rdm1, double* rdm2, cudaStream_t s);
 
 // Debug / parity entry points (synchronous).
 // Column of one determinant: writes up to `cap` (a, b, value) entries.
