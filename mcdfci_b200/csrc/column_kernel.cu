@@ -522,10 +522,11 @@ __device__ __forceinline__ int confirm_picked(const IterState* St, ColumnShared&
 // One CTA's share of one column: CTA `blk` of the launch described by L
 // (column blk / groups, slice blk % groups).  kOverlap: launched to start
 // beside the leader; the first block is probed from the determinants as the
-// leader publishes them when it has picked, while it solves for dx.
-template <bool kOverlap>
+// leader publishes them when it has picked, while it solves for dx.  kSingle:
+// groups is 1.
+template <bool kOverlap, bool kSingle>
 __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
-  const int G = L.groups;
+  const int G = kSingle ? 1 : L.groups;
   const int col = blk / G;
   const int g = blk - col * G;
   IterState* St = L.st;
@@ -580,7 +581,7 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
         atomicAdd(L.sect + 5, static_cast<unsigned long long>(c_rounds - c_start));
         atomicAdd(L.sect + 8, 1ull);
       }
-      if (tid < M) {
+      if (!kSingle && tid < M) {
         L.part_key[part * M + tid] = tid < n_list ? S.list_key[tid] : 0ull;
         L.part_slot[part * M + tid] = tid < n_list ? S.list_slot[tid] : 0u;
       }
@@ -605,7 +606,7 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
         __syncwarp();
         // One fence for the whole CTA's list and sums (the barriers order
         // them before it), then the ticket.
-        if (lane == 0) {
+        if (!kSingle && lane == 0) {
           if (bound != 0ull) atomicMax(L.bound + col, bound);
           __threadfence();
           S.last = (atomicAdd(L.done + col, 1u) == static_cast<unsigned>(G - 1));
@@ -614,6 +615,7 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
       __syncthreads();
       c_merge = timed ? clock64() : 0;
       if (timed) atomicAdd(L.sect + 6, static_cast<unsigned long long>(c_merge - c_post));
+      if (kSingle) break;  // the CTA's list is the column's
       if (!S.last) return;
       __threadfence();
       merging = true;
@@ -678,7 +680,9 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
   }
   if (tid < L.m)
     L.cand_slot[static_cast<size_t>(col) * L.m + tid] =
-        tid < n_list ? __ldcg(L.part_slot + static_cast<size_t>(col) * G * M + S.list_slot[tid]) : kNoSlot;
+        tid >= n_list ? kNoSlot
+        : kSingle    ? S.list_slot[tid]
+                     : __ldcg(L.part_slot + static_cast<size_t>(col) * G * M + S.list_slot[tid]);
   if (warp < kPartSum) {
     // Column sums in a fixed order, one per warp: lane-strided partials, then a fixed tree.
     double t = 0.0;
@@ -716,9 +720,9 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
   }
 }
 
-template <bool kOverlap>
+template <bool kOverlap, bool kSingle>
 __global__ void __launch_bounds__(kNT, kColumnCtasPerSm) column_kernel(ColumnLaunch L) {
-  column_body<kOverlap>(L, blockIdx.x);
+  column_body<kOverlap, kSingle>(L, blockIdx.x);
 }
 
 // Several instances in one grid: CTAs [cta_begin[i], cta_begin[i+1]) belong
@@ -732,7 +736,7 @@ __global__ void __launch_bounds__(kNT, kColumnCtasPerSm) column_kernel_batch(Col
     else
       hi = mid;
   }
-  column_body<false>(B.L[lo], static_cast<int>(blockIdx.x) - B.cta_begin[lo]);
+  column_body<false, false>(B.L[lo], static_cast<int>(blockIdx.x) - B.cta_begin[lo]);
 }
 
 __global__ void __launch_bounds__(kNT) debug_column_kernel(HamDev h, Det d, double hd, uint64_t* ao,
@@ -990,12 +994,20 @@ int column_groups(int entries, int k, int resident) {
   return g < 1 ? 1 : g;
 }
 
-bool column_overlaps(int ctas, int sms) { return ctas <= kColumnCtasPerSm * (sms - 1); }
+// Up to four waves of CTAs beside the leader's SM.  96 columns of 15 CTAs (64
+// iterations of 24 orbitals): 14.4 ms started early, 14.9 ms after the
+// leader.  64 columns of 96 CTAs (42 orbitals): 24.15 and 24.07 ms, the first
+// wave being too small a part to pay for the second reading of x.
+bool column_overlaps(int ctas, int sms) { return ctas <= 4 * kColumnCtasPerSm * (sms - 1); }
 
 cudaError_t launch_column(const ColumnLaunch& a, cudaStream_t s) {
   const dim3 grid(a.k_grid * a.groups), block(kNT);
-  if (a.overlap) return launch_overlapped(column_kernel<true>, grid, block, 0, s, a);
-  column_kernel<false><<<grid, block, 0, s>>>(a);
+  // One CTA a column: no ticket, no lists in global memory, no merge.  600
+  // iterations of 8 columns of 171 entries 14.3 ms, 16.4 ms with them.
+  const bool single = a.groups == 1;
+  if (a.overlap)
+    return launch_overlapped(single ? column_kernel<true, true> : column_kernel<true, false>, grid, block, 0, s, a);
+  (single ? column_kernel<false, true> : column_kernel<false, false>)<<<grid, block, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -69,3 +69,24 @@ def test_first_candidates_are_the_largest(problems, sector, spread, mm, groups):
     assert len(set(picked)) == len(picked) == len(want)
     got = np.sort(np.array([score[d] for d in picked]))[::-1]
     assert np.all(np.abs(got - want) <= 1e-12 * want)
+
+
+@pytest.mark.parametrize("groups", [1, 60, 96])
+def test_launch_forms_agree(problems, groups):
+    """One CTA a column, several waves of CTAs started beside the leader, and
+    more waves than that, against one wave: 32 columns, the same table and
+    energy after a few iterations up to the order of the sums (64-bit sums of
+    at most 1e5 terms, 1e-16 each, relative to the energy)."""
+    path, _ = problems[19, 0]
+    sums = []
+    for g in (18, groups):
+        s = m.CDFCI(m.Fcidump(path), num_of_coordinate=32, estimate=128, max_memory=0.05, threshold=0.0,
+                    z_threshold=0.0, groups=g)
+        s.reset()
+        s.run_iterations(6)
+        r = s.report()
+        sums.append((r["energy"], r["z_size"], r["x_size"], s.table_sums()))
+        s.close()
+    (e0, z0, x0, t0), (e1, z1, x1, t1) = sums
+    assert abs(e0 - e1) <= 1e-11 * abs(e0)
+    assert (z0, x0, t0["occupied"]) == (z1, x1, t1["occupied"])
