@@ -55,6 +55,7 @@ class GpuBatch {
     cudaGraphExec_t graph = nullptr;
   };
   void join_streams();
+  void read_states();
   void launch_iteration(Group& g);
   void build_graphs();
   // The groups' launch descriptors over the active instances (instance i in
@@ -71,6 +72,7 @@ class GpuBatch {
   std::vector<double> energies_;
   std::vector<char> active_;
   Slot* pool_ = nullptr;  // every instance's hash table, one allocation
+  GpuSolver::StateRead* reads_ = nullptr;  // one per instance, pinned
 };
 
 }  // namespace mcd

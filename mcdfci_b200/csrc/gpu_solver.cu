@@ -851,12 +851,12 @@ void GpuSolver::release() {
   own_stream_ = false;
 }
 
-void GpuSolver::reset() {
+void GpuSolver::reset(bool wait) {
   const auto t0 = std::chrono::steady_clock::now();
   check(launch_table_fill(d_slots_, capacity_, stream_), "table fill");
   check(cudaMemsetAsync(d_err_, 0, sizeof(unsigned), stream_), "memset");
   check(cudaMemsetAsync(d_occ_, 0, sizeof(unsigned long long), stream_), "memset");
-  check(cudaStreamSynchronize(stream_), "table fill");
+  if (wait) check(cudaStreamSynchronize(stream_), "table fill");
   setup_ms_[3] = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   std::memset(&h_state_, 0, sizeof(h_state_));
   h_state_.zt = zt_;
@@ -1159,28 +1159,48 @@ void GpuSolver::run_iterations_timed(long long n, double* leader_ms, double* col
   for (auto& e : ev) cudaEventDestroy(e);
 }
 
-void GpuSolver::read_state() {
+void GpuSolver::enqueue_state_read(StateRead* r) {
   check(launch_finish(ll_, stream_), "finish");
-  check(cudaMemcpyAsync(&h_state_, d_state_, sizeof(IterState), cudaMemcpyDeviceToHost, stream_), "state read");
-  unsigned err = 0;
-  check(cudaMemcpyAsync(&err, d_err_, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_), "error read");
-  check(cudaStreamSynchronize(stream_), "synchronize");
-  if (err) {
-    if (err & (kErrProbe | kErrOverflow))
+  check(cudaMemcpyAsync(&r->state, d_state_, sizeof(IterState), cudaMemcpyDeviceToHost, stream_), "state read");
+  check(cudaMemcpyAsync(&r->err, d_err_, sizeof(unsigned), cudaMemcpyDeviceToHost, stream_), "error read");
+  check(cudaMemcpyAsync(&r->occupied, d_occ_, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream_),
+        "occupancy read");
+}
+
+void GpuSolver::take_state(const StateRead& r) {
+  h_state_ = r.state;
+  if (r.err) {
+    if (r.err & (kErrProbe | kErrOverflow))
       throw McdError(MCD_ERR_OVERFLOW, "The hash table is full. Please increase max_memory or z_threshold.");
-    if (err & kErrEig)
+    if (r.err & kErrEig)
       throw McdError(MCD_ERR_EIG,
                      "The subspace eigenvalue problem failed (its lowest eigenvalue must be negative: the method "
                      "minimises ||H + x x^T||_F^2, which needs a negative ground-state energy; a positive core "
                      "energy in the FCIDUMP can make it positive).");
-    if (err & kErrCandidates) throw McdError(MCD_ERR_NO_CANDIDATES, "The candidate list is empty.");
-    throw McdError(MCD_ERR_CUDA, "device error word " + std::to_string(err));
+    if (r.err & kErrCandidates) throw McdError(MCD_ERR_NO_CANDIDATES, "The candidate list is empty.");
+    throw McdError(MCD_ERR_CUDA, "device error word " + std::to_string(r.err));
   }
+}
+
+void GpuSolver::read_state() {
+  StateRead r;
+  enqueue_state_read(&r);
+  check(cudaStreamSynchronize(stream_), "synchronize");
+  take_state(r);
 }
 
 mcd_report GpuSolver::report() {
   const auto t0 = std::chrono::steady_clock::now();
-  read_state();
+  StateRead s;
+  enqueue_state_read(&s);
+  check(cudaStreamSynchronize(stream_), "synchronize");
+  const mcd_report r = report_of(s);
+  setup_ms_[6] += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+  return r;
+}
+
+mcd_report GpuSolver::report_of(const StateRead& s) {
+  take_state(s);
   mcd_report r{};
   r.iteration = h_state_.iter;
   const dd xz{dd_to_d(h_state_.xz), 0.0};
@@ -1195,8 +1215,7 @@ mcd_report GpuSolver::report() {
   r.z_threshold = zt_;
   r.emitted_total = h_state_.emitted_total;
   r.updates_total = h_state_.updates_total;
-  r.occupied = 0;
-  check(cudaMemcpy(&r.occupied, d_occ_, sizeof(unsigned long long), cudaMemcpyDeviceToHost), "occupancy read");
+  r.occupied = s.occupied;
   r.last_k = h_state_.k_cur;
   r.inv_steps_last = h_state_.inv_steps_curr;
   r.inv_updates = h_state_.inv_updates;
@@ -1205,7 +1224,6 @@ mcd_report GpuSolver::report() {
   r.max_abs_evec = h_state_.max_abs_evec;
   occ_exact_ = r.occupied;
   occ_exact_iters_ = iters_enqueued_;
-  setup_ms_[6] += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   return r;
 }
 

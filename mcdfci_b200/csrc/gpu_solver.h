@@ -69,7 +69,8 @@ class GpuSolver {
   // Full solve with reports and z_threshold_search restarts.
   int solve(mcd_report_cb cb, void* user);
   // Initial state with the current z_threshold.
-  void reset();
+  // wait: until the table is filled (its time is a set-up time).
+  void reset(bool wait = true);
   // Enqueue n iterations (asynchronous).
   void run_iterations(long long n);
   // Run n iterations with direct launches and a CUDA event between every
@@ -78,6 +79,16 @@ class GpuSolver {
   void run_iterations_timed(long long n, double* leader_ms, double* column_ms, double* total_ms);
   // Apply the pending end-of-iteration step, wait, and read the state.
   mcd_report report();
+  // report() in two steps, for callers with several solvers to read: the
+  // copies are enqueued on the solver's stream (into pinned memory, or they
+  // wait for it), and after it has been waited for, the report made of them.
+  struct StateRead {
+    IterState state;
+    unsigned long long occupied;
+    unsigned err;
+  };
+  void enqueue_state_read(StateRead* r);
+  mcd_report report_of(const StateRead& r);
 
   double result_energy() const { return result_energy_; }
   cudaStream_t stream() const { return stream_; }
@@ -161,6 +172,7 @@ class GpuSolver {
   void check(cudaError_t e, const char* what);
   void release();
   void read_state();
+  void take_state(const StateRead& r);
   void raise_device_error();
   void build_graph();
   unsigned char* read_scratch(size_t bytes);
