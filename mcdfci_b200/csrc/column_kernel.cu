@@ -44,10 +44,11 @@
 // slot, one record per entry in shared memory.  The second needs dx: it adds
 // to z (inserting where the rule says so) and scores the entry.
 //
-// Overlap.  When all CTAs of a launch fit beside the leader's (one SM is its
-// own), they start while it runs (programmatic dependent launch): the leader
-// publishes its picks before it builds and solves the subspace problem, and
-// the CTAs probe their first block meanwhile, then wait for its end.  Keys do
+// Overlap.  Launches of up to four waves of CTAs beside the leader's SM
+// (column_overlaps) are enqueued with programmatic dependent launch: the first
+// CTAs start while the leader runs.  It publishes its picks before it builds
+// and solves the subspace problem, and the CTAs probe their first block
+// meanwhile, then wait for its end.  Keys do
 // not change while the leader runs; x does, on the picked determinants, so the
 // slots that a small filter of these holds have x read again.  What was read
 // before the wait is compared with the final picks after it.  The leader in
@@ -56,8 +57,7 @@
 // overlapped: 7 orbitals, k = 8, 600 iterations 18.6 and 16.8 ms; 12 orbitals,
 // k = 32, 256 iterations 10.7 and 10.3 ms; 24 orbitals, k = 32, 256 iterations
 // 20.8 and 19.3 ms (with the launch overlapped but the probes after the wait,
-// 21.9 ms).  Launches of more CTAs keep the order: the first wave's probes
-// would hide little, and its idle CTAs hold the others back.
+// 21.9 ms).
 //
 // Candidates.  The keys of a block and the CTA's list so far (at most m) are
 // reduced to the m largest by a radix selection over the whole CTA
@@ -70,6 +70,7 @@
 // it are dropped before the selection.
 #include "device_common.cuh"
 #include <algorithm>
+#include <cstddef>
 
 #include "kernels.h"
 #include "select.cuh"
@@ -302,6 +303,8 @@ struct alignas(16) ColumnShared {
   unsigned long long list_key[kMaxM];    // the CTA's candidates so far
   unsigned list_slot[kMaxM];
   SelectScratch sel;
+  double newz[kNT], dot[kNT];  // the threads' sums and counts so far
+  unsigned emit[kNT], upd[kNT], ins[kNT];
   double w_sum[kPartSum][kW];
   double dx, hdiag, zt;  // the column's scalars
   dd xss, scale;
@@ -311,39 +314,103 @@ struct alignas(16) ColumnShared {
   int last, some;
 };
 
-// Reduces the CTA's candidates, S.list's n_list and the keys k[0..kRounds) (0:
-// none) with payloads p, to the m largest in S.list, in no particular order.
-// Returns how many there are, and raises `bound` to the smallest value a kept
-// key can have when some were left out.  k[kRounds], p[kRounds] are scratch.
-// Called by the whole CTA; ends with a barrier.
-__device__ __forceinline__ int cta_select(ColumnShared& S, unsigned long long (&k)[kRounds + 1],
-                                          unsigned (&p)[kRounds + 1], int n_list, int m, unsigned long long& bound) {
+struct Selected {
+  int n_list;
+  unsigned long long bound;
+};
+
+// Reduces the CTA's candidates, S.list's n_list and the keys of n / kBlock
+// whole blocks from S.val on (0 and those below `bound` left out), to the m largest in S.list, in no
+// particular order.  Their payloads: the slots in S.rec, or base + index when
+// base is not kNoSlot.  Raises `bound` to the smallest value a kept key can
+// have when some were left out.  Called by the whole CTA, each thread having
+// written the keys tid + j kNT itself (0 beyond the last); ends with a barrier.  One copy of the
+// code, out of line, serves a CTA's blocks and the merge of the lists: the
+// rounds keep their registers, and a column's last CTA finds its instructions
+// in the cache.
+__device__ __noinline__ Selected cta_select(ColumnShared* s, int n, unsigned base, int n_list, int m,
+                                            unsigned long long bound) {
+  __builtin_assume(__isShared(s));
+  ColumnShared& S = *s;
+  const unsigned long long* pool = &S.val[0][0];
   const int tid = threadIdx.x;
+  const unsigned long long floor = bound > 1ull ? bound : 1ull;
   bool any = false;
+#pragma unroll 1
+  for (int i = tid; i < n; i += kRounds * kNT)
 #pragma unroll
-  for (int j = 0; j < kRounds; ++j) any |= k[j] != 0ull;
-  if (!__syncthreads_or(any)) return n_list;  // nothing new above the bound
-  k[kRounds] = tid < n_list ? S.list_key[tid] : 0ull;
-  p[kRounds] = tid < n_list ? S.list_slot[tid] : 0u;
+    for (int j = 0; j < kRounds; ++j) any |= pool[i + j * kNT] >= floor;
+  if (!__syncthreads_or(any)) return Selected{n_list, bound};  // nothing new above the bound
+  const unsigned long long list_key = tid < n_list ? S.list_key[tid] : 0ull;
+  const unsigned list_slot = tid < n_list ? S.list_slot[tid] : 0u;
   if (tid == 0) {
     S.out = 0u;
     S.ties = 0u;
   }
   const unsigned want = static_cast<unsigned>(m);
   const SelectEdge E = select_edge(S.sel, want, [&](auto f) {
+    f(list_key);
+#pragma unroll 1
+    for (int i = tid; i < n; i += kRounds * kNT) {
+      unsigned long long key[kRounds];
 #pragma unroll
-    for (int j = 0; j <= kRounds; ++j) f(k[j]);
+      for (int j = 0; j < kRounds; ++j) key[j] = pool[i + j * kNT];
+#pragma unroll
+      for (int j = 0; j < kRounds; ++j) f(key[j] >= floor ? key[j] : 0ull);
+    }
   });
-#pragma unroll
-  for (int j = 0; j <= kRounds; ++j) {
-    if (k[j] < E.edge || (E.tied && k[j] == E.edge && atomicAdd(&S.ties, 1u) >= E.need)) continue;
+  const unsigned long long least = E.edge > floor ? E.edge : floor;
+  const auto keep = [&](unsigned long long key, unsigned slot) {
+    if (E.tied && key == E.edge && atomicAdd(&S.ties, 1u) >= E.need) return;
     const unsigned pos = atomicAdd(&S.out, 1u);
-    S.list_key[pos] = k[j];
-    S.list_slot[pos] = p[j];
+    S.list_key[pos] = key;
+    S.list_slot[pos] = slot;
+  };
+  if (list_key >= E.edge) keep(list_key, list_slot);
+#pragma unroll 1
+  for (int i0 = tid; i0 < n; i0 += kRounds * kNT) {
+    unsigned long long key[kRounds];
+#pragma unroll
+    for (int j = 0; j < kRounds; ++j) key[j] = pool[i0 + j * kNT];
+#pragma unroll
+    for (int j = 0; j < kRounds; ++j) {
+      const int i = i0 + j * kNT;
+      if (key[j] >= least)
+        keep(key[j], base == kNoSlot ? static_cast<unsigned>((&S.rec[0][0])[i]) : base + static_cast<unsigned>(i));
+    }
   }
-  if (E.total > want && E.edge > bound) bound = E.edge;
+  if (E.total > want) bound = least;
   __syncthreads();
-  return static_cast<int>(min(E.total, want));
+  return Selected{static_cast<int>(min(E.total, want)), bound};
+}
+
+// The m largest of the n keys of a column's lists, those below `bound` (which m
+// keys reach) left out, into S.list with their indexes: up to 3,072 keys at a
+// time in the shared memory of the rounds, where 1,024 at a time in registers
+// took a selection for each (23 lists of 128: 200 iterations of 24 columns
+// 10.9 ms, now 10.25; 96 lists of 128: 24.2 and 23.9 ms for 16 of 64 columns).
+__device__ __forceinline__ int merge_lists(ColumnShared& S, const unsigned long long* keys, int n, int m,
+                                           unsigned long long bound) {
+  constexpr int kKeys = 3 * kRounds * kNT;
+  static_assert(offsetof(ColumnShared, rec) == offsetof(ColumnShared, val) + sizeof(S.val) &&
+                    offsetof(ColumnShared, x) == offsetof(ColumnShared, rec) + sizeof(S.rec),
+                "the rounds' arrays follow one another");
+  unsigned long long* pool = &S.val[0][0];
+  Selected r{0, bound};
+#pragma unroll 1
+  for (int at = 0; at < n; at += kKeys) {
+    const int some = min(n - at, kKeys);
+#pragma unroll 1
+    for (int i = threadIdx.x; i < some; i += kRounds * kNT) {
+      unsigned long long key[kRounds];
+#pragma unroll
+      for (int j = 0; j < kRounds; ++j) key[j] = i + j * kNT < some ? __ldcg(keys + at + i + j * kNT) : 0ull;
+#pragma unroll
+      for (int j = 0; j < kRounds; ++j) pool[i + j * kNT] = key[j];
+    }
+    r = cta_select(&S, some, static_cast<unsigned>(at), r.n_list, m, r.bound);
+  }
+  return r.n_list;
 }
 
 // Continues a probe at slot i, which was empty when the first phase ended
@@ -441,13 +508,13 @@ __device__ __forceinline__ void block_probe(const ColumnLaunch& L, ColumnShared&
 // before the leader's update of x, so x is read again for the slots that
 // S.filter holds.
 template <bool kOverlap>
-__device__ __forceinline__ void block_update(const ColumnLaunch& L, ColumnShared& S, int nr, bool early, double& acc_newz,
-                                             double& acc_dot, unsigned& emit, unsigned& upd, unsigned& ins,
-                                             bool timed) {
+__device__ __forceinline__ void block_update(const ColumnLaunch& L, ColumnShared& S, int nr, bool early, bool timed) {
   const int tid = threadIdx.x;
   const double dxc = S.dx, zt = S.zt;
   const dd xss = S.xss, scale = S.scale;
   const long long q2 = timed ? clock64() : 0;
+  double acc_newz = S.newz[tid], acc_dot = S.dot[tid];
+  unsigned emit = S.emit[tid], upd = S.upd[tid], ins = S.ins[tid];
 #pragma unroll 1
   for (int r = 0; r < nr; ++r) {
     const unsigned long long rec = S.rec[r][tid];
@@ -485,6 +552,11 @@ __device__ __forceinline__ void block_update(const ColumnLaunch& L, ColumnShared
     }
     S.val[r][tid] = key;
   }
+  S.newz[tid] = acc_newz;
+  S.dot[tid] = acc_dot;
+  S.emit[tid] = emit;
+  S.upd[tid] = upd;
+  S.ins[tid] = ins;
   if (timed) atomicAdd(L.sect + 2, static_cast<unsigned long long>(clock64() - q2));
 }
 
@@ -550,133 +622,103 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
   const int beg = kNT * (g * chunks / G);
   const int end = min(total, kNT * ((g + 1) * chunks / G));
 
-  double acc_newz = 0.0, acc_dot = 0.0;
-  unsigned emit = 0, upd = 0, ins = 0;
+  S.newz[tid] = S.dot[tid] = 0.0;
+  S.emit[tid] = S.upd[tid] = S.ins[tid] = 0u;
   int n_list = 0;
   unsigned long long bound = 0ull;  // a lower bound of the column's m-th largest key
 
   const long long c_rounds = timed ? clock64() : 0;
-  long long c_merge = 0;
   const int M = L.list;
-  const size_t part = static_cast<size_t>(col) * G + g;
-  // Blocks of this CTA's entries, and after them, in the column's last CTA,
-  // blocks of the G lists (`merging`).
-  bool merging = false;
-  int at = beg, stop = end;
+  int at = beg;
 #pragma unroll 1
-  while (true) {
-    unsigned long long k[kRounds + 1];
-    unsigned p[kRounds + 1];
-    if (at >= stop) {
-      if (merging) break;
-      if (kOverlap && early) {  // an empty slice
-        pdl_wait();
-        early = false;
-        if (col >= __ldcg(&St->k_cur)) return;
+  while (at < end) {
+    block_probe(L, S, at, end, timed);
+    if (at == beg) {
+      if (kOverlap && early) {
+        const int state = confirm_picked(St, S, col, L.ham.norb);
+        if (state == 0) return;
+        if (state == 2) {  // read before the leader had published it: probe again
+          early = false;
+          continue;
+        }
+        if (tid < kMaxK && tid < __ldcg(&St->k_cur)) {
+          const unsigned h = filter_bit(static_cast<unsigned>(__ldcg(&St->slot[tid])));
+          atomicOr(&S.filter[h >> 5], 1u << (h & 31u));
+        }
       }
-      // This CTA's list and partial sums to global memory, then a ticket: the
-      // last CTA of the column merges all of them.
-      const long long c_post = timed ? clock64() : 0;
-      if (timed) {
-        atomicAdd(L.sect + 5, static_cast<unsigned long long>(c_rounds - c_start));
-        atomicAdd(L.sect + 8, 1ull);
-      }
-      if (!kSingle && tid < M) {
-        L.part_key[part * M + tid] = tid < n_list ? S.list_key[tid] : 0ull;
-        L.part_slot[part * M + tid] = tid < n_list ? S.list_slot[tid] : 0u;
-      }
-      // The counters travel with the sums (exact in a double) and are added
-      // once per column by its last CTA, not by every CTA into the same words.
-      const double v[kPartSum] = {warp_sum(acc_newz), warp_sum(acc_dot),
-                                  static_cast<double>(__reduce_add_sync(~0u, emit)),
-                                  static_cast<double>(__reduce_add_sync(~0u, upd)),
-                                  static_cast<double>(__reduce_add_sync(~0u, ins))};
-      if (lane == 0) {
-#pragma unroll
-        for (int j = 0; j < kPartSum; ++j) S.w_sum[j][warp] = v[j];
+      if (tid == 0) {
+        S.dx = __ldcg(&St->dx[col]);
+        S.hdiag = __ldcg(&St->hdiag[col]);
+        S.zt = __ldcg(&St->zt);
+        S.xss = dd{__ldcg(&St->xss.hi), __ldcg(&St->xss.lo)};
+        S.scale = dd{__ldcg(&St->scale.hi), __ldcg(&St->scale.lo)};
       }
       __syncthreads();
-      if (warp == 0) {
-        if (lane < kPartSum) {
-          double t = 0.0;
-#pragma unroll
-          for (int w = 0; w < kW; ++w) t += S.w_sum[lane][w];
-          L.part_sum[kPartSum * part + lane] = t;
-        }
-        __syncwarp();
-        // One fence for the whole CTA's list and sums (the barriers order
-        // them before it), then the ticket.
-        if (!kSingle && lane == 0) {
-          if (bound != 0ull) atomicMax(L.bound + col, bound);
-          __threadfence();
-          S.last = (atomicAdd(L.done + col, 1u) == static_cast<unsigned>(G - 1));
-        }
-      }
-      __syncthreads();
-      c_merge = timed ? clock64() : 0;
-      if (timed) atomicAdd(L.sect + 6, static_cast<unsigned long long>(c_merge - c_post));
-      if (kSingle) break;  // the CTA's list is the column's
-      if (!S.last) return;
-      __threadfence();
-      merging = true;
-      at = 0;
-      stop = G * M;
-      n_list = 0;
-      bound = __ldcg(L.bound + col);
-      continue;
     }
-    if (merging) {
-      // Keys below the best bound of any CTA are left out.
-      const size_t base = static_cast<size_t>(col) * G * M;
-#pragma unroll
-      for (int r = 0; r < kRounds; ++r) {
-        const int i = at + r * kNT + tid;
-        k[r] = i < stop ? __ldcg(L.part_key + base + i) : 0ull;
-        p[r] = i < stop ? static_cast<unsigned>(i) : 0u;
-      }
-    } else {
-      block_probe(L, S, at, stop, timed);
-      if (at == beg) {
-        if (kOverlap && early) {
-          const int state = confirm_picked(St, S, col, L.ham.norb);
-          if (state == 0) return;
-          if (state == 2) {  // read before the leader had published it: probe again
-            early = false;
-            continue;
-          }
-          if (tid < kMaxK && tid < __ldcg(&St->k_cur)) {
-            const unsigned h = filter_bit(static_cast<unsigned>(__ldcg(&St->slot[tid])));
-            atomicOr(&S.filter[h >> 5], 1u << (h & 31u));
-          }
-        }
-        if (tid == 0) {
-          S.dx = __ldcg(&St->dx[col]);
-          S.hdiag = __ldcg(&St->hdiag[col]);
-          S.zt = __ldcg(&St->zt);
-          S.xss = dd{__ldcg(&St->xss.hi), __ldcg(&St->xss.lo)};
-          S.scale = dd{__ldcg(&St->scale.hi), __ldcg(&St->scale.lo)};
-        }
-        __syncthreads();
-      }
-      const int nr = min(kRounds, (stop - at + kNT - 1) / kNT);
-      block_update<kOverlap>(L, S, nr, early, acc_newz, acc_dot, emit, upd, ins, timed);
-      early = false;
-      const unsigned long long shared_bound = __ldcg(L.bound + col);
-      if (shared_bound > bound) bound = shared_bound;
-#pragma unroll
-      for (int r = 0; r < kRounds; ++r) {
-        k[r] = r < nr ? S.val[r][tid] : 0ull;
-        p[r] = r < nr ? static_cast<unsigned>(S.rec[r][tid]) : 0u;
-      }
-      if (timed) atomicAdd(L.sect + 4, static_cast<unsigned long long>(nr));
-    }
-#pragma unroll
-    for (int r = 0; r < kRounds; ++r)
-      if (k[r] < bound) k[r] = 0ull;
+    const int nr = min(kRounds, (end - at + kNT - 1) / kNT);
+    block_update<kOverlap>(L, S, nr, early, timed);
+    early = false;
+    const unsigned long long shared_bound = __ldcg(L.bound + col);
+    if (shared_bound > bound) bound = shared_bound;
+    if (timed) atomicAdd(L.sect + 4, static_cast<unsigned long long>(nr));
     const long long q3 = timed ? clock64() : 0;
-    n_list = cta_select(S, k, p, n_list, L.m, bound);
-    if (timed && !merging) atomicAdd(L.sect + 3, static_cast<unsigned long long>(clock64() - q3));
+    for (int r = nr; r < kRounds; ++r) S.val[r][tid] = 0ull;
+    const Selected sel = cta_select(&S, kBlock, kNoSlot, n_list, L.m, bound);
+    n_list = sel.n_list;
+    bound = sel.bound;
+    if (timed) atomicAdd(L.sect + 3, static_cast<unsigned long long>(clock64() - q3));
     at += kBlock;
+  }
+  if (kOverlap && early) {  // an empty slice
+    pdl_wait();
+    if (col >= __ldcg(&St->k_cur)) return;
+  }
+  // This CTA's list and partial sums to global memory, then a ticket: the
+  // last CTA of the column merges all of them.
+  const size_t part = blk;  // column col's CTA g
+  const long long c_post = timed ? clock64() : 0;
+  if (timed) {
+    atomicAdd(L.sect + 5, static_cast<unsigned long long>(c_rounds - c_start));
+    atomicAdd(L.sect + 8, 1ull);
+  }
+  if (!kSingle && tid < M) {
+    L.part_key[part * M + tid] = tid < n_list ? S.list_key[tid] : 0ull;
+    L.part_slot[part * M + tid] = tid < n_list ? S.list_slot[tid] : 0u;
+  }
+  // The counters travel with the sums (exact in a double) and are added
+  // once per column by its last CTA, not by every CTA into the same words.
+  const double v[kPartSum] = {warp_sum(S.newz[tid]), warp_sum(S.dot[tid]),
+                              static_cast<double>(__reduce_add_sync(~0u, S.emit[tid])),
+                              static_cast<double>(__reduce_add_sync(~0u, S.upd[tid])),
+                              static_cast<double>(__reduce_add_sync(~0u, S.ins[tid]))};
+  if (lane == 0) {
+#pragma unroll
+    for (int j = 0; j < kPartSum; ++j) S.w_sum[j][warp] = v[j];
+  }
+  __syncthreads();
+  if (warp == 0) {
+    if (lane < kPartSum) {
+      double t = 0.0;
+#pragma unroll
+      for (int w = 0; w < kW; ++w) t += S.w_sum[lane][w];
+      L.part_sum[kPartSum * part + lane] = t;
+    }
+    __syncwarp();
+    // One fence for the whole CTA's list and sums (the barriers order
+    // them before it), then the ticket.
+    if (!kSingle && lane == 0) {
+      if (bound != 0ull) atomicMax(L.bound + col, bound);
+      __threadfence();
+      S.last = (atomicAdd(L.done + col, 1u) == static_cast<unsigned>(G - 1));
+    }
+  }
+  __syncthreads();
+  const long long c_merge = timed ? clock64() : 0;
+  if (timed) atomicAdd(L.sect + 6, static_cast<unsigned long long>(c_merge - c_post));
+  if (!kSingle) {
+    if (!S.last) return;
+    __threadfence();
+    n_list = merge_lists(S, L.part_key + static_cast<size_t>(col) * G * M, G * M, L.m, __ldcg(L.bound + col));
   }
   if (tid < L.m)
     L.cand_slot[static_cast<size_t>(col) * L.m + tid] =
