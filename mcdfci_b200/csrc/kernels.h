@@ -150,26 +150,24 @@ struct RdmLaunch {
   double *g1, *g2ss, *g2ab;
 };
 
-// Phases of the leader kernel timed into LeaderLaunch::sect: 0 state load,
-// 1 finish + prefix, 2 candidate gather (slots, dedupe, scores), 3 top-k,
-// 4 full sort when the k-th score is tied, 5 picked determinants, 6 H_sub,
-// 7 update_x, 8 publish, 9 eig setup, 10 tridiagonalisation, 11 multisection,
-// 12 inverse iteration, 13 back-transformation, 14 Rayleigh quotient,
-// 15 eig finish,
-// 16 the fast solver of eig_method 1 or 2 (when it runs, in place of 10-13:
-// its set-up and, when it fails, the restore), the rest of it in 17-20:
-// method 1: 17 Cholesky factorisation, 18 explicit inverse, 19 power steps,
-// 20 refinement steps; method 2: 17 set-up (packing of H_sub's nonzeros, the
-// bounds), 18 products and reciprocals of its steps, 19 their reductions and
-// tests, 20 their stores.  The eig set-up (9) is split further: 21 H_sub into
-// B, 22 H x, 23 the double-double sums of x'x, x'z, x'Hx (9 is then the first
-// row of B), and the Rayleigh quotient (14): 24 the product B v (14 is then
-// the double-double quotient, normalisation and residual).
+// Phases of the leader kernel timed into LeaderLaunch::sect: 0 set-up, the
+// wait for the column kernel and the state load, 1 finish of the previous
+// iteration, candidate slots and their duplicates, 2 their scores, 3 top-k
+// selection, 4 order of the picks (with the full sort when the k-th score is
+// tied), 5 the picked determinants, read and handed to the column kernel,
+// 6 H_sub, 7 update_x, 8 publish, 15 end of the eig update, 16 the bordered
+// fixed point of eig_method 2 (or the set-up of method 1's solver).  The
+// general form (eig_method 0 and 1, and the fallback of 2): 21 H_sub into B,
+// 22 H x, 23 the double-double sums of x'x, x'z, x'Hx, 9 the first row of B,
+// 10 tridiagonalisation, 11 multisection, 12 inverse iteration, 13
+// back-transformation, 24 the product B v, 14 the Rayleigh quotient,
+// normalisation and residual; method 1: 17 Cholesky factorisation, 18 explicit
+// inverse, 19 power steps, 20 refinement steps.
 constexpr int kLeaderSections = 25;
 
 // Phases of the column kernel timed into ColumnLaunch::sect (thread 0 of each
-// CTA, summed): 0 entry decode and integral value, 1 that and the slot probe,
-// 2 z atomic and score, 3 candidate selection, 4 rounds counted, 5 prelude (CTA
+// CTA, summed): 0 unused (an entry's decoding runs under the probe before it),
+// 1 entries decoded, their integrals and slots, 2 z atomic and score, 3 candidate selection, 4 rounds counted, 5 prelude (CTA
 // start to the first round), 6 CTA list store and ticket, 7 the
 // column's final merge (last CTA), 8 CTAs counted, 9 final merges counted.
 constexpr int kColumnSections = 10;
