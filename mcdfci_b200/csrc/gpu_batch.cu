@@ -103,8 +103,13 @@ GpuBatch::GpuBatch(const std::vector<const Fcidump*>& fcis, const SolverOptions&
     for (const auto& e : errs)
       if (e) std::rethrow_exception(e);
     void* reads = nullptr;
-    check(cudaMallocHost(&reads, n * sizeof(GpuSolver::StateRead)), "cudaMallocHost(batch states)");
-    reads_ = static_cast<GpuSolver::StateRead*>(reads);
+    if (cudaMallocHost(&reads, n * sizeof(GpuSolver::StateRead)) == cudaSuccess) {
+      reads_ = pinned_reads_ = static_cast<GpuSolver::StateRead*>(reads);
+    } else {  // each copy waits then
+      (void)cudaGetLastError();
+      pageable_reads_.resize(n);
+      reads_ = pageable_reads_.data();
+    }
     energies_.assign(fcis.size(), 0.0);
     active_.assign(fcis.size(), 1);
     set_groups();
@@ -112,7 +117,7 @@ GpuBatch::GpuBatch(const std::vector<const Fcidump*>& fcis, const SolverOptions&
     inst_.clear();
     if (pool_) cudaFree(pool_);
     pool_ = nullptr;
-    cudaFreeHost(reads_);
+    cudaFreeHost(pinned_reads_);
     for (size_t g = 0; g < groups_.size(); ++g)
       if (g > 0 && groups_[g].stream) cudaStreamDestroy(groups_[g].stream);
     for (auto e : join_)
@@ -128,7 +133,7 @@ GpuBatch::~GpuBatch() {
   }
   inst_.clear();
   if (pool_) cudaFree(pool_);
-  cudaFreeHost(reads_);
+  cudaFreeHost(pinned_reads_);
   for (size_t g = 1; g < groups_.size(); ++g)
     if (groups_[g].stream) cudaStreamDestroy(groups_[g].stream);
   for (auto e : join_)

@@ -72,7 +72,9 @@ class GpuBatch {
   std::vector<double> energies_;
   std::vector<char> active_;
   Slot* pool_ = nullptr;  // every instance's hash table, one allocation
-  GpuSolver::StateRead* reads_ = nullptr;  // one per instance, pinned
+  GpuSolver::StateRead* reads_ = nullptr;  // one per instance, pinned when pinned memory is had
+  GpuSolver::StateRead* pinned_reads_ = nullptr;
+  std::vector<GpuSolver::StateRead> pageable_reads_;
 };
 
 }  // namespace mcd
