@@ -35,8 +35,8 @@
 // (33 us without the load).  So a probe reads key and x in one load, and the
 // add comes later with no load beside it.  Per launch, before (a 16-byte key
 // load, then x and the atomic together; sorted warp lists) and after: 24
-// orbitals 6a5b, k = 32, m = 64: 70.8 us and 47.9 us; 42 orbitals 24a23b,
-// k = 64, m = 128: 1,757 us and 1,316 us; 12 orbitals 6a6b, k = 1, m = 100
+// orbitals 6a5b, k = 32, m = 64: 70.8 us and 46.1 us; 42 orbitals 24a23b,
+// k = 64, m = 128: 1,757 us and 1,272 us; 12 orbitals 6a6b, k = 1, m = 100
 // (the lists alone): 34.7 us and 19.8 us.
 //
 // A block has two phases.  The first needs only the picked determinant: it

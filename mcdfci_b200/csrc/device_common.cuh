@@ -197,85 +197,30 @@ __device__ __forceinline__ void load_xz(const Slot* s, double& x, double& z) {
   asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(x), "=d"(z) : "l"(&s->x) : "memory");
 }
 
-// Linear probing, continuing from the home slot i whose key (ka, kb) the
-// caller has already loaded (so that the first probe can be in flight while
-// the caller does other work).  Returns the slot index of (a,b) or -1 if absent.
-__device__ __forceinline__ long long table_find_from(const TableDev& t, uint64_t a, uint64_t b, uint64_t i,
-                                                     uint64_t ka, uint64_t kb) {
-  for (int p = 0; p < t.max_probe; ++p) {
-    if (p > 0) load_key(t.slots + i, ka, kb);
-    if (ka == a && kb == b) return static_cast<long long>(i);
-    if (ka == kEmptyKey && kb == kEmptyKey) return -1;
-    i = (i + 1) & t.mask;
-  }
-  atomicOr(t.err, kErrProbe);
-  return -1;
-}
-
-__device__ __forceinline__ long long table_find(const TableDev& t, uint64_t a, uint64_t b) {
-  const uint64_t i = det_hash(a, b) & t.mask;
-  uint64_t ka, kb;
-  load_key(t.slots + i, ka, kb);
-  return table_find_from(t, a, b, i, ka, kb);
-}
-
-// Find, and insert when `insert` (one loop for both, so that the lanes of a
-// warp that insert and those that only update stay on one path), continuing
-// from a loaded home slot as table_find_from.
-__device__ __forceinline__ long long table_probe_from(const TableDev& t, uint64_t a, uint64_t b, uint64_t i,
-                                                      uint64_t ka, uint64_t kb, bool insert, bool& inserted) {
-  inserted = false;
-  for (int p = 0; p < t.max_probe; ++p) {
-    if (p > 0) load_key(t.slots + i, ka, kb);
-    if (ka == a && kb == b) return static_cast<long long>(i);
-    if (ka == kEmptyKey && kb == kEmptyKey) {
-      if (!insert) return -1;
-      uint64_t oa, ob;
-      cas_key(t.slots + i, a, b, oa, ob);
-      if (oa == kEmptyKey && ob == kEmptyKey) {
-        inserted = true;
-        atomicAdd(t.n_occupied, 1ull);
-        return static_cast<long long>(i);
-      }
-      if (oa == a && ob == b) return static_cast<long long>(i);
-    }
-    i = (i + 1) & t.mask;
-  }
-  atomicOr(t.err, kErrProbe);
-  return -1;
-}
-
-// Find or insert, continuing from a loaded home slot as table_find_from.
-// `inserted` is set when this call created the slot (x = z = 0 from the
-// table's initialisation).  Returns -1 only when the probe limit is hit,
-// after raising kErrProbe.
-__device__ __forceinline__ long long table_upsert_from(const TableDev& t, uint64_t a, uint64_t b, uint64_t i,
-                                                       uint64_t ka, uint64_t kb, bool& inserted) {
-  inserted = false;
-  for (int p = 0; p < t.max_probe; ++p) {
-    if (p > 0) load_key(t.slots + i, ka, kb);
-    if (ka == a && kb == b) return static_cast<long long>(i);
-    if (ka == kEmptyKey && kb == kEmptyKey) {
-      uint64_t oa, ob;
-      cas_key(t.slots + i, a, b, oa, ob);
-      if (oa == kEmptyKey && ob == kEmptyKey) {
-        inserted = true;
-        atomicAdd(t.n_occupied, 1ull);
-        return static_cast<long long>(i);
-      }
-      if (oa == a && ob == b) return static_cast<long long>(i);
-    }
-    i = (i + 1) & t.mask;
-  }
-  atomicOr(t.err, kErrProbe);
-  return -1;
-}
-
+// Find or insert, by linear probing from the home slot.  `inserted` is set when
+// this call created the slot (x = z = 0 from the table's initialisation).
+// Returns -1 only when the probe limit is hit, after raising kErrProbe.
 __device__ __forceinline__ long long table_upsert(const TableDev& t, uint64_t a, uint64_t b, bool& inserted) {
-  const uint64_t i = det_hash(a, b) & t.mask;
-  uint64_t ka, kb;
-  load_key(t.slots + i, ka, kb);
-  return table_upsert_from(t, a, b, i, ka, kb, inserted);
+  uint64_t i = det_hash(a, b) & t.mask;
+  inserted = false;
+  for (int p = 0; p < t.max_probe; ++p) {
+    uint64_t ka, kb;
+    load_key(t.slots + i, ka, kb);
+    if (ka == a && kb == b) return static_cast<long long>(i);
+    if (ka == kEmptyKey && kb == kEmptyKey) {
+      uint64_t oa, ob;
+      cas_key(t.slots + i, a, b, oa, ob);
+      if (oa == kEmptyKey && ob == kEmptyKey) {
+        inserted = true;
+        atomicAdd(t.n_occupied, 1ull);
+        return static_cast<long long>(i);
+      }
+      if (oa == a && ob == b) return static_cast<long long>(i);
+    }
+    i = (i + 1) & t.mask;
+  }
+  atomicOr(t.err, kErrProbe);
+  return -1;
 }
 
 // gcd_grad score of a determinant, |x xx scale^2 + z| (CoordinatePickGcdGrad,
