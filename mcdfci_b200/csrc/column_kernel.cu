@@ -613,7 +613,10 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
     if (tid == 0) pdl_trigger();
     if (tid < 64) S.filter[tid] = 0u;
     early = read_picked(St, S, col, L.ham.norb);
-    if (!early) pdl_wait();
+    if (!early) {
+      pdl_wait();
+      __syncthreads();  // every warp has S.some of the first reading before the second writes it
+    }
   }
   if (!early && !read_picked(St, S, col, L.ham.norb)) return;
   const int total = S.P.total;
