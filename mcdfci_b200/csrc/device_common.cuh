@@ -93,7 +93,10 @@ __device__ __forceinline__ uint64_t interleaved_word(uint64_t a, uint64_t b, int
 // The reference's determinant order used to break ties between equal
 // gradients (detComp_global, src/wavefunction.h:30-36): words compared from
 // word 0, first differing word decides through the sign of the wrapped
-// difference.  Returns >0 if x sorts after y.
+// difference (words that differ in bit 63 alone, of which the reference sorts
+// neither first: the one with the bit set).  Returns >0 if x sorts after y.
+// From 32 orbitals on, where words reach 2^63, three determinants can each sort
+// after the next: a ranking must not rely on an order of all of them.
 __device__ __forceinline__ int det_ref_compare(uint64_t xa, uint64_t xb, uint64_t ya, uint64_t yb, int nwords) {
   int w = 0;
   uint64_t xw = interleaved_word(xa, xb, 0), yw = interleaved_word(ya, yb, 0);
@@ -102,6 +105,7 @@ __device__ __forceinline__ int det_ref_compare(uint64_t xa, uint64_t xb, uint64_
     yw = interleaved_word(ya, yb, w + 1);
   }
   const long long diff = static_cast<long long>(xw - yw);
+  if (static_cast<uint64_t>(diff) == 1ull << 63) return xw > yw ? 1 : -1;
   return (diff > 0) - (diff < 0);
 }
 

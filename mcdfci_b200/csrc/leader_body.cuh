@@ -946,6 +946,43 @@ __device__ __noinline__ void sort_candidates(const Candidates& C, int k, const S
   __syncthreads();
 }
 
+// The ranks of k picked keys once more, for equal ones that det_ref_compare
+// leaves in a circle (two of them then have the same number of determinants
+// sorted before them, and a place stays empty): by that number, and where it is
+// equal by the larger occupation strings.
+__device__ __noinline__ void rank_circular(const unsigned long long* key, const unsigned* slot, int k, const Slot* slots,
+                                           int nwords, unsigned* out) {
+  __shared__ unsigned char s_before[kMaxK];
+  const int i = threadIdx.x;
+  const unsigned long long mine = i < k ? key[i] : 0ull;
+  uint64_t ia = 0, ib = 0;
+  int before = 0;
+  if (i < k) {
+    load_key(slots + slot[i], ia, ib);
+    for (int j = 0; j < k; ++j) {
+      if (j == i || key[j] != mine) continue;
+      uint64_t ja, jb;
+      load_key(slots + slot[j], ja, jb);
+      before += det_ref_compare(ja, jb, ia, ib, nwords) > 0;
+    }
+    s_before[i] = static_cast<unsigned char>(before);
+  }
+  __syncthreads();
+  if (i < k) {
+    int rank = 0;
+    for (int j = 0; j < k; ++j) {
+      rank += key[j] > mine;
+      if (j == i || key[j] != mine) continue;
+      uint64_t ja, jb;
+      load_key(slots + slot[j], ja, jb);
+      const int bj = s_before[j];
+      rank += bj < before || (bj == before && (ja > ia || (ja == ia && jb > ib)));
+    }
+    out[rank] = slot[i];
+  }
+  __syncthreads();
+}
+
 __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ __align__(16) IterState sS;  // the scalars; the per-column arrays stay in global memory
@@ -975,6 +1012,7 @@ __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
   for (int i = tid; i < C.pr / 2; i += kLT)
     reinterpret_cast<uint4*>(C.set)[i] = make_uint4(kNoSlot, kNoSlot, kNoSlot, kNoSlot);
   if (tid == 0) s_out = s_newx = 0u;
+  if (tid < kMaxK) s_slot[tid] = kNoSlot;
 
   pdl_wait();  // for the column kernel
 
@@ -1099,8 +1137,10 @@ __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
     }
     __syncthreads();
     clk.mark(3);
-    // Ranks by counting, 16 lanes per key.
+    // Ranks by counting, 16 lanes per key; a place that two keys claim shows
+    // equal keys without an order of their own.
     const int part = tid & 15;
+    bool claimed = false;
 #pragma unroll 1
     for (int i0 = 0; i0 < k; i0 += kLT / 16) {
       const int i = i0 + (tid >> 4);
@@ -1128,10 +1168,10 @@ __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
             rank += det_ref_compare(ja, jb, ia, ib, sS.n_words) > 0 ? 1u : 0u;
           }
         }
-        s_slot[rank] = slot;
+        claimed |= atomicExch(&s_slot[rank], slot) != kNoSlot;
       }
     }
-    __syncthreads();
+    if (__syncthreads_or(claimed)) rank_circular(s_sel_key, s_sel_slot, k, T.slots, sS.n_words, s_slot);
   } else {
     __syncthreads();
     sort_candidates(C, k, T.slots, sS.n_words, s_slot);
