@@ -612,7 +612,9 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
   if (kOverlap) {
     if (tid == 0) pdl_trigger();
     if (tid < 64) S.filter[tid] = 0u;
-    early = read_picked(St, S, col, L.ham.norb);
+    // (a determinant that the leader has not published yet may be of no sector:
+    // the slice below holds for all determinants of the launch's own)
+    early = read_picked(St, S, col, L.ham.norb) && S.P.na == L.na && S.P.nb == L.nb;
     if (!early) {
       pdl_wait();
       __syncthreads();  // every warp has S.some of the first reading before the second writes it

@@ -109,3 +109,14 @@ def test_walk_finds_a_missing_barrier():
     answer for the first."""
     found = _outcomes([("read", 0), ("read", 1)], (False, True))
     assert found - {(1, 1)}
+
+
+def test_slice_is_taken_of_the_own_sector_only():
+    """A CTA that finds after the leader's end that its first reading named
+    another determinant probes the new one over the slice it already has.  The
+    number of entries depends on the electrons per spin alone, so the first
+    reading counts only with those of the launch; anything else (the zeroed state
+    of a column that no iteration has had) waits for the second reading."""
+    body = _function("column_body")
+    first = re.search(r"early = ([^;]*);", body[body.index("pdl_trigger"):]).group(1)
+    assert re.fullmatch(r"read_picked\([^)]*\) && S\.P\.na == L\.na && S\.P\.nb == L\.nb", first)
