@@ -62,7 +62,8 @@
 // Candidates.  The keys of a block and the CTA's list so far (at most m) are
 // reduced to the m largest by a radix selection over the whole CTA
 // (cta_select): a histogram per pass and one barrier, no sort, since nothing
-// downstream depends on the order of a candidate list.  Each CTA's list goes
+// downstream depends on the order of a candidate list.  Of equal keys at the
+// m-th place the larger determinants stay, whichever warp comes first.  Each CTA's list goes
 // to global memory with its sums, and the last CTA of the column to finish
 // (atomic ticket) selects the column's m from the G lists and adds the sums
 // in a fixed order.  A full list's smallest key is a lower bound of the
@@ -309,7 +310,9 @@ struct alignas(16) ColumnShared {
   double dx, hdiag, zt;  // the column's scalars
   dd xss, scale;
   unsigned filter[64];  // of the picked slots
-  unsigned out, ties;
+  unsigned out, n_tied, tied[kMaxM];
+  const Slot* slots;          // the table, and
+  const unsigned* part_slot;  // the slots of the keys that the merge selects from
   unsigned slot;        // the picked determinant's
   int last, some;
 };
@@ -319,10 +322,109 @@ struct Selected {
   unsigned long long bound;
 };
 
+// The determinant of a payload of cta_select's.
+__device__ __forceinline__ void payload_key(const ColumnShared& S, unsigned base, unsigned payload, uint64_t& a,
+                                            uint64_t& b) {
+  load_key(S.slots + (base == kNoSlot ? payload : __ldcg(S.part_slot + payload)), a, b);
+}
+
+// cta_keep_tied for more keys than a warp ranks, n_listed of them from the list:
+// the largest strings that `need` keys reach, bit by bit.
+__device__ __noinline__ void cta_keep_tied_many(ColumnShared* s, int n, unsigned base, int n_listed,
+                                                unsigned long long edge, int need, bool in_pool) {
+  __builtin_assume(__isShared(s));
+  ColumnShared& S = *s;
+  const int tid = threadIdx.x;
+  unsigned* counts = &S.sel.hist[0][0];
+  counts[tid] = 0u;
+  __syncthreads();
+  const int norb = S.P.na + S.P.va, last = 2 * norb;
+  uint64_t cut_a = 0, cut_b = 0;
+  // A step for each bit of alpha and then of beta; the last keeps what reaches the cut.
+#pragma unroll 1
+  for (int step = 0;; ++step) {
+    const bool alpha = step < norb;
+    const uint64_t bit = step < last ? 1ull << (norb - 1 - (alpha ? step : step - norb)) : 0ull;
+    const uint64_t try_a = alpha ? cut_a | bit : cut_a, try_b = alpha ? cut_b : cut_b | bit;
+    unsigned c = 0;
+#pragma unroll 1
+    for (int i = tid - kNT; i < n; i += kNT) {
+      const bool tied = i < 0 ? tid < n_listed : in_pool && (&S.val[0][0])[i] == edge;
+      if (!tied) continue;
+      const unsigned payload = i < 0            ? S.tied[tid]
+                               : base == kNoSlot ? static_cast<unsigned>((&S.rec[0][0])[i])
+                                                 : base + i;
+      uint64_t a, b;
+      payload_key(S, base, payload, a, b);
+      if (a < try_a || (a == try_a && b < try_b)) continue;
+      ++c;
+      if (step == last) {
+        const unsigned pos = atomicAdd(&S.out, 1u);
+        S.list_key[pos] = edge;
+        S.list_slot[pos] = payload;
+      }
+    }
+    if (step == last) return;
+    c = __reduce_add_sync(~0u, c);
+    if ((tid & 31) == 0) atomicAdd(&counts[step], c);
+    __syncthreads();
+    const int reach = static_cast<int>(counts[step]);
+    if (reach < need) continue;
+    cut_a = try_a;
+    cut_b = try_b;
+    if (reach == need) step = last - 1;
+  }
+}
+
+// Of cta_select's keys equal to `edge`, the payloads in S.tied (from the list)
+// and those of the pool (with in_pool), the `need` whose determinants have the
+// largest (alpha, beta) strings, added to S.list.  Out of line: few selections
+// need it, and what the others run should stay small.
+__device__ __noinline__ void cta_keep_tied(ColumnShared* s, int n, unsigned base, unsigned long long edge, int need,
+                                           bool in_pool) {
+  __builtin_assume(__isShared(s));
+  ColumnShared& S = *s;
+  const unsigned long long* pool = &S.val[0][0];
+  const int tid = threadIdx.x;
+  __syncthreads();
+  const unsigned listed = S.n_tied;
+  __syncthreads();
+  if (in_pool)
+#pragma unroll 1
+    for (int i = tid; i < n; i += kNT)
+      if (pool[i] == edge) {
+        const unsigned pos = atomicAdd(&S.n_tied, 1u);
+        if (pos < 32u) S.tied[pos] = base == kNoSlot ? static_cast<unsigned>((&S.rec[0][0])[i]) : base + i;
+      }
+  __syncthreads();
+  const unsigned tied = S.n_tied;
+  if (tied > 32u) {
+    cta_keep_tied_many(s, n, base, static_cast<int>(listed), edge, need, in_pool);
+    return;
+  }
+  if (tid >= 32) return;
+  const bool mine = static_cast<unsigned>(tid) < tied;
+  const unsigned payload = mine ? S.tied[tid] : 0u;
+  uint64_t a = 0, b = 0;
+  if (mine) payload_key(S, base, payload, a, b);
+  unsigned rank = 0;
+#pragma unroll 1
+  for (unsigned j = 0; j < tied; ++j) {
+    const uint64_t oa = __shfl_sync(~0u, a, j), ob = __shfl_sync(~0u, b, j);
+    rank += oa > a || (oa == a && ob > b) ? 1u : 0u;
+  }
+  if (mine && static_cast<int>(rank) < need) {
+    const unsigned pos = atomicAdd(&S.out, 1u);
+    S.list_key[pos] = edge;
+    S.list_slot[pos] = payload;
+  }
+}
+
 // Reduces the CTA's candidates, S.list's n_list and the keys of n / kBlock
 // whole blocks from S.val on (0 and those below `bound` left out), to the m largest in S.list, in no
-// particular order.  Their payloads: the slots in S.rec, or base + index when
-// base is not kNoSlot.  Raises `bound` to the smallest value a kept key can
+// particular order; of equal keys at the m-th place the larger determinants
+// stay, so that the set follows from the keys alone.  Their payloads: the slots in S.rec, or base + index when
+// base is not kNoSlot (the slots then in S.part_slot).  Raises `bound` to the smallest value a kept key can
 // have when some were left out.  Called by the whole CTA, each thread having
 // written the keys tid + j kNT itself (0 beyond the last); ends with a barrier.  One copy of the
 // code, out of line, serves a CTA's blocks and the merge of the lists: the
@@ -345,7 +447,7 @@ __device__ __noinline__ Selected cta_select(ColumnShared* s, int n, unsigned bas
   const unsigned list_slot = tid < n_list ? S.list_slot[tid] : 0u;
   if (tid == 0) {
     S.out = 0u;
-    S.ties = 0u;
+    S.n_tied = 0u;
   }
   const unsigned want = static_cast<unsigned>(m);
   const SelectEdge E = select_edge(S.sel, want, [&](auto f) {
@@ -360,13 +462,16 @@ __device__ __noinline__ Selected cta_select(ColumnShared* s, int n, unsigned bas
     }
   });
   const unsigned long long least = E.edge > floor ? E.edge : floor;
+  const unsigned long long from = E.edge + (E.tied ? 1ull : 0ull), pool_from = from > floor ? from : floor;
   const auto keep = [&](unsigned long long key, unsigned slot) {
-    if (E.tied && key == E.edge && atomicAdd(&S.ties, 1u) >= E.need) return;
     const unsigned pos = atomicAdd(&S.out, 1u);
     S.list_key[pos] = key;
     S.list_slot[pos] = slot;
   };
-  if (list_key >= E.edge) keep(list_key, list_slot);
+  if (list_key >= from)
+    keep(list_key, list_slot);
+  else if (list_key == E.edge)
+    S.tied[atomicAdd(&S.n_tied, 1u)] = list_slot;
 #pragma unroll 1
   for (int i0 = tid; i0 < n; i0 += kRounds * kNT) {
     unsigned long long key[kRounds];
@@ -375,13 +480,14 @@ __device__ __noinline__ Selected cta_select(ColumnShared* s, int n, unsigned bas
 #pragma unroll
     for (int j = 0; j < kRounds; ++j) {
       const int i = i0 + j * kNT;
-      if (key[j] >= least)
+      if (key[j] >= pool_from)
         keep(key[j], base == kNoSlot ? static_cast<unsigned>((&S.rec[0][0])[i]) : base + static_cast<unsigned>(i));
     }
   }
-  if (E.total > want) bound = least;
+  const Selected r{static_cast<int>(min(E.total, want)), E.total > want ? least : bound};
+  if (E.tied) cta_keep_tied(s, n, base, E.edge, static_cast<int>(E.need), E.edge >= floor);
   __syncthreads();
-  return Selected{static_cast<int>(min(E.total, want)), bound};
+  return r;
 }
 
 // The m largest of the n keys of a column's lists, those below `bound` (which m
@@ -389,13 +495,14 @@ __device__ __noinline__ Selected cta_select(ColumnShared* s, int n, unsigned bas
 // time in the shared memory of the rounds, where 1,024 at a time in registers
 // took a selection for each (23 lists of 128: 200 iterations of 24 columns
 // 10.9 ms, now 10.25; 96 lists of 128: 24.2 and 23.9 ms for 16 of 64 columns).
-__device__ __forceinline__ int merge_lists(ColumnShared& S, const unsigned long long* keys, int n, int m,
-                                           unsigned long long bound) {
+__device__ __forceinline__ int merge_lists(ColumnShared& S, const unsigned long long* keys, const unsigned* slots,
+                                           int n, int m, unsigned long long bound) {
   constexpr int kKeys = 3 * kRounds * kNT;
   static_assert(offsetof(ColumnShared, rec) == offsetof(ColumnShared, val) + sizeof(S.val) &&
                     offsetof(ColumnShared, x) == offsetof(ColumnShared, rec) + sizeof(S.rec),
                 "the rounds' arrays follow one another");
   unsigned long long* pool = &S.val[0][0];
+  if (threadIdx.x == 0) S.part_slot = slots;
   Selected r{0, bound};
 #pragma unroll 1
   for (int at = 0; at < n; at += kKeys) {
@@ -655,6 +762,7 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
         S.dx = __ldcg(&St->dx[col]);
         S.hdiag = __ldcg(&St->hdiag[col]);
         S.zt = __ldcg(&St->zt);
+        S.slots = L.tab.slots;
         S.xss = dd{__ldcg(&St->xss.hi), __ldcg(&St->xss.lo)};
         S.scale = dd{__ldcg(&St->scale.hi), __ldcg(&St->scale.lo)};
       }
@@ -723,7 +831,8 @@ __device__ __forceinline__ void column_body(const ColumnLaunch& L, int blk) {
   if (!kSingle) {
     if (!S.last) return;
     __threadfence();
-    n_list = merge_lists(S, L.part_key + static_cast<size_t>(col) * G * M, G * M, L.m, __ldcg(L.bound + col));
+    const size_t lists = static_cast<size_t>(col) * G * M;
+    n_list = merge_lists(S, L.part_key + lists, L.part_slot + lists, G * M, L.m, __ldcg(L.bound + col));
   }
   if (tid < L.m)
     L.cand_slot[static_cast<size_t>(col) * L.m + tid] =
