@@ -909,7 +909,11 @@ struct Candidates {
 
 // Full sort by decreasing key, equal keys in the reference's determinant
 // order (rare: the k-th and (k+1)-th keys are equal); the first k slots to out.
-__device__ __noinline__ void sort_candidates(const Candidates& C, int k, const Slot* slots, int nwords, unsigned* out) {
+// Where that is no order of all determinants (norb >= 32, det_ref_compare) the
+// outcome depends on the candidates' places, which differ from run to run: a
+// pass before puts equal keys by their larger occupation strings.
+__device__ __noinline__ void sort_candidates(const Candidates& C, int k, const Slot* slots, int nwords, int norb,
+                                             unsigned* out) {
   int P = 1;
   while (P < C.n) P <<= 1;
   for (int u = C.n + threadIdx.x; u < P; u += kLT) {
@@ -917,29 +921,32 @@ __device__ __noinline__ void sort_candidates(const Candidates& C, int k, const S
     C.slot[u] = kNoSlot;
   }
   __syncthreads();
-  for (int size = 2; size <= P; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int t = threadIdx.x; t < (P >> 1); t += kLT) {
-        const int i = 2 * stride * (t / stride) + (t % stride);
-        const int j = i + stride;
-        const unsigned long long ki = C.key[i], kj = C.key[j];
-        bool jfirst = kj > ki;
-        if (ki == kj && ki != 0ull) {
-          uint64_t ia, ib, ja, jb;
-          load_key(slots + C.slot[i], ia, ib);
-          load_key(slots + C.slot[j], ja, jb);
-          jfirst = det_ref_compare(ja, jb, ia, ib, nwords) > 0;
+#pragma unroll 1
+  for (int pass = norb < 32 ? 1 : 0; pass < 2; ++pass) {
+    for (int size = 2; size <= P; size <<= 1) {
+      for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        for (int t = threadIdx.x; t < (P >> 1); t += kLT) {
+          const int i = 2 * stride * (t / stride) + (t % stride);
+          const int j = i + stride;
+          const unsigned long long ki = C.key[i], kj = C.key[j];
+          bool jfirst = kj > ki;
+          if (ki == kj && ki != 0ull) {
+            uint64_t ia, ib, ja, jb;
+            load_key(slots + C.slot[i], ia, ib);
+            load_key(slots + C.slot[j], ja, jb);
+            jfirst = pass == 0 ? ja > ia || (ja == ia && jb > ib) : det_ref_compare(ja, jb, ia, ib, nwords) > 0;
+          }
+          const bool up = (i & size) == 0;
+          if (jfirst == up && (ki != kj || ki != 0ull)) {
+            C.key[i] = kj;
+            C.key[j] = ki;
+            const unsigned tmp = C.slot[i];
+            C.slot[i] = C.slot[j];
+            C.slot[j] = tmp;
+          }
         }
-        const bool up = (i & size) == 0;
-        if (jfirst == up && (ki != kj || ki != 0ull)) {
-          C.key[i] = kj;
-          C.key[j] = ki;
-          const unsigned tmp = C.slot[i];
-          C.slot[i] = C.slot[j];
-          C.slot[j] = tmp;
-        }
+        __syncthreads();
       }
-      __syncthreads();
     }
   }
   if (threadIdx.x < k) out[threadIdx.x] = C.slot[threadIdx.x];
@@ -1174,7 +1181,7 @@ __device__ __forceinline__ void leader_body(const LeaderLaunch& L) {
     if (__syncthreads_or(claimed)) rank_circular(s_sel_key, s_sel_slot, k, T.slots, sS.n_words, s_slot);
   } else {
     __syncthreads();
-    sort_candidates(C, k, T.slots, sS.n_words, s_slot);
+    sort_candidates(C, k, T.slots, sS.n_words, L.ham.norb, s_slot);
   }
   clk.mark(4);
   if (tid < k) {

@@ -79,3 +79,27 @@ def test_one_coordinate_repeats(synth_fcidumps, name):
         runs.append((a[order].tolist(), b[order].tolist(), x[order].tobytes(), s.report()["energy"]))
         s.close()
     assert all(r == runs[0] for r in runs[1:])
+
+
+def test_circular_order_repeats(tmp_path):
+    """34 orbitals, where the reference's order of determinants has circles (alpha
+    30 and beta 32 sorts after 31 and 31, that after 33 and 31, and that after the
+    first): picks among 127 equal scores."""
+    n = 34
+    lines = [f"&FCI NORB={n},NELEC=2,MS2=0,", " ORBSYM=" + "1," * n, " ISYM=1,", "&END"]
+    for r in range(1, n):
+        lines += [f"0.125 {r + 1} 1 {s + 1} 1" for s in range(1, r + 1)]
+    lines += ["-10.0 1 1 0 0"] + [f"1.0 {r + 1} {r + 1} 0 0" for r in range(1, n)]
+    lines += ["-10.0 1 0 0 0"] + [f"1.0 {r + 1} 0 0 0" for r in range(1, n)] + ["0.0 0 0 0 0"]
+    p = tmp_path / "equal.fcidump"
+    p.write_text("\n".join(lines) + "\n")
+    for k in (8, 64):
+        seen = set()
+        for groups in (1, 2, 5) * 4:
+            s = m.CDFCI(m.Fcidump(str(p)), num_of_coordinate=k, estimate=128, max_memory=0.05, threshold=0.0,
+                        z_threshold=0.0, groups=groups)
+            s.reset()
+            s.run_iterations(1)
+            seen.add(tuple(zip(*(v.tolist() for v in s.picked()[:2]))))
+            s.close()
+        assert len(seen) == 1
