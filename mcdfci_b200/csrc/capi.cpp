@@ -522,7 +522,9 @@ int debug_eig_host(int32_t k, const double* hsub, const double* x, const double*
     }
   } b;
   auto ck = [](cudaError_t e) {
-    if (e != cudaSuccess) throw mcd::McdError(MCD_ERR_CUDA, cudaGetErrorString(e));
+    if (e == cudaSuccess) return;
+    (void)cudaGetLastError();  // the next launch is not to report it
+    throw mcd::McdError(MCD_ERR_CUDA, cudaGetErrorString(e));
   };
   ck(cudaMalloc(&b.h, sizeof(double) * k * k));
   ck(cudaMalloc(&b.x, sizeof(double) * k));

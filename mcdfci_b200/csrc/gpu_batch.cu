@@ -22,7 +22,9 @@ constexpr int kBatchGroups = MCD_BATCH_GROUPS;
 }  // namespace
 
 void GpuBatch::check(cudaError_t e, const char* what) {
-  if (e != cudaSuccess) throw McdError(MCD_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+  if (e == cudaSuccess) return;
+  (void)cudaGetLastError();  // the next launch is not to report it
+  throw McdError(MCD_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
 GpuBatch::GpuBatch(const std::vector<const Fcidump*>& fcis, const SolverOptions& opt) : opt_(opt) {
@@ -58,10 +60,8 @@ GpuBatch::GpuBatch(const std::vector<const Fcidump*>& fcis, const SolverOptions&
     size_t total = 0;
     for (size_t i = 0; i < fcis.size(); ++i) total += caps[i] = GpuSolver::full_capacity(*fcis[i], opt_.max_memory);
     void* pool = nullptr;
-    cudaError_t ae = cudaMalloc(&pool, total * sizeof(Slot));
-    if (ae != cudaSuccess)
-      throw McdError(MCD_ERR_CUDA, "cudaMalloc(batch tables, " + std::to_string(total * sizeof(Slot)) +
-                                       " bytes): " + cudaGetErrorString(ae));
+    const std::string what = "cudaMalloc(batch tables, " + std::to_string(total * sizeof(Slot)) + " bytes)";
+    check(cudaMalloc(&pool, total * sizeof(Slot)), what.c_str());
     pool_ = static_cast<Slot*>(pool);
     // Instance i goes to group i % ng, on that group's stream.  The
     // instances are independent, so they are constructed on up to eight host

@@ -414,9 +414,11 @@ template <typename T>
 T* device_alloc(size_t count, const char* what) {
   void* p = nullptr;
   const cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-  if (e != cudaSuccess)
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();  // the next launch is not to report it
     throw McdError(MCD_ERR_CUDA, std::string("cudaMalloc(") + what + ", " + std::to_string(count * sizeof(T)) +
                                      " bytes): " + cudaGetErrorString(e));
+  }
   return static_cast<T*>(p);
 }
 
@@ -434,7 +436,10 @@ unsigned long long* pinned_words_acquire() {
     constexpr int kPairs = 256;
     void* p = nullptr;
     const cudaError_t e = cudaMallocHost(&p, kPairs * 2 * sizeof(unsigned long long));
-    if (e != cudaSuccess) throw McdError(MCD_ERR_CUDA, std::string("cudaMallocHost: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();
+      throw McdError(MCD_ERR_CUDA, std::string("cudaMallocHost: ") + cudaGetErrorString(e));
+    }
     auto* b = static_cast<unsigned long long*>(p);
     for (int i = kPairs - 1; i >= 0; --i) g_pin_free.push_back(b + 2 * i);
   }
@@ -487,7 +492,9 @@ void staging_release(const StagingBlock& b) {
 }  // namespace
 
 void GpuSolver::check(cudaError_t e, const char* what) {
-  if (e != cudaSuccess) throw McdError(MCD_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+  if (e == cudaSuccess) return;
+  (void)cudaGetLastError();
+  throw McdError(MCD_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
 size_t GpuSolver::full_capacity(const Fcidump& fci, double max_memory) {
@@ -1344,9 +1351,7 @@ unsigned long long GpuSolver::compact(double z_threshold) {
   std::vector<void*> owned;
   auto alloc = [&](size_t bytes, const char* what) {
     void* p = nullptr;
-    const cudaError_t e = cudaMalloc(&p, bytes);
-    if (e != cudaSuccess)
-      throw McdError(MCD_ERR_CUDA, std::string("cudaMalloc(") + what + "): " + cudaGetErrorString(e));
+    check(cudaMalloc(&p, bytes), (std::string("cudaMalloc(") + what + ")").c_str());
     owned.push_back(p);
     return p;
   };
