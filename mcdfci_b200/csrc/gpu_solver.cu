@@ -978,6 +978,7 @@ bool GpuSolver::grow_now(int mode, long long* wrap) {
 void GpuSolver::grow_to(size_t new_capacity, int mode) {
   const auto t0 = std::chrono::steady_clock::now();
   read_state();  // applies the pending end of the iteration; nothing in flight
+  trim_read_scratch(0);
   const auto t_alloc = std::chrono::steady_clock::now();
   const int m = opt_.m;
   Slot* fresh = nullptr;
@@ -1236,7 +1237,8 @@ mcd_report GpuSolver::report_of(const StateRead& s) {
 
 // Device scratch of the calls that read the wavefunction out, kept between them
 // up to kReadScratch (a device allocation and its release take 0.6 ms beside a
-// large table, as long as a scan of 4 GB).
+// large table, as long as a scan of 4 GB), until the solver allocates for
+// something else.
 unsigned char* GpuSolver::read_scratch(size_t bytes) {
   if (bytes > read_bytes_) {
     cudaFree(d_read_);
@@ -1249,8 +1251,9 @@ unsigned char* GpuSolver::read_scratch(size_t bytes) {
   return d_read_;
 }
 
-void GpuSolver::trim_read_scratch() {
-  if (read_bytes_ <= kReadScratch) return;
+// Gives back what is above `keep` bytes.
+void GpuSolver::trim_read_scratch(size_t keep) {
+  if (read_bytes_ <= keep) return;
   cudaFree(d_read_);
   d_read_ = nullptr;
   read_bytes_ = 0;
@@ -1276,6 +1279,7 @@ Slot* GpuSolver::collect_x(unsigned long long* n, size_t extra, unsigned char** 
 
 void GpuSolver::wavefunction(std::vector<Det>& dets, std::vector<double>& x) {
   read_state();
+  const ReadScratchUse use{*this};
   unsigned long long n = 0;
   const Slot* d_list = collect_x(&n, 0, nullptr);
   std::vector<Slot> list(n);
@@ -1283,7 +1287,6 @@ void GpuSolver::wavefunction(std::vector<Det>& dets, std::vector<double>& x) {
     check(cudaMemcpyAsync(list.data(), d_list, n * sizeof(Slot), cudaMemcpyDeviceToHost, stream_), "list read");
     check(cudaStreamSynchronize(stream_), "synchronize");
   }
-  trim_read_scratch();
   // In slot order (the index, as a double, is exact).
   std::sort(list.begin(), list.end(), [](const Slot& p, const Slot& q) { return p.z < q.z; });
   dets.resize(n);
@@ -1297,6 +1300,7 @@ void GpuSolver::wavefunction(std::vector<Det>& dets, std::vector<double>& x) {
 void GpuSolver::rdm(double* rdm1, double* rdm2, int route) {
   if (uhf_) throw McdError(MCD_ERR_UNSUPPORTED, "RDMs are implemented for RHF FCIDUMPs.");
   read_state();
+  const ReadScratchUse use{*this};
   const int n = ham_.norb;
   const size_t n2 = static_cast<size_t>(n) * n, n4 = n2 * n2;
   const size_t out = n2 + n4, acc = n2 + 2 * n4;
@@ -1336,7 +1340,6 @@ void GpuSolver::rdm(double* rdm1, double* rdm2, int route) {
     throw;
   }
   staging_release(stage);
-  trim_read_scratch();
 }
 
 unsigned long long GpuSolver::compact(double z_threshold) {
@@ -1345,6 +1348,7 @@ unsigned long long GpuSolver::compact(double z_threshold) {
   const double sc = std::fabs(dd_to_d(h_state_.scale));
   // |dz scale| > zt is the insertion rule; |z scale| <= zt is dropped here.
   const double zlim = z_threshold / std::max(sc, 1e-300);
+  trim_read_scratch(0);
   const int nb = 148 * 8;
   const size_t chunk = (capacity_ + nb - 1) / nb;
   const int m = opt_.m;
@@ -1442,6 +1446,7 @@ uint64_t ham_fingerprint(const HamHost& h) {
 }  // namespace
 
 void GpuSolver::gather_slots(double zlim, std::vector<Slot>& out) {
+  trim_read_scratch(0);
   const int nb = 148 * 8;
   const size_t chunk = (capacity_ + nb - 1) / nb;
   unsigned long long* d_counts = device_alloc<unsigned long long>(nb, "gather counts");
@@ -1547,6 +1552,7 @@ void GpuSolver::checkpoint_load(const std::string& path) {
   if (slots.size() > limit)
     throw McdError(MCD_ERR_OVERFLOW, "The hash table is full. Please increase max_memory or z_threshold.");
   check(cudaStreamSynchronize(stream_), "synchronize");
+  trim_read_scratch(0);
   // A table that grows on demand is enlarged first to hold the saved entries
   // below 3/4 full (its contents are replaced anyway).
   {

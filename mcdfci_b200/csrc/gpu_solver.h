@@ -176,7 +176,11 @@ class GpuSolver {
   void raise_device_error();
   void build_graph();
   unsigned char* read_scratch(size_t bytes);
-  void trim_read_scratch();
+  void trim_read_scratch(size_t keep);
+  struct ReadScratchUse {  // for the length of a call, whether it returns or throws
+    GpuSolver& s;
+    ~ReadScratchUse() { s.trim_read_scratch(kReadScratch); }
+  };
   Slot* collect_x(unsigned long long* n, size_t extra, unsigned char** extra_at);
   void gather_slots(double zlim, std::vector<Slot>& out);  // occupied slots kept by zlim, in slot order
   // Table growth: before `upcoming` iterations are enqueued, make sure that

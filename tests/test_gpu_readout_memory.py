@@ -2,6 +2,8 @@
 keep.
 
 - An allocation that fails is reported by its own call alone.
+- The scratch that a read-out leaves is given back to the solver's other
+  allocations.
 """
 import ctypes
 
@@ -50,3 +52,21 @@ def test_an_error_is_reported_once(synth_fcidumps):
     s.grow()
     assert s.report()["occupied"] == before and s.table_info()["capacity"] == 1 << 17
     s.close()
+
+
+def test_growth_takes_the_scratch(synth_fcidumps):
+    """A table of 2 MB grows to 4 MB with nothing free but the 8 MB that the
+    density matrices of 24 orbitals left."""
+    path = synth_fcidumps["n24_6a6b"]
+    for full in (False, True):
+        s = _solver(path, 1, 0, num_iterations=1, report_interval=1)
+        s.rdm()
+        before = s.table_info()["capacity"]
+        assert before == 1 << 16
+        if full:
+            with _Full():
+                s.grow(0)
+        else:
+            s.grow(0)
+        assert s.table_info()["capacity"] == 2 * before
+        s.close()
