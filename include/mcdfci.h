@@ -306,7 +306,9 @@ int mcd_debug_eig_method(int32_t k, const double* hsub, const double* x, const d
                          const double xz[2], int32_t method, double drop, double* dx, double new_xx[2],
                          double new_scale[2], int32_t* branch, int32_t* steps);
 /* mcd_rdm with the pairs found by comparing every two determinants (route 1),
- * by looking up every excitation in the table (2), or as mcd_rdm does (0). */
+ * by looking up every excitation in the table (2), the same for a few
+ * determinants at a time, as without device memory for all of them (3), or as
+ * mcd_rdm does (0). */
 int mcd_debug_rdm(mcd_solver* s, double* rdm1, double* rdm2, int32_t route);
 /* mcd_debug_eig without any allocation: no counterpart in the reference.
  * The same update, solved as the leader solves it by default (method 2 at

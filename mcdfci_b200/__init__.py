@@ -413,7 +413,8 @@ class CDFCI:
 
     def debug_rdm(self, route: int):
         """rdm() with the connected pairs found by comparing determinants
-        (1) or by looking up excitations (2) (mcd_debug_rdm)."""
+        (1), by looking up excitations (2) or by that for a few
+        determinants at a time (3) (mcd_debug_rdm)."""
         import numpy as np
 
         n = self.norb

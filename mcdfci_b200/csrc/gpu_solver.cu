@@ -678,7 +678,7 @@ GpuSolver::GpuSolver(const Fcidump& fci, const SolverOptions& opt) : opt_(opt) {
                  o_pk = carve(parts * list_ * sizeof(unsigned long long)), o_ps = carve(parts * list_ * sizeof(unsigned)),
                  o_psum = carve(parts * kPartSum * sizeof(double)), o_done = carve(kMaxK * sizeof(unsigned)),
                  o_bound = carve(kMaxK * sizeof(unsigned long long)),
-                 o_scan = carve(2 * kScanBlocks * sizeof(dd) + sizeof(unsigned long long));
+                 o_scan = carve(kScanBytes);
     d_tables_ = device_alloc<unsigned char>(mo, "hamiltonian tables and iteration buffers");
     unsigned char* base = static_cast<unsigned char*>(d_tables_);
     auto up = [&](size_t o, const void* src, size_t bytes) {
@@ -1239,14 +1239,21 @@ mcd_report GpuSolver::report_of(const StateRead& s) {
 // up to kReadScratch (a device allocation and its release take 0.6 ms beside a
 // large table, as long as a scan of 4 GB), until the solver allocates for
 // something else.
+// nullptr when there is no memory for it.
 unsigned char* GpuSolver::read_scratch(size_t bytes) {
   if (bytes > read_bytes_) {
-    cudaFree(d_read_);
-    d_read_ = nullptr;
-    read_bytes_ = 0;
+    trim_read_scratch(0);
     const size_t want = std::max(bytes, static_cast<size_t>(2) << 20);
-    d_read_ = device_alloc<unsigned char>(want, "read-out scratch");
-    read_bytes_ = want;
+    void* p = nullptr;
+    for (size_t size : {want, bytes}) {
+      if (cudaMalloc(&p, size) == cudaSuccess) {
+        d_read_ = static_cast<unsigned char*>(p);
+        read_bytes_ = size;
+        return d_read_;
+      }
+      (void)cudaGetLastError();
+    }
+    return nullptr;
   }
   return d_read_;
 }
@@ -1259,42 +1266,80 @@ void GpuSolver::trim_read_scratch(size_t keep) {
   read_bytes_ = 0;
 }
 
-// The occupied slots with x != 0 into read_scratch: one scan of the table,
-// which writes each as {alpha, beta, x, slot index in z's place}.  *extra_at
-// (if given): `extra` bytes of the caller's behind the list, 256-byte aligned.
-Slot* GpuSolver::collect_x(unsigned long long* n, size_t extra, unsigned char** extra_at) {
-  for (unsigned long long cap = h_state_.x_size + 64;;) {
-    const size_t list_bytes = align_up(cap * sizeof(Slot), 256);
-    unsigned char* base = read_scratch(list_bytes + 256 + extra);
-    auto* d_count = reinterpret_cast<unsigned long long*>(base + list_bytes);
-    if (extra_at) *extra_at = base + list_bytes + 256;
-    check(cudaMemsetAsync(d_count, 0, sizeof(*n), stream_), "memset");
-    check(launch_collect_x(td_, capacity_, reinterpret_cast<Slot*>(base), d_count, cap, stream_), "x list");
-    check(cudaMemcpyAsync(n, d_count, sizeof(*n), cudaMemcpyDeviceToHost, stream_), "count read");
+// The occupied slots with x != 0, {alpha, beta, x, slot index in z's place}, by
+// one scan of the table into read_scratch.  Where that list (32 bytes a
+// determinant) finds no memory beside the table it is halved until it does, and
+// at last lies in the solver's own partial sums, and the table is scanned in
+// ranges that fit it.  use(list, n, first slot, whether it is all of them, the
+// caller's `extra` bytes of scratch) for each range, in slot order.
+void GpuSolver::collect_x(size_t extra, bool in_parts, const std::function<void(const XPart&)>& use) {
+  constexpr size_t kLeast = kScanBytes / sizeof(Slot) - 1;  // (the count behind it)
+  XPart part{};
+  size_t cap = 0;
+  unsigned long long* d_count = nullptr;
+  // A list of up to `want` determinants; whether it is of that many.
+  const auto place = [&](size_t want) {
+    cap = std::max(kLeast, want);
+    unsigned char* base = read_scratch(cap * sizeof(Slot) + 256 + extra);
+    while (!base && cap > kLeast) {
+      cap = std::max(kLeast, cap / 2);
+      base = read_scratch(cap * sizeof(Slot) + 256 + extra);
+    }
+    if (!base && extra)
+      throw McdError(MCD_ERR_CUDA, "no device memory for the read-out scratch (" + std::to_string(extra) + " bytes)");
+    unsigned char* list = base ? base : d_scan_;
+    part.list = reinterpret_cast<Slot*>(list);
+    d_count = reinterpret_cast<unsigned long long*>(list + cap * sizeof(Slot));
+    part.extra = base ? base + align_up(cap * sizeof(Slot) + sizeof(*d_count), 256) : nullptr;
+    return cap >= want;
+  };
+  bool room = place(in_parts ? 0 : h_state_.x_size + 64) && !in_parts;
+  size_t step = capacity_;
+  for (size_t lo = 0; lo < capacity_;) {
+    step = std::min(step, capacity_ - lo);
+    TableDev t = td_;
+    t.slots += lo;
+    check(cudaMemsetAsync(d_count, 0, sizeof(*d_count), stream_), "memset");
+    check(launch_collect_x(t, step, part.list, d_count, cap, stream_), "x list");
+    unsigned long long n = 0;
+    check(cudaMemcpyAsync(&n, d_count, sizeof(n), cudaMemcpyDeviceToHost, stream_), "count read");
     check(cudaStreamSynchronize(stream_), "synchronize");
-    if (*n <= cap) return reinterpret_cast<Slot*>(base);
-    cap = *n;
+    if (n > cap && room) {  // more than x_size says
+      room = place(n);
+      continue;
+    }
+    if (n > cap) {  // (never for a range of at most cap slots)
+      step = std::max<size_t>(cap, std::min<size_t>(step / 2, static_cast<size_t>(0.9 * step * cap / n)));
+      continue;
+    }
+    part.n = n;
+    part.first = lo;
+    part.all = step == capacity_;
+    use(part);
+    lo += step;
   }
 }
 
 void GpuSolver::wavefunction(std::vector<Det>& dets, std::vector<double>& x) {
   read_state();
-  const ReadScratchUse use{*this};
-  unsigned long long n = 0;
-  const Slot* d_list = collect_x(&n, 0, nullptr);
-  std::vector<Slot> list(n);
-  if (n) {
-    check(cudaMemcpyAsync(list.data(), d_list, n * sizeof(Slot), cudaMemcpyDeviceToHost, stream_), "list read");
+  const ReadScratchUse scratch{*this};
+  dets.clear();
+  x.clear();
+  std::vector<Slot> list;
+  collect_x(0, false, [&](const XPart& part) {
+    list.resize(part.n);
+    if (!part.n) return;
+    check(cudaMemcpyAsync(list.data(), part.list, part.n * sizeof(Slot), cudaMemcpyDeviceToHost, stream_), "list read");
     check(cudaStreamSynchronize(stream_), "synchronize");
-  }
-  // In slot order (the index, as a double, is exact).
-  std::sort(list.begin(), list.end(), [](const Slot& p, const Slot& q) { return p.z < q.z; });
-  dets.resize(n);
-  x.resize(n);
-  for (size_t i = 0; i < n; ++i) {
-    dets[i] = Det{list[i].a, list[i].b};
-    x[i] = list[i].x;
-  }
+    // In slot order (the index, as a double, is exact).
+    std::sort(list.begin(), list.end(), [](const Slot& p, const Slot& q) { return p.z < q.z; });
+    dets.reserve(dets.size() + part.n);
+    x.reserve(x.size() + part.n);
+    for (const Slot& s : list) {
+      dets.push_back(Det{s.a, s.b});
+      x.push_back(s.x);
+    }
+  });
 }
 
 void GpuSolver::rdm(double* rdm1, double* rdm2, int route) {
@@ -1304,25 +1349,27 @@ void GpuSolver::rdm(double* rdm1, double* rdm2, int route) {
   const int n = ham_.norb;
   const size_t n2 = static_cast<size_t>(n) * n, n4 = n2 * n2;
   const size_t out = n2 + n4, acc = n2 + 2 * n4;
-  unsigned long long cnt = 0;
-  unsigned char* extra = nullptr;
   RdmLaunch r{};
-  r.list = collect_x(&cnt, (acc + out) * sizeof(double), &extra);
   r.ham = hd_;
   r.tab = td_;
-  r.nlist = static_cast<long long>(cnt);
   r.excitations = static_cast<long long>(entries_);
-  r.route = route;
-  r.g1 = reinterpret_cast<double*>(extra);
-  r.g2ss = r.g1 + n2;
-  r.g2ab = r.g2ss + n4;
+  collect_x((acc + out) * sizeof(double), route == 3, [&](const XPart& part) {
+    if (part.first == 0) {
+      r.g1 = reinterpret_cast<double*>(part.extra);
+      r.g2ss = r.g1 + n2;
+      r.g2ab = r.g2ss + n4;
+      check(cudaMemsetAsync(r.g1, 0, acc * sizeof(double), stream_), "memset");
+    }
+    r.list = part.list;
+    r.nlist = static_cast<long long>(part.n);
+    r.route = part.all && route != 3 ? route : 2;  // (a part has pairs with the others: the table is asked)
+    check(launch_rdm(r, stream_), "rdm");
+  });
   double* d_out = r.g2ab + n4;
   // Out through a pinned block (a copy into pageable memory runs at a third of
   // its rate), or straight when none is had.
   const StagingBlock stage = staging_acquire(out * sizeof(double));
   try {
-    check(cudaMemsetAsync(r.g1, 0, acc * sizeof(double), stream_), "memset");
-    check(launch_rdm(r, stream_), "rdm");
     check(launch_rdm_fold(r, 1.0 / dd_to_d(h_state_.xx), d_out, d_out + n2, stream_), "rdm fold");
     if (stage.p) {
       check(cudaMemcpyAsync(stage.p, d_out, out * sizeof(double), cudaMemcpyDeviceToHost, stream_), "rdm read");

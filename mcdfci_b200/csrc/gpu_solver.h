@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -111,7 +112,8 @@ class GpuSolver {
   // (rdm1[P*n+Q] = sum_s <a+_{Ps} a_{Qs}>, rdm2[((P*n+Q)*n+R)*n+S] =
   // sum_{s,t} <a+_{Ps} a+_{Qt} a_{St} a_{Rs}>, n spatial orbitals), so that
   // E = sum h_PQ rdm1 + 1/2 sum (PR|QS) rdm2 + E_core.
-  // rdm1 and rdm2: n^2 and n^4 doubles; route as RdmLaunch::route.
+  // rdm1 and rdm2: n^2 and n^4 doubles; route as RdmLaunch::route, or 3: by
+  // lookups for a few determinants at a time, as without room for all of them.
   void rdm(double* rdm1, double* rdm2, int route = 0);
   // Raise z_threshold to `z_threshold` and remove the entries with x = 0 and
   // |z scale| <= z_threshold, rebuilding the table; returns the occupied slots.
@@ -181,7 +183,14 @@ class GpuSolver {
     GpuSolver& s;
     ~ReadScratchUse() { s.trim_read_scratch(kReadScratch); }
   };
-  Slot* collect_x(unsigned long long* n, size_t extra, unsigned char** extra_at);
+  struct XPart {
+    Slot* list;
+    unsigned long long n;
+    size_t first;  // the range's first slot
+    bool all;
+    unsigned char* extra;
+  };
+  void collect_x(size_t extra, bool in_parts, const std::function<void(const XPart&)>& use);
   void gather_slots(double zlim, std::vector<Slot>& out);  // occupied slots kept by zlim, in slot order
   // Table growth: before `upcoming` iterations are enqueued, make sure that
   // the table keeps its load below 3/4 even if every one of them inserts a
@@ -249,7 +258,8 @@ class GpuSolver {
   unsigned* d_done_ = nullptr;
   unsigned long long* d_bound_ = nullptr;
   static constexpr int kScanBlocks = 148 * 4;  // of the whole-table scans
-  unsigned char* d_scan_ = nullptr;            // their partial sums
+  static constexpr size_t kScanBytes = 2 * kScanBlocks * sizeof(dd) + sizeof(unsigned long long);
+  unsigned char* d_scan_ = nullptr;  // their partial sums
   static constexpr size_t kReadScratch = static_cast<size_t>(128) << 20;
   unsigned char* d_read_ = nullptr;
   size_t read_bytes_ = 0;

@@ -4,9 +4,14 @@ keep.
 - An allocation that fails is reported by its own call alone.
 - The scratch that a read-out leaves is given back to the solver's other
   allocations.
+- Coefficients need no memory beside the table: the list of determinants is
+  made in ranges of the table that fit what there is, down to the solver's own
+  partial sums.
+- Density matrices summed from parts of the list equal those from all of it.
 """
 import ctypes
 
+import numpy as np
 import pytest
 
 import mcdfci_b200 as m
@@ -70,3 +75,34 @@ def test_growth_takes_the_scratch(synth_fcidumps):
             s.grow(0)
         assert s.table_info()["capacity"] == 2 * before
         s.close()
+
+
+def test_coefficients_without_memory(synth_fcidumps):
+    """3,000 determinants and more in a table of 2^22 slots: several times the 591
+    that the partial sums hold."""
+    path = synth_fcidumps["n16_5a5b"]
+    first = _solver(path, 64, 8)
+    first.wavefunction()  # (its kernels are loaded with memory at hand)
+    first.close()
+    s = _solver(path, 64, 96, table_growth=False)
+    with _Full():
+        a, b, x = s.wavefunction()
+    sa, sb, sx, _ = s.slots()
+    keep = sx != 0.0
+    assert keep.sum() > 3000
+    np.testing.assert_array_equal(a, sa[keep])
+    np.testing.assert_array_equal(b, sb[keep])
+    np.testing.assert_array_equal(x, sx[keep])
+    s.close()
+
+
+def test_matrices_from_parts(synth_fcidumps):
+    s = _solver(synth_fcidumps["n16_5a5b"], 64, 96)
+    n = len(s.wavefunction()[2])
+    assert n > 3000
+    g1, g2 = s.debug_rdm(2)
+    h1, h2 = s.debug_rdm(3)
+    s.close()
+    # An element sums at most one term per determinant and electron, each below 1.
+    tol = 4 * n * np.finfo(float).eps * 10
+    assert np.max(np.abs(g1 - h1)) <= tol and np.max(np.abs(g2 - h2)) <= tol
