@@ -453,8 +453,8 @@ void pinned_words_release(unsigned long long* w) {
   g_pin_free.push_back(w);
 }
 
-// Pinned host blocks for the Hamiltonian-table upload, kept for the process
-// and reused (a copy from pageable memory runs at a fraction of the DMA
+// Pinned host blocks for the Hamiltonian-table upload and, up to kReadStage, the
+// density matrices' way out, kept for the process and reused (a copy from pageable memory runs at a fraction of the DMA
 // rate): the smallest free block that holds `bytes`, else a new one of at
 // least 8 MB; nullptr when pinned memory cannot be had (the caller then
 // uploads from pageable memory).
@@ -1366,20 +1366,22 @@ void GpuSolver::rdm(double* rdm1, double* rdm2, int route) {
     check(launch_rdm(r, stream_), "rdm");
   });
   double* d_out = r.g2ab + n4;
-  // Out through a pinned block (a copy into pageable memory runs at a third of
-  // its rate), or straight when none is had.
-  const StagingBlock stage = staging_acquire(out * sizeof(double));
+  check(launch_rdm_fold(r, 1.0 / dd_to_d(h_state_.xx), d_out, d_out + n2, stream_), "rdm fold");
+  // Out through a pinned block of at most kReadStage (a copy into pageable
+  // memory runs at a third of its rate), or straight when none is had.
+  const StagingBlock stage = staging_acquire(std::min(out * sizeof(double), kReadStage));
   try {
-    check(launch_rdm_fold(r, 1.0 / dd_to_d(h_state_.xx), d_out, d_out + n2, stream_), "rdm fold");
-    if (stage.p) {
-      check(cudaMemcpyAsync(stage.p, d_out, out * sizeof(double), cudaMemcpyDeviceToHost, stream_), "rdm read");
+    const size_t most = stage.p ? kReadStage / sizeof(double) : n4;
+    for (size_t at = 0, n; at < out; at += n) {
+      const size_t left = at < n2 ? n2 - at : 0;  // of rdm1
+      n = std::min(most, stage.p || !left ? out - at : left);
+      double* to = stage.p ? static_cast<double*>(stage.p) : left ? rdm1 + at : rdm2 + (at - n2);
+      check(cudaMemcpyAsync(to, d_out + at, n * sizeof(double), cudaMemcpyDeviceToHost, stream_), "rdm read");
       check(cudaStreamSynchronize(stream_), "synchronize");
-      std::memcpy(rdm1, stage.p, n2 * sizeof(double));
-      std::memcpy(rdm2, static_cast<double*>(stage.p) + n2, n4 * sizeof(double));
-    } else {
-      check(cudaMemcpyAsync(rdm1, d_out, n2 * sizeof(double), cudaMemcpyDeviceToHost, stream_), "rdm read");
-      check(cudaMemcpyAsync(rdm2, d_out + n2, n4 * sizeof(double), cudaMemcpyDeviceToHost, stream_), "rdm read");
-      check(cudaStreamSynchronize(stream_), "synchronize");
+      if (!stage.p) continue;
+      const size_t first = std::min(n, left);
+      std::memcpy(rdm1 + std::min(at, n2), to, first * sizeof(double));
+      std::memcpy(rdm2 + (at + first - n2), to + first, (n - first) * sizeof(double));
     }
   } catch (...) {
     cudaStreamSynchronize(stream_);

@@ -261,6 +261,7 @@ class GpuSolver {
   static constexpr size_t kScanBytes = 2 * kScanBlocks * sizeof(dd) + sizeof(unsigned long long);
   unsigned char* d_scan_ = nullptr;  // their partial sums
   static constexpr size_t kReadScratch = static_cast<size_t>(128) << 20;
+  static constexpr size_t kReadStage = static_cast<size_t>(32) << 20;
   unsigned char* d_read_ = nullptr;
   size_t read_bytes_ = 0;
   HamDev hd_{};
