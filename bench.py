@@ -494,8 +494,8 @@ def curve_sharded_arm(args, rank, world, local_rank):
 
 def autotune_object(mc, tmp, args, local_rank):
     """CTAs per column chosen by the autotuner against the fixed rule, from
-    its timed trials (16 iterations per candidate, column-kernel device time),
-    on three workloads."""
+    its timed trials (16 iterations per candidate; device time of an iteration,
+    the column kernel overlapping the leader), on three workloads."""
     from mcdfci_b200 import synth
 
     out = {}

@@ -503,6 +503,8 @@ class CDFCI:
                     "device_setup", "upload_copy", "upload_sync", "growth_alloc", "growth_rehash", "growth_free")
 
     def autotune_info(self) -> dict:
+        """The autotuner's record (mcd_debug_autotune_info); `column_us` is the
+        time of an iteration, the column kernel overlapping the leader."""
         rule, chosen, n = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_int32()
         g = (ctypes.c_int32 * 16)()
         us = (ctypes.c_double * 16)()

@@ -1097,16 +1097,54 @@ long long GpuSolver::autotune_groups(long long budget) {
   int best = groups_;
   double best_us = 1e300;
   tune_trials_.clear();
-  for (int g : cand) {
-    set_groups(g);
-    double lead = 0.0, col = 0.0, tot = 0.0;
-    run_iterations_timed(kTuneIters, &lead, &col, &tot);
-    done += kTuneIters;
-    const double us = 1000.0 * col / kTuneIters;
-    tune_trials_.push_back({g, us});
-    if (us < best_us) {
-      best_us = us;
-      best = g;
+  // The iterations of a trial run as a solve's do, with nothing between their
+  // kernels, which overlap (an event there would keep them apart: the column
+  // kernel would be timed with the probes that otherwise run beside the
+  // leader).  A solve's first iterations, whose subspace problems are the
+  // hardest, come before the trials, and each candidate runs twice, the second
+  // time in the opposite order, since the table fills meanwhile; the first
+  // iteration of a run loads the launch's form.  16 iterations per candidate:
+  constexpr int kBefore = 4, kRun = 6, kTimed = kRun - 1;
+  static_assert(kBefore + 2 * kRun == kTuneIters, "iterations per candidate");
+  const int nc = static_cast<int>(cand.size());
+  std::vector<double> us(cand.size(), 0.0);
+  const auto run = [&](long long n) {
+    ensure_room(n);
+    launch_chunk(n);
+    record_occupancy(n);
+    done += n;
+  };
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  try {
+    for (auto& e : ev) check(cudaEventCreate(&e), "cudaEventCreate");
+    set_groups(cand[0]);
+    run(kBefore * nc);
+    for (int t = 0; t < 2 * nc; ++t) {
+      const int i = t < nc ? t : 2 * nc - 1 - t;
+      set_groups(cand[i]);
+      run(1);
+      ensure_room(kTimed);
+      check(cudaEventRecord(ev[0], stream_), "cudaEventRecord");
+      launch_chunk(kTimed);
+      check(cudaEventRecord(ev[1], stream_), "cudaEventRecord");
+      record_occupancy(kTimed);
+      done += kTimed;
+      check(cudaEventSynchronize(ev[1]), "cudaEventSynchronize");
+      float ms = 0.f;
+      check(cudaEventElapsedTime(&ms, ev[0], ev[1]), "cudaEventElapsedTime");
+      us[i] += 1000.0 * ms / (2 * kTimed);
+    }
+  } catch (...) {
+    for (auto& e : ev)
+      if (e) cudaEventDestroy(e);
+    throw;
+  }
+  for (auto& e : ev) cudaEventDestroy(e);
+  for (int i = 0; i < nc; ++i) {
+    tune_trials_.push_back({cand[i], us[i]});
+    if (us[i] < best_us) {
+      best_us = us[i];
+      best = cand[i];
     }
   }
   set_groups(best);

@@ -224,7 +224,7 @@ class GpuSolver {
   bool own_table_ = true;
   int groups_rule_ = 1;      // the CTAs per column the fixed rule gives
   bool tuned_ = false;
-  std::vector<std::pair<int, double>> tune_trials_;  // (CTAs per column, column kernel us per iteration)
+  std::vector<std::pair<int, double>> tune_trials_;  // (CTAs per column, us per iteration)
   double setup_ms_[kSetupStages] = {};
   // Occupancy reads after the last two chunks: pinned host words, events, and
   // the iterations enqueued since the reset when each was recorded.

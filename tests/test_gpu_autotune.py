@@ -30,3 +30,28 @@ def test_autotune_picks_fastest_and_caches(synth_fcidumps):
     assert i2["trials"] == [] and i2["chosen"] == info["chosen"]
     assert s2.report()["iteration"] == 200
     s2.close()
+
+
+def test_trials_time_the_iteration(synth_fcidumps):
+    """A trial's time is that of an iteration of the solve.  Here, with short
+    columns, the leader is more than half of it, so that the column kernel's own
+    time would be below the half."""
+    import time
+
+    path = synth_fcidumps["n7_5a5b"]
+    kw = dict(num_of_coordinate=8, estimate=8, max_memory=0.01, threshold=0.0, z_threshold=0.0)
+    s = m.CDFCI(m.Fcidump(path), autotune=True, **kw)
+    s.reset()
+    s.run_iterations(640)
+    info = s.autotune_info()
+    assert len(info["trials"]) >= 3
+    s.report()
+    times = []
+    for _ in range(3):
+        t = time.perf_counter()
+        s.run_iterations(640)
+        s.report()
+        times.append((time.perf_counter() - t) / 640 * 1e6)
+    chosen = next(t["column_us"] for t in info["trials"] if t["groups"] == info["chosen"])
+    assert 0.6 * min(times) < chosen < 2.0 * min(times)
+    s.close()
