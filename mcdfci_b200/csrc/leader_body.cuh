@@ -747,8 +747,7 @@ __device__ __forceinline__ void eig_bordered(BorderShared& S, const double* H, i
       vvs += S.part[w][1];
     }
     rn = sqrt(rrs / vvs);
-    // (the exact residual may be a little above what the test saw)
-    ok = rn <= 32.0 * tol && lam + rn < gl ? 1 : 0;
+    ok = rn <= 16.0 * tol && lam + rn < gl ? 1 : 0;
   }
   if (!ok) {
     if (tid == 0) S.ok = 0;

@@ -54,3 +54,68 @@ def test_update_matches_numpy(path, k, mm):
         g = np.min(np.diag(H) - (np.abs(H).sum(axis=1) - np.abs(np.diag(H))))
         assert steps == 0 or w[0] < g + 1e-9
     s.close()
+
+
+def _fixed_point(H, x, z, xx, xz):
+    """The bordered fixed point of the leader (eig_bordered) with numpy: the
+    steps it takes to converge, or None when it gives up, and its tolerance."""
+    d = np.diag(H).copy()
+    E = H - np.diag(d)
+    rest = xx - float(x @ x)
+    a, b = (xz - 2.0 * float(x @ z) + float(x @ H @ x)) / rest, (z - H @ x) / np.sqrt(rest)
+    off = np.abs(E).sum(axis=1)
+    g = np.min(d - off)
+    tol = 1e-15 * max(np.max(np.abs(d) + off + np.abs(b)), abs(a) + np.abs(b).sum())
+    y = x / np.sqrt(rest)
+    lam = a + b @ y
+    cold = not lam < g
+    if cold:
+        y, lam = np.zeros_like(x), min(a, g) - 1e-3 * (1.0 + abs(a))
+    last = np.inf
+    for t in range(64):
+        s = b + E @ y
+        new = -s / (d - lam)
+        r = np.linalg.norm((d - lam) * (y - new)) / np.sqrt(1.0 + y @ y)
+        if t % 2 == 0:
+            if (r <= tol or (t >= 2 and r > 0.25 * last and r <= 16 * tol)) and not (cold and t == 0):
+                return t + 1, tol
+            if not r < 1e140 or (t >= 8 and r > 0.8 * last) or (t >= 4 and not lam < g):
+                return None, tol
+            last = r
+        y = new
+        lam = a + b @ y
+    return None, tol
+
+
+@pytest.mark.parametrize("k", [8, 33, 65, 96, 127, 128])
+def test_bordered_form_is_taken(tmp_path, k):
+    """Where the fixed point converges (in 48 steps or fewer, the limit being 64),
+    the leader takes its result, with a residual of at most 16 times its
+    tolerance (17 for the rounding of dx, 2^-53 |x + dx| times a row of B, below
+    a tenth of it)."""
+    p = str(tmp_path / "n16.fcidump")
+    synth.write_fcidump(p, synth.SynthSpec(16, 5, 4, -20.0, 1.0, 0.1, 32), seed=4)
+    s = m.CDFCI(m.Fcidump(p), num_of_coordinate=k, estimate=min(128, 2 * k), max_memory=1.0, threshold=0.0,
+                z_threshold=0.0)
+    s.reset()
+    taken = 0
+    for it in range(24):
+        s.run_iterations(1)
+        if it == 0:
+            continue
+        steps = s.report()["inv_steps_last"]
+        e = s.last_eig_inputs()
+        H, x, z, xx, xz = e["hsub"], e["x"], e["z"], float(e["xx"].sum()), float(e["xz"].sum())
+        want, tol = _fixed_point(H, x, z, xx, xz)
+        if want is not None and want <= 48:
+            assert steps > 0, (it, want)
+        if steps == 0:
+            continue
+        taken += 1
+        rest = xx - float(x @ x)
+        b = (z - H @ x) / np.sqrt(rest)
+        y = (x + s.picked()[2]) / np.sqrt(rest)
+        lam = (xz - 2.0 * float(x @ z) + float(x @ H @ x)) / rest + b @ y
+        assert np.linalg.norm(b + H @ y - lam * y) <= 17.0 * tol * np.sqrt(1.0 + y @ y)
+    s.close()
+    assert taken >= 12
