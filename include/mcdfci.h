@@ -300,7 +300,8 @@ int mcd_debug_eig_shifted(int32_t k, const double* hsub, const double* x, const 
                           int32_t* branch, int32_t* steps);
 /* mcd_debug_eig with a given method, as mcd_options.eig_method selects it:
  * 0 the full reduction, 1 shifted inverse iteration first (`drop` > 0 as in
- * mcd_debug_eig_shifted), 2 the bordered fixed point first (`drop` unused).
+ * mcd_debug_eig_shifted), 2 the bordered fixed point first (`drop` unused;
+ * here up to k = 64, the reduction above: a solve has no such limit).
  * *steps receives the fast method's steps, 0 when the reduction ran. */
 int mcd_debug_eig_method(int32_t k, const double* hsub, const double* x, const double* z, const double xx[2],
                          const double xz[2], int32_t method, double drop, double* dx, double new_xx[2],

@@ -760,7 +760,7 @@ def debug_eig_shifted(hsub, x, z, xx, xz, drop):
 def debug_eig_method(hsub, x, z, xx, xz, method, drop=0.0):
     """debug_eig with a given method (mcd_options.eig_method): 0 the full
     reduction, 1 shifted inverse iteration first (drop > 0), 2 the bordered
-    fixed point first.  Returns (dx, new_xx, new_scale, branch, steps); steps
+    fixed point first (up to k = 64 here).  Returns (dx, new_xx, new_scale, branch, steps); steps
     = 0 when the full reduction ran."""
     import numpy as np
 
