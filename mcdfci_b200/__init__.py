@@ -422,6 +422,7 @@ class CDFCI:
         _check(library().mcd_debug_rdm(self._h, g1.ctypes.data_as(_dp), g2.ctypes.data_as(_dp), route))
         return g1, g2
 
+    # "decode" is 0: an entry's decoding runs under the probe of the one before.
     COLUMN_SECTIONS = ("decode", "probe", "update", "offer", "rounds", "prelude", "post", "merge", "ctas", "merges")
 
     def column_sections(self, enable: bool = True) -> dict:

@@ -139,7 +139,9 @@ __device__ __forceinline__ void load_key(const Slot* s, uint64_t& a, uint64_t& b
 // changes once, from the empty key's, so a key caught between its two words
 // has exactly one of them empty.  whole_key, on the loaded words, reads such a
 // key again; it is apart so that the load can stay in flight.  x is not written
-// while keys are inserted.
+// while keys are inserted.  (PTX's memory model promises nothing for accesses of
+// different sizes to the same bytes, here 64-bit reads beside a 128-bit
+// compare-and-swap; it takes hardware that keeps an aligned 64-bit word whole.)
 __device__ __forceinline__ void load_slot(const Slot* s, uint64_t& a, uint64_t& b, double& x) {
   uint64_t xb;
   [[maybe_unused]] uint64_t zb;

@@ -181,8 +181,8 @@ int column_list_size(int m);
 // slots of the GPU empty (resident = 0: never more); at most 96.
 constexpr int kColumnCtasPerSm = 4;
 int column_groups(int entries, int k, int resident);
-// Whether a launch of `ctas` column CTAs is to start beside the leader: when
-// all of them fit on the SMs that the leader leaves free.
+// Whether a launch of `ctas` column CTAs is to start beside the leader: up to
+// four times those that the SMs it leaves free can hold.
 bool column_overlaps(int ctas, int sms);
 // The most CTAs per column the autotuner tries, and its iterations per trial.
 constexpr int kMaxGroups = 96;
